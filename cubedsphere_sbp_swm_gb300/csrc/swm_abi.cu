@@ -14,8 +14,10 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <set>
 #include <tuple>
 #include <string>
@@ -247,9 +249,15 @@ long long round_up(long long a, long long b) { return (a + b - 1) / b * b; }
 
 // Work units of the fused stage kernel: column strips x row segments, as
 // many as fit on the GPU at once (target_ctas) so no CTA waits for a wave,
-// or exactly nseg_fixed row segments per strip when that is > 0.
+// or exactly nseg_fixed row segments per strip when that is > 0, or units of
+// a modelled cost of at most tau_fixed when that is > 0 (the ensemble, whose
+// members share one launch).
+constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
+constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
+double row_closure_cost(const SbpC& s) { return s.ne >= 6 ? 2.0 : 1.0; }
+
 bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<WorkUnit>& out,
-                std::string& why, int nseg_fixed = 0) {
+                std::string& why, int nseg_fixed = 0, double tau_fixed = 0.0) {
   auto need_lo = [&](int k) {
     if (k < s.ne) return 0;
     if (k >= n - s.ne) return n - s.last[n - 1 - k];
@@ -285,7 +293,7 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
   // counts fill one wave of target_ctas.  Each strip is cut at equal shares
   // of its row cost.
   std::vector<std::vector<int>> cuts(nstrip);
-  const double kStripEdge = 0.3, kRowClosure = s.ne >= 6 ? 2.0 : 1.0, over = 0.8 * s.rmax;
+  const double kRowClosure = row_closure_cost(s), over = kUnitHalo * s.rmax;
   std::vector<double> pre(n + 1, 0.0);
   for (int j = 0; j < n; ++j)
     pre[j + 1] = pre[j] + ((j < s.ne || j >= n - s.ne) ? 1.0 + kRowClosure : 1.0);
@@ -308,7 +316,12 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
       cut_equal(k, std::max(1, std::min(n, (int)std::lround(m))));
     }
   } else {
-    const int max_units = std::max(1, n / std::min(8, n));   // at least 8 rows a unit
+    // At least 3 rows a unit.  On a panel too small to fill the GPU the row
+    // loop of a unit is the launch's latency: N=48 d42 FP32, width 128, took
+    // 51.4 us a step at 8 rows a unit, 41.3 at 3 and 39.2 at 2 (one instance
+    // at a time; three at once 18.4, 15.9 and 18.9: the halo rows of shorter
+    // units are then paid for).
+    const int max_units = std::max(1, n / 3);
     // units of strip k for a unit cost of at most tau: m units of a strip of
     // factor f cost f * (pre[n] + m * over) in total
     auto units_of = [&](int k, double tau) {
@@ -323,9 +336,9 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
       return 6 * t;
     };
     // the smallest unit cost whose units fit the wave
-    double lo = 0.0, hi = (1.0 + kStripEdge) * (pre[n] + over);
+    double lo = 0.0, hi = tau_fixed > 0.0 ? tau_fixed : (1.0 + kStripEdge) * (pre[n] + over);
     const int budget = std::max(target_ctas, 6 * nstrip);
-    for (int it = 0; it < 60; ++it) {
+    for (int it = 0; it < 60 && !(tau_fixed > 0.0); ++it) {
       const double mid = 0.5 * (lo + hi);
       if (total(mid) <= budget) hi = mid; else lo = mid;
     }
@@ -348,6 +361,14 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
         out.push_back(w);
       }
   return true;
+}
+
+// Modelled cost of a unit, in row-equivalents (the model of make_units).
+double unit_cost(const SbpC& s, int n, const WorkUnit& w) {
+  const double f = (w.i0 == 0 || w.i1 == n) ? 1.0 + kStripEdge : 1.0;
+  const int closed = std::max(0, std::min((int)w.j1, s.ne) - (int)w.j0) +
+                     std::max(0, (int)w.j1 - std::max((int)w.j0, n - s.ne));
+  return f * ((w.j1 - w.j0) + closed * row_closure_cost(s) + kUnitHalo * s.rmax);
 }
 
 bool name_order(const std::string& nm, const char* prefix, const char* suffix, int& order) {
@@ -2241,7 +2262,8 @@ struct swm_ensemble {
   void* dinst = nullptr;             // InstDev<T> [4 stages][nmem]
   WorkUnit* dunits = nullptr;
   int nunits = 0, cap_units = 0;
-  int seg_rows = 0;                  // rows per work unit (0: whole panel height)
+  int seg_rows = 0;                  // rows per work unit (0: whole panel height, kAutoRows: modelled)
+  int unit_rows = 0;                 // rows of the tallest unit
   int grid = 0;                      // persistent CTAs (0: one CTA per unit)
   cudaGraphExec_t graph = nullptr;
   std::string err;
@@ -2278,21 +2300,78 @@ std::string mem_err(swm_ensemble* ens) {
 }
 
 // Work units of every member: `seg_rows` rows per unit (0: one segment per
-// strip), largest units first so the persistent CTAs finish together.
+// strip), largest units first so that the CTAs finish together; or, with
+// kAutoRows, units of equal modelled cost tau over all members: the tau whose
+// longest-first schedule on the resident CTAs ends first, among the smallest
+// ones that give 1 to 4 waves of units (few members need short units to fill
+// the GPU, many need several waves to even out their sizes).  Whole-panel
+// units, the earlier default, left a small ensemble on a few CTAs: 9 members
+// (3 each of N=48, 96, 192, d42, FP32) 485 us a step, with 456 such units
+// 125 us; 96 members 1044 us whole-panel, 1010 with 1728 units.
+constexpr int kAutoRows = -1;
+
+double ens_makespan(const std::vector<double>& cost, int slots) {
+  std::priority_queue<double, std::vector<double>, std::greater<double>> q;
+  for (int k = 0; k < slots; ++k) q.push(0.0);
+  double end = 0.0;
+  for (double c : cost) {
+    const double t = q.top() + c;
+    q.pop();
+    q.push(t);
+    end = std::max(end, t);
+  }
+  return end;
+}
+
 int ens_units(swm_ensemble* ens, int seg_rows) {
-  std::vector<WorkUnit> all;
   std::string why;
+  std::map<int, int> sizes;   // members of each edge length
+  for (const swm_ctx* c : ens->mem) ++sizes[c->n];
+  const SbpC& tab = kTables[sbp_index(ens->order)];
+  const int slots = std::max(1, ens->occ) * ens->num_sms;
+  // the units of one member size
+  auto units_of = [&](int n, int rows, double tau, std::vector<WorkUnit>& u) {
+    u.clear();
+    const int nseg = rows > 0 ? std::max(1, (n + rows - 1) / rows) : rows == 0 ? 1 : 0;
+    return make_units(tab, n, ens->cols, 1, u, why, nseg, tau);
+  };
+  std::vector<WorkUnit> u;
+  double tau = 0.0;
+  if (seg_rows == kAutoRows) {
+    double best = 0.0, top = 0.0;
+    for (const auto& sz : sizes) top = std::max(top, (1.0 + kStripEdge) * (3.0 * sz.first + kUnitHalo * tab.rmax));
+    for (int waves = 1; waves <= 4; ++waves) {
+      double lo = 0.0, hi = top;
+      for (int it = 0; it < 16; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        long long total = 0;
+        for (const auto& sz : sizes) {
+          if (!units_of(sz.first, kAutoRows, mid, u)) return efail(ens, SWM_E_INVALID, why);
+          total += (long long)sz.second * u.size();
+        }
+        if (total <= (long long)waves * slots) hi = mid; else lo = mid;
+      }
+      std::vector<double> cost;
+      for (const auto& sz : sizes) {
+        if (!units_of(sz.first, kAutoRows, hi, u)) return efail(ens, SWM_E_INVALID, why);
+        for (int m = 0; m < sz.second; ++m)
+          for (const WorkUnit& w : u) cost.push_back(unit_cost(tab, sz.first, w));
+      }
+      std::sort(cost.begin(), cost.end(), std::greater<double>());
+      const double t = ens_makespan(cost, slots);
+      if (tau == 0.0 || t < best) { tau = hi; best = t; }
+    }
+  }
+  std::vector<WorkUnit> all;
   for (int m = 0; m < ens->nmem; ++m) {
-    const swm_ctx* c = ens->mem[m];
-    const int nseg = seg_rows > 0 ? std::max(1, (c->n + seg_rows - 1) / seg_rows) : 1;
-    std::vector<WorkUnit> u;
-    if (!make_units(kTables[sbp_index(c->order)], c->n, ens->cols, 1, u, why, nseg))
-      return efail(ens, SWM_E_INVALID, why);
+    if (!units_of(ens->mem[m]->n, seg_rows, tau, u)) return efail(ens, SWM_E_INVALID, why);
     for (WorkUnit& w : u) { w.inst = (int16_t)m; all.push_back(w); }
   }
-  std::stable_sort(all.begin(), all.end(), [](const WorkUnit& a, const WorkUnit& b) {
-    return (a.rl1 - a.rl0) * (a.cl1 - a.cl0) > (b.rl1 - b.rl0) * (b.cl1 - b.cl0);
+  std::stable_sort(all.begin(), all.end(), [&](const WorkUnit& a, const WorkUnit& b) {
+    return unit_cost(tab, ens->mem[a.inst]->n, a) > unit_cost(tab, ens->mem[b.inst]->n, b);
   });
+  ens->unit_rows = 0;
+  for (const WorkUnit& w : all) ens->unit_rows = std::max(ens->unit_rows, (int)(w.j1 - w.j0));
   if ((int)all.size() > ens->cap_units) {
     if (ens->dunits) cudaFree(ens->dunits);
     ens->dunits = nullptr;
@@ -2471,11 +2550,9 @@ int swm_ensemble_create(const swm_config* base, int nmembers, const int* member_
     return bail(e == cudaErrorMemoryAllocation ? SWM_E_NOMEM : SWM_E_CUDA,
                 std::string("ensemble alloc: ") + cudaGetErrorString(e));
   ens_box(ens);
-  // default tile shape: whole-panel strips on persistent CTAs (FP32) or one
-  // CTA per unit of 64 rows (FP64); swm_ensemble_tune measures the others
-  const bool f32 = ens->prec == SWM_FP32_FUSED;
-  if (int rc = ens_rebuild(ens, f32 ? 0 : 64, f32 ? std::max(1, ens->occ) * ens->num_sms : 0))
-    return bail(rc, ens->err);
+  // default tile shape: units of equal modelled cost, one CTA each;
+  // swm_ensemble_tune measures the others
+  if (int rc = ens_rebuild(ens, kAutoRows, 0)) return bail(rc, ens->err);
   *out = ens;
   return SWM_OK;
 }
@@ -2560,7 +2637,8 @@ int swm_ensemble_get_width(const swm_ensemble* ens, int* cols) {
 
 int swm_ensemble_get_shape(const swm_ensemble* ens, int* seg_rows, int* grid, int* nunits) {
   if (!ens) return efail(nullptr, SWM_E_INVALID, "null ensemble");
-  if (seg_rows) *seg_rows = ens->seg_rows;
+  // the modelled split reports its tallest unit
+  if (seg_rows) *seg_rows = ens->seg_rows == kAutoRows ? ens->unit_rows : ens->seg_rows;
   if (grid) *grid = ens->grid;
   if (nunits) *nunits = ens->nunits;
   return SWM_OK;
@@ -2593,7 +2671,7 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
       if (lob[m]) cudaMemcpyAsync(ens->state[m]->lo, (char*)keep[m] + hib[m], lob[m], cudaMemcpyDeviceToDevice, ens->st);
     }
   };
-  const int segs[] = {0, 192, 128, 96, 64, 48, 32, 24, 16};
+  const int segs[] = {kAutoRows, 0, 192, 128, 96, 64, 48, 32, 24, 16};
   const bool f32 = ens->prec == SWM_FP32_FUSED;
   double best = 1e30;
   int best_seg = ens->seg_rows, best_grid = ens->grid, best_cols = ens->cols;
@@ -2611,6 +2689,7 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
       if (segs[si] > 0 && segs[si] >= ens->max_n) continue;
       for (int gi = 0; gi < 2 && rc == SWM_OK; ++gi) {
         if (!f32 && grids[gi] != 0) continue;  // FP64 kernel: one CTA per unit
+        if (segs[si] == kAutoRows && grids[gi] != 0) continue;
         if ((rc = ens_rebuild(ens, segs[si], grids[gi]))) break;
         cudaGraphLaunch(ens->graph, ens->st);                          // warm-up
         cudaEventRecord(a, ens->st);
@@ -2635,7 +2714,7 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
   if (rc == SWM_OK) rc = ens_rebuild(ens, best_seg, best_grid);
   if (rc == SWM_OK) {
     EMEM(sync_check(ens->mem[0], ens->st));
-    if (seg_rows_out) *seg_rows_out = best_seg;
+    if (seg_rows_out) *seg_rows_out = best_seg == kAutoRows ? ens->unit_rows : best_seg;
     if (grid_out) *grid_out = best_grid;
     if (ms_per_step_out) *ms_per_step_out = best;
   }

@@ -137,3 +137,26 @@ def test_wide_members_match_single_instance():
     for m in range(len(wide)):
         for a, b in zip(ens.download(m), ref[m]):
             assert np.array_equal(a, b), f"member {m} (N={wide[m]}) differs"
+
+
+# the default (modelled) split: one member, members of one size, a mix with
+# the smallest panel, and more strips than resident CTAs
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("sizes", [(16,), (40,) * 3, (16, 97, 33), (24, 48) * 60])
+def test_default_split_matches_single_instance(prec, sizes):
+    start = {N: initial.balanced_zonal(N, 7 + N, 4)[:3] for N in set(sizes)}
+    want = {}
+    for N, st in start.items():
+        op = swm.OperatorSWM(swm.ModelConfig(N=N, precision=prec))
+        s = op.create_stvec()
+        s.upload(*st)
+        swm.RK4().step(s, op, _dt(N), 2)
+        want[N] = s.download()
+    ens = swm.Ensemble(swm.ModelConfig(N=sizes[0], precision=prec), sizes, [_dt(N) for N in sizes])
+    for m, N in enumerate(sizes):
+        ens.upload(m, *start[N])
+    ens.step(2)
+    ens.synchronize()
+    for m, N in enumerate(sizes):
+        for a, b in zip(ens.download(m), want[N]):
+            assert np.array_equal(a, b), f"member {m} (N={N}) differs"
