@@ -385,6 +385,12 @@ bool name_order(const std::string& nm, const char* prefix, const char* suffix, i
   return true;
 }
 
+// The two sets of FP64 stencil-input fields that the stages of a step take
+// turns with: work fields 0..9, free while a stage runs (the unfused operators
+// and the diagnostics use them in calls of their own, transfers use 11..13).
+constexpr int kDerFields = 5;
+double* der_fields(swm_ctx* c, int set) { return c->tmp + (long long)set * kDerFields * c->fs; }
+
 template <class T>
 InstDev<T> base_inst(swm_ctx* c) {
   InstDev<T> I{};
@@ -394,8 +400,14 @@ InstDev<T> base_inst(swm_ctx* c) {
   I.qw = c->qw;
   I.hs = (const T*)c->hsT;
   I.edge = (T*)c->edge;
+  if constexpr (sizeof(T) == 8) I.der = der_fields(c, 0);
   I.ghs = (T)c->ghs;
   I.grav = (T)c->cfg.grav;
+  // constants of the FP64 stage, so that no thread forms them
+  const SbpC& tab = kTables[sbp_index(c->order)];
+  I.grav2 = (T)(2.0 * c->cfg.grav);
+  I.ghs2 = (T)(0.5 * c->ghs);
+  for (int o = 1; o <= tab.H; ++o) I.gc[o - 1] = (T)(0.5 * c->ghs * tab.Qin[o - tab.inshift]);
   return I;
 }
 
@@ -489,8 +501,10 @@ int make_maps(swm_ctx* ctx, const InstDev<T>& I, int mode, StageMaps* m) {
   return SWM_OK;
 }
 
+// One stage on instance I.  FP64: I.der holds the stencil inputs of I.in, or
+// with `derive` they are formed first.
 template <class T>
-int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode) {
+int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode, bool derive = true) {
   StageMaps maps;
   if (int rc = make_maps<T>(ctx, I, mode, &maps)) return rc;
   cudaEvent_t a = nullptr, b = nullptr;
@@ -498,9 +512,14 @@ int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode) {
     CK(cudaEventCreate(&a), "event"); CK(cudaEventCreate(&b), "event");
     CK(cudaEventRecord(a, ctx->st), "event record");
   }
-  CK(launch_stage<T>(ctx->order, ctx->shape.cols, ctx->shape.fixbw != 0, &maps, I, nullptr, ctx->units,
-                     ctx->nunits, mode, ctx->shape.boxw, ctx->stage_grid, ctx->derr, ctx->st),
-     "stage kernel");
+  if constexpr (sizeof(T) == 8) {
+    if (derive) CK(launch_derive64(I, nullptr, 1, ctx->n, ctx->st), "stencil inputs");
+    CK(launch_stage64(ctx->order, I, nullptr, 1, ctx->n, mode, ctx->st), "stage kernel");
+  } else {
+    CK(launch_stage<T>(ctx->order, ctx->shape.cols, ctx->shape.fixbw != 0, &maps, I, nullptr, ctx->units,
+                       ctx->nunits, mode, ctx->shape.boxw, ctx->stage_grid, ctx->derr, ctx->st),
+       "stage kernel");
+  }
   if (ctx->timing) {
     CK(cudaEventRecord(b, ctx->st), "event record");
     ctx->ev_stage.emplace_back(a, b);
@@ -515,6 +534,16 @@ int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode) {
   return SWM_OK;
 }
 
+// FP64: stage `stage` (0..) of a chain reads one set of stencil-input fields
+// and, with `next`, writes the other.
+template <class T>
+void set_der(swm_ctx* ctx, InstDev<T>& I, int stage, bool next) {
+  if constexpr (sizeof(T) == 8) {
+    I.der = der_fields(ctx, stage & 1);
+    I.der_out = next ? der_fields(ctx, 1 - (stage & 1)) : nullptr;
+  }
+}
+
 // One RK4 step of the fused path on state s (see rk4_mod.f90:20-42).
 template <class T>
 int enqueue_rk4(swm_ctx* ctx, swm_state* s, double dt) {
@@ -525,19 +554,24 @@ int enqueue_rk4(swm_ctx* ctx, swm_state* s, double dt) {
   InstDev<T> I = base_inst<T>(ctx);
   int rc;
   // stage 1: k1 = A(v0); y = v0 + dt/2 k1; running sum from v0 + dt/6 k1
+  // (FP64: each stage leaves the stencil inputs of the next)
   I.in = v0; I.base = v0; I.out = ya; I.acc = acc;
   I.c_in = (T)(0.5 * dt); I.c_acc = (T)(dt / 6.0);
+  set_der(ctx, I, 0, true);
   if ((rc = run_stage<T>(ctx, I, MODE_RK1))) return rc;
   // stage 2: k2 = A(y); y = v0 + dt/2 k2; sum += dt/3 k2
   I.in = ya; I.out = yb; I.c_in = (T)(0.5 * dt); I.c_acc = (T)(dt / 3.0);
-  if ((rc = run_stage<T>(ctx, I, MODE_RK2))) return rc;
+  set_der(ctx, I, 1, true);
+  if ((rc = run_stage<T>(ctx, I, MODE_RK2, false))) return rc;
   // stage 3: k3 = A(y); y = v0 + dt k3; sum += dt/3 k3
   I.in = yb; I.out = ya; I.c_in = (T)dt; I.c_acc = (T)(dt / 3.0);
-  if ((rc = run_stage<T>(ctx, I, MODE_RK3))) return rc;
+  set_der(ctx, I, 2, true);
+  if ((rc = run_stage<T>(ctx, I, MODE_RK3, false))) return rc;
   // stage 4: k4 = A(y); v0 = sum + dt/6 k4
   I.in = ya; I.out = nullptr; I.base_out = v0; I.base_lo = s->lo ? (T*)(void*)s->lo : nullptr;
   I.c_acc = (T)(dt / 6.0);
-  return run_stage<T>(ctx, I, MODE_RK4);
+  set_der(ctx, I, 3, false);
+  return run_stage<T>(ctx, I, MODE_RK4, false);
 }
 
 int check_state(swm_ctx* ctx, const swm_state* s) {
@@ -2412,6 +2446,7 @@ int ens_tables(swm_ensemble* ens) {
           I.in = ya; I.base = v0; I.out = nullptr; I.base_out = v0;
           I.base_lo = s->lo ? (T*)(void*)s->lo : nullptr; I.c_acc = (T)(dt / 6.0);
       }
+      set_der(c, I, i, i < 3);
       if (int rc = make_maps<T>(c, I, MODE_RK1 + i, &maps[i * M + m])) return efail(ens, rc, c->err);
       I.maps = c->shape.tma ? ens->dmaps + i * M + m : nullptr;
       inst[i * M + m] = I;
@@ -2435,8 +2470,15 @@ int ens_capture(swm_ensemble* ens) {
   ECK(cudaStreamBeginCapture(ens->st, cudaStreamCaptureModeThreadLocal), "begin capture");
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
-    e = launch_stage<T>(ens->order, ens->cols, ens->fixbw, nullptr, InstDev<T>{}, I + i * ens->nmem,
-                        ens->dunits, ens->nunits, MODE_RK1 + i, ens->boxw, ens->grid, derr, ens->st);
+    if constexpr (sizeof(T) == 8) {
+      if (i == 0) e = launch_derive64(InstDev<T>{}, I, ens->nmem, ens->max_n, ens->st);
+      if (e == cudaSuccess)
+        e = launch_stage64(ens->order, InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, MODE_RK1 + i,
+                           ens->st);
+    } else {
+      e = launch_stage<T>(ens->order, ens->cols, ens->fixbw, nullptr, InstDev<T>{}, I + i * ens->nmem,
+                          ens->dunits, ens->nunits, MODE_RK1 + i, ens->boxw, ens->grid, derr, ens->st);
+    }
     if (e == cudaSuccess)
       e = launch_edge<T>(InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i,
                          ens->st);
@@ -2826,18 +2868,19 @@ int ad_apply(swm_ctx* ctx, const T* y, const T* lk, T* out) {
   return ad_stage<T>(ctx, y, lk, nullptr, 1.0, 0.0, out, nullptr, nullptr);
 }
 
-// out = base + c F(in) by the fused stage kernel (RK stage mode; scratch
-// takes its running-sum output)
+// out = base + c F(in) by the stage kernel (RK stage mode), stage `stage` of
+// a chain of `count`.  FP64 needs no running sum; FP32 writes it to scratch.
 template <class T>
-int stage_state(swm_ctx* ctx, const T* in, const T* base, double c, T* out, T* scratch) {
+int stage_state(swm_ctx* ctx, int stage, int count, const T* in, const T* base, double c, T* out, T* scratch) {
   InstDev<T> I = base_inst<T>(ctx);
   I.in = in;
   I.base = base;
   I.out = out;
-  I.acc = scratch;
+  I.acc = sizeof(T) == 8 ? nullptr : scratch;
   I.c_in = (T)c;
   I.c_acc = T(0);
-  return run_stage<T>(ctx, I, MODE_RK1);
+  set_der(ctx, I, stage, stage + 1 < count);
+  return run_stage<T>(ctx, I, MODE_RK1, stage == 0);
 }
 
 // dx <- Phi'(x) dx for one RK4 step Phi (rk4_mod.f90:20-42)
@@ -2873,9 +2916,9 @@ int rk4_ad(swm_ctx* ctx, const T* x, T* lx, double dt) {
   T *Y2 = ads<T>(ctx, 0), *Y3 = ads<T>(ctx, 1), *Y4 = ads<T>(ctx, 2), *K = ads<T>(ctx, 3);
   T *MU = ads<T>(ctx, 5), *ACC = ads<T>(ctx, 6);
   int rc;
-  if ((rc = stage_state<T>(ctx, x, x, 0.5 * dt, Y2, K))) return rc;
-  if ((rc = stage_state<T>(ctx, Y2, x, 0.5 * dt, Y3, K))) return rc;
-  if ((rc = stage_state<T>(ctx, Y3, x, dt, Y4, K))) return rc;
+  if ((rc = stage_state<T>(ctx, 0, 3, x, x, 0.5 * dt, Y2, K))) return rc;
+  if ((rc = stage_state<T>(ctx, 1, 3, Y2, x, 0.5 * dt, Y3, K))) return rc;
+  if ((rc = stage_state<T>(ctx, 2, 3, Y3, x, dt, Y4, K))) return rc;
   if ((rc = ad_stage<T>(ctx, Y4, lx, nullptr, dt / 6.0, 0.0, MU, lx, ACC))) return rc;     // ACC = l + mu4
   if ((rc = ad_stage<T>(ctx, Y3, lx, MU, dt / 3.0, dt, MU, ACC, ACC))) return rc;          // ACC += mu3
   if ((rc = ad_stage<T>(ctx, Y2, lx, MU, dt / 3.0, 0.5 * dt, MU, ACC, ACC))) return rc;    // ACC += mu2

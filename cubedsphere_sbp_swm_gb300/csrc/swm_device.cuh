@@ -207,11 +207,15 @@ struct InstDev {
   T* base_lo;                 // FP32 RK4 final stage: S_lo; S_hi is written via base_out
   T* base_out;                // final stage: new state (FP64 v0 / FP32 S_hi)
   T* edge;                    // edge buffer (6*4*4*n)
+  const T* der;               // FP64: stencil inputs of `in` (DR_N fields)
+  T* der_out;                 // FP64: stencil inputs of the next stage state (nullable)
   const StageMaps* maps;      // TMA maps of this instance (batched launches; else null)
   T c_in;                     // stage coefficient for the next stage state
   T c_acc;                    // stage coefficient for the running sum
   T ghs;                      // 1 / (hx * a)
   T grav;
+  T grav2, ghs2;              // FP64 stage: 2 grav, ghs / 2
+  T gc[3];                    // FP64 stage: ghs / 2 times the interior coefficients
 };
 
 enum StageMode { MODE_APPLY = 0, MODE_RK1 = 1, MODE_RK2 = 2, MODE_RK3 = 3, MODE_RK4 = 4 };

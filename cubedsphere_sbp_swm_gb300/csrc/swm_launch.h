@@ -6,7 +6,7 @@
 
 namespace swm {
 
-// Fused stage kernel over nunits work units.  maps describes the buffers of
+// FP32 fused stage kernel over nunits work units.  maps describes the buffers of
 // a one-instance launch to the TMA unit (batched instances carry their own
 // maps in InstDev::maps) and boxw is the widest TMA box of the instances
 // (TMA kernels only); grid > 0 runs the TMA kernel persistently on that many
@@ -42,6 +42,13 @@ template <int CONS>
 int stage_f32_occupancy(int order, bool fixbw, int boxw);
 template <int CONS>
 cudaError_t stage_f32_prepare(int order);
+// FP64 stage: the stencil inputs of I.in into I.der, and the stage kernel that
+// reads them (and, where I.der_out is set, leaves those of the next stage
+// state), over ninst instances whose largest edge has max_n nodes.
+cudaError_t launch_derive64(const InstDev<double>& one, const InstDev<double>* many, int ninst,
+                            int max_n, cudaStream_t st);
+cudaError_t launch_stage64(int order, const InstDev<double>& one, const InstDev<double>* many,
+                           int ninst, int max_n, int mode, cudaStream_t st);
 // Cube-edge kernel over ninst instances whose largest edge has max_n nodes.
 template <class T>
 cudaError_t launch_edge(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,

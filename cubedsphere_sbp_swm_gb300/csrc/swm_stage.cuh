@@ -1,16 +1,23 @@
-// swm_stage.cuh -- fused vector-invariant RHS + RK4 stage epilogue, and the
-// cube-edge pass that finishes the panel-boundary nodes.
+// swm_stage.cuh -- SBP derivatives, the RHS tendency and RK stage epilogue,
+// the FP64 stage kernels, and the cube-edge pass that finishes the
+// panel-boundary nodes (both precisions; the FP32 stage kernel is in
+// swm_stage_tma.cuh).
 //
-// One RK stage is two launches:
-//   stage_kernel  every node: co2contra, mass flux, KE, SBP grad(KE),
-//                 curl = div(v/J, -u/J) and div(h u) with their one-sided
-//                 boundary closures; interior nodes then get Coriolis, the
-//                 tendency and the RK stage combination; panel-boundary nodes
-//                 write their pre-sync (gx, gy, zeta, div) to the edge buffer.
-//   edge_kernel   every panel-boundary node: the reference's cube-edge syncs
-//                 (2-way average on edges, 3-way at cube corners, metric-
-//                 weighted for the covariant gradient), then the same
-//                 Coriolis / tendency / RK epilogue.
+// One FP64 RK stage:
+//   point_derive_kernel  (first stage of a step only) the pointwise stencil
+//                        inputs of the state: 2(KE + g(h+hs)), J h ut, J h vt,
+//                        J ut, J vt
+//   point_stage_kernel   every node: SBP grad(KE), curl and div(h u) with
+//                        their one-sided closures from those fields; interior
+//                        nodes then get Coriolis, the tendency, the RK stage
+//                        combination and the next stage's stencil inputs;
+//                        panel-boundary nodes write their pre-sync
+//                        (gx, gy, zeta, div) to the edge buffer.
+//   edge_kernel          every panel-boundary node: the reference's cube-edge
+//                        syncs (2-way average on edges, 3-way at cube
+//                        corners, metric-weighted for the covariant
+//                        gradient), then the same tendency, RK epilogue and
+//                        (FP64) next stencil inputs.
 // Reference: operator_swm_mod.f90:61-113, rk4_mod.f90:20-42,
 // sbp_operator_mod.f90:152-228, div_ah_sbp_mod.f90:46-96,
 // grad_ah_sbp_mod.f90:51-88, curl_div_based_mod.f90:26-66,
@@ -28,16 +35,8 @@ template <> struct Ord<42> { static constexpr int idx = 1, NE = 4, NW = 6, H = 2
 template <> struct Ord<43> { static constexpr int idx = 2, NE = 4, NW = 6, H = 2, RMAX = 5; };
 template <> struct Ord<63> { static constexpr int idx = 3, NE = 6, NW = 9, H = 3, RMAX = 5; };
 
-// Threads per CTA of the FP64 kernel = the most columns a unit reads.  Two
-// warps: the column strips (own columns + 2*RMAX halo) then fill both warps,
-// and every FP64 instruction runs on nearly full warps (GB300's FP64 pipe is
-// the bound; at 128 threads a strip of N=384 left a warp with 6 live lanes).
-constexpr int STAGE_BW = 64;
-// Derived fields of the FP64 kernel's row rings: the y ring holds what the
-// y stencils read along a column (2*RMAX+1 rows), the x ring what is read
-// only on the row being finished (RMAX+1 rows: written RMAX rows ahead).
-enum { RY_KE = 0, RY_U, RY_GV, RY_N };
-enum { RX_V = 0, RX_GU, RX_JUT, RX_JVT, RX_N };
+// Stencil-input fields of the FP64 stage (InstDev::der, der_out).
+enum { DR_K2 = 0, DR_GU, DR_GV, DR_JUT, DR_JVT, DR_N };
 
 // Interior central difference with the antisymmetric coefficients of the
 // order's interior stencil; fm(o) returns the value at offset o.
@@ -77,69 +76,18 @@ __device__ __forceinline__ T d_line(int k, int n, FA fa) {
   return d_interior<ORD, T>([&](int o) { return fa(k + o); });
 }
 
-// Tendency at one node from its (synced) derivative terms and the RK stage
-// epilogue.  kk = (k_h, k_u, k_v).
-template <class T>
-__device__ __forceinline__ void stage_epilogue(const InstDev<T>& I, int mode, long long idx,
-                                               T kh, T ku, T kv) {
-  const long long fs = I.fs;
-  const T kk[3] = {kh, ku, kv};
-  if (mode == MODE_APPLY) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) I.out[c * fs + idx] = kk[c];
-    return;
-  }
-  if constexpr (sizeof(T) == 8) {
-    // FP64: the reference's order.  y = 1*v0 + c*k; w = v0 + dt/6 k1,
-    // w += dt/3 k2, w += dt/3 k3, v0 = w + dt/6 k4 (rk4_mod.f90:28-40).
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const long long o = c * fs + idx;
-      if (mode == MODE_RK1) {
-        const T b = I.base[o];
-        I.out[o] = T(1.0) * b + I.c_in * kk[c];
-        I.acc[o] = b + I.c_acc * kk[c];
-      } else if (mode == MODE_RK4) {
-        I.base_out[o] = I.acc[o] + I.c_acc * kk[c];
-      } else {
-        I.out[o] = T(1.0) * I.base[o] + I.c_in * kk[c];
-        I.acc[o] = I.acc[o] + I.c_acc * kk[c];
-      }
-    }
-  } else {
-    // FP32 compensated form: the stage increments accumulate separately from
-    // the state (dacc = dt/6 k1 + dt/3 k2 + dt/3 k3), and the final stage adds
-    // dacc + dt/6 k4 to the (hi, lo) state pair with an exact two-sum, so the
-    // FP32 state keeps the low-order bits across steps.
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const long long o = c * fs + idx;
-      if (mode == MODE_RK1) {
-        I.out[o] = I.base[o] + I.c_in * kk[c];
-        I.acc[o] = I.c_acc * kk[c];
-      } else if (mode == MODE_RK4) {
-        const T d = I.acc[o] + I.c_acc * kk[c];
-        const T hi = I.base_out[o], lo = I.base_lo[o];
-        const T t = lo + d;
-        const T s = hi + t;
-        const T bb = s - hi;
-        const T err = (hi - (s - bb)) + (t - bb);
-        I.base_out[o] = s;
-        I.base_lo[o] = err;
-      } else {
-        I.out[o] = I.base[o] + I.c_in * kk[c];
-        I.acc[o] = I.acc[o] + I.c_acc * kk[c];
-      }
-    }
-  }
-}
-
-// The same epilogue with the RK inputs already loaded: rb = base (FP32 RK4:
-// the state's high part), ra = running sum, rl = state's low part.
+// RK stage epilogue of one node from its tendency and its RK inputs: rb =
+// base (FP32 RK4: the state's high part), ra = running sum, rl = state's low
+// part.  FP64 keeps the reference's order: y = 1*v0 + c*k; w = v0 + dt/6 k1,
+// w += dt/3 k2, w += dt/3 k3, v0 = w + dt/6 k4 (rk4_mod.f90:28-40).  FP32
+// compensated form: the stage increments accumulate apart from the state, and
+// the last stage adds them to the (hi, lo) state pair with an exact two-sum,
+// so the FP32 state keeps the low-order bits across steps.  A null acc (FP64)
+// skips the running sum: the stage states of the adjoint need none.
 template <class T>
 __device__ __forceinline__ void stage_epilogue_pre(const InstDev<T>& I, int mode, long long idx,
                                                    T kh, T ku, T kv, const T* rb, const T* ra,
-                                                   const T* rl) {
+                                                   const T* rl, T* y) {
   const long long fs = I.fs;
   const T kk[3] = {kh, ku, kv};
 #pragma unroll
@@ -148,14 +96,12 @@ __device__ __forceinline__ void stage_epilogue_pre(const InstDev<T>& I, int mode
     if (mode == MODE_APPLY) {
       I.out[o] = kk[c];
     } else if (sizeof(T) == 8) {
-      if (mode == MODE_RK1) {
-        I.out[o] = T(1.0) * rb[c] + I.c_in * kk[c];
-        I.acc[o] = rb[c] + I.c_acc * kk[c];
-      } else if (mode == MODE_RK4) {
+      if (mode == MODE_RK4) {
         I.base_out[o] = ra[c] + I.c_acc * kk[c];
       } else {
-        I.out[o] = T(1.0) * rb[c] + I.c_in * kk[c];
-        I.acc[o] = ra[c] + I.c_acc * kk[c];
+        y[c] = T(1.0) * rb[c] + I.c_in * kk[c];   // the next stage's state
+        I.out[o] = y[c];
+        if (I.acc) I.acc[o] = (mode == MODE_RK1 ? rb[c] : ra[c]) + I.c_acc * kk[c];
       }
     } else {
       if (mode == MODE_RK1) {
@@ -186,181 +132,183 @@ __device__ __forceinline__ void node_tendency(T gx, T gy, T zeta, T dv, T f, T J
   kv = -gy - fz * (J * ut);
   kh = -dv;
 }
-// The same with J*ut and J*vt formed beforehand.
+// ---------------------------------------------------------------------------
+// FP64 stage.  GB300 issues a warp-wide FP64 instruction to an SM quarter
+// once in 64 cycles, so the FP64 instructions per node are the cost and
+// memory traffic is nearly free beside them.  Hence:
+//   - the pointwise stencil inputs are formed once per node, by the kernel
+//     that makes the state, and kept in fields (a row-streaming kernel that
+//     formed them for its halo rows and columns as well took 0.451 ms a step
+//     at N=384 d42 and 0.251 ms at N=192, where units had 8 rows and 6 halo
+//     rows);
+//   - one thread per node and no work units, so that every SM quarter gets
+//     the same number of warps at any size;
+//   - the nodes of the NE closure columns at either panel side are separate
+//     warps that run along the column, so that a warp's closure row is
+//     uniform and the other warps never meet one (in warps along the row, 2
+//     of 13 at N=384 ran closures and interior one after the other);
+//   - differences are taken before they are scaled, and the constants come
+//     from the host: 32 FP64 instructions a node and 11 for the stencil inputs
+//     (4/2), against 58; with constants formed per thread 50 instead of 45
+//     (0.343 against 0.306 ms a step).
+// Measured, RK4 steps d42: N=48 0.239 -> 0.090 ms, N=192 0.251 -> 0.139 ms,
+// N=384 0.451 -> 0.306 ms (N=48, 192 one instance alone; the FP64 pipe is 82%
+// busy in a lone launch).  Blocks of 64 and 256 threads measured within 1% of
+// 128; 12 blocks a SM by capping the registers 1.5% slower.
+// ---------------------------------------------------------------------------
+constexpr int PT_TPB = 128;
+
+// Node of thread tid: first the closure columns (along the column), then
+// the others (along the row).  False past the last node.
+template <int ORD>
+__host__ __device__ inline bool point_node(int n, int tid, int& p, int& i, int& j) {
+  constexpr int NE = Ord<ORD>::NE;
+  const int nclosed = 12 * NE * n, ni = n - 2 * NE;
+  if (tid < nclosed) {
+    const int r = tid / n;
+    j = tid - r * n;
+    const int c = r % NE, s = r / NE;
+    i = (s & 1) ? n - 1 - c : c;
+    p = s >> 1;
+    return true;
+  }
+  const int t = tid - nclosed, row = t / ni;
+  p = row / n;
+  j = row - p * n;
+  i = NE + t - row * ni;
+  return p < 6;
+}
+// Stencil inputs of a node with state (h, u, v).
 template <class T>
-__device__ __forceinline__ void node_tendency_j(T gx, T gy, T zeta, T dv, T f, T jut, T jvt,
-                                                T& kh, T& ku, T& kv) {
-  const T fz = f + zeta;
-  ku = -gx + fz * jvt;
-  kv = -gy - fz * jut;
-  kh = -dv;
+__device__ __forceinline__ void derive_store(T* der, long long fs, long long idx, T h, T u, T v, T J,
+                                             T q1, T q2, T q3, T grav2, const T* hs) {
+  const T ut = q1 * u + q2 * v, vt = q2 * u + q3 * v;
+  const T jut = J * ut, jvt = J * vt;
+  T k2 = (u * ut + v * vt) + grav2 * h;   // twice the Bernoulli function: ghs takes the half
+  if (hs) k2 = k2 + grav2 * hs[idx];
+  der[DR_K2 * fs + idx] = k2;
+  der[DR_GU * fs + idx] = h * jut;
+  der[DR_GV * fs + idx] = h * jvt;
+  der[DR_JUT * fs + idx] = jut;
+  der[DR_JVT * fs + idx] = jvt;
 }
 
-// SBP derivative times s: interior rows with the interior coefficients
-// pre-multiplied by s (sc[o-1] for offset o), closure rows as d_line * s.
-template <int ORD, class T>
-struct ScaledInterior {
-  T c[Ord<ORD>::H];
-};
-template <int ORD, class T>
-__device__ __forceinline__ ScaledInterior<ORD, T> scaled_interior(T s) {
-  ScaledInterior<ORD, T> r;
-  if constexpr (Ord<ORD>::H == 1) {
-    r.c[0] = T(0.5) * s;
-  } else if constexpr (Ord<ORD>::H == 2) {
-    r.c[0] = T(2.0 / 3.0) * s;
-    r.c[1] = T(-1.0 / 12.0) * s;
-  } else {
-    r.c[0] = T(3.0 / 4.0) * s;
-    r.c[1] = T(-3.0 / 20.0) * s;
-    r.c[2] = T(1.0 / 60.0) * s;
-  }
-  return r;
+template <class T>
+__global__ void __launch_bounds__(PT_TPB)
+    point_derive_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many) {
+  const InstDev<T>& I = many ? many[blockIdx.y] : one;
+  const int t = blockIdx.x * PT_TPB + threadIdx.x, row = t / I.n;
+  if (row >= 6 * I.n) return;
+  const long long fs = I.fs, x = (long long)row * I.P + (t - row * I.n);
+  derive_store<T>(const_cast<T*>(I.der), fs, x, I.in[x], I.in[fs + x], I.in[2 * fs + x],
+                  I.metric[MJ * fs + x], I.metric[MQI1 * fs + x], I.metric[MQI2 * fs + x],
+                  I.metric[MQI3 * fs + x], I.grav2, I.hs);
 }
-template <int ORD, class T, class FA>
-__device__ __forceinline__ T d_line_scaled(int k, int n, FA fa, const ScaledInterior<ORD, T>& sc,
-                                           T s) {
-  constexpr int NE = Ord<ORD>::NE, H = Ord<ORD>::H;
-  if (k >= NE && k < n - NE) {
-    T acc = sc.c[0] * (fa(k + 1) - fa(k - 1));
+
+// Interior coefficients of the first derivative (offset o = 1..H) and their
+// ratios to the first: sum_o c_o dif(o) = c_1 d_ratio(dif).
+template <int ORD>
+__host__ __device__ constexpr double d_coef(int o) {
+  return Ord<ORD>::H == 1 ? 0.5 : Ord<ORD>::H == 2 ? (o == 1 ? 2.0 / 3.0 : -1.0 / 12.0)
+                                : (o == 1 ? 3.0 / 4.0 : o == 2 ? -3.0 / 20.0 : 1.0 / 60.0);
+}
+template <int ORD, class T, class F>
+__device__ __forceinline__ T d_ratio(F dif) {
+  T s = dif(1);
 #pragma unroll
-    for (int o = 2; o <= H; ++o) acc += sc.c[o - 1] * (fa(k + o) - fa(k - o));
-    return acc;
-  }
-  return d_line<ORD, T>(k, n, fa) * s;
+  for (int o = 2; o <= Ord<ORD>::H; ++o) s += T(d_coef<ORD>(o) / d_coef<ORD>(1)) * dif(o);
+  return s;
+}
+template <int ORD, class T, class F>
+__device__ __forceinline__ T d_scaled(const T (&c)[3], F dif) {
+  T s = c[0] * dif(1);
+#pragma unroll
+  for (int o = 2; o <= Ord<ORD>::H; ++o) s += c[o - 1] * dif(o);
+  return s;
 }
 
-// ---------------------------------------------------------------------------
-// Fused stage kernel.  One CTA = one work unit (panel strip x row segment);
-// thread t owns column cl0+t.  Rows stream through shared-memory rings of
-// the derived fields (KE, u and J h vt for 2*RMAX+1 rows; v, J h ut, ut, vt
-// and J for RMAX+1 rows), so every input node is read from global memory
-// once per unit.
-// ---------------------------------------------------------------------------
-template <class T, int ORD>
-__global__ void __launch_bounds__(STAGE_BW)
-    stage_kernel(InstDev<T> one, const InstDev<T>* many, const WorkUnit* units, int mode) {
-  constexpr int RMAX = Ord<ORD>::RMAX, RB = 2 * RMAX + 1, RX1 = RMAX + 1, NE = Ord<ORD>::NE;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T(*yring)[RY_N][STAGE_BW] = reinterpret_cast<T(*)[RY_N][STAGE_BW]>(smem_raw);
-  T(*xring)[RX_N][STAGE_BW] =
-      reinterpret_cast<T(*)[RX_N][STAGE_BW]>(smem_raw + sizeof(T) * RB * RY_N * STAGE_BW);
-
-  const WorkUnit wu = units[blockIdx.x];
-  const InstDev<T>& I = many ? many[wu.inst] : one;
+template <class T, int ORD, int MODE>
+__global__ void __launch_bounds__(PT_TPB)
+    point_stage_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many) {
+  constexpr int NE = Ord<ORD>::NE;
+  constexpr bool needB = MODE == MODE_RK1 || MODE == MODE_RK2 || MODE == MODE_RK3;
+  constexpr bool needA = MODE == MODE_RK2 || MODE == MODE_RK3 || MODE == MODE_RK4;
+  const InstDev<T>& I = many ? many[blockIdx.y] : one;
   const int n = I.n, P = I.P;
-  const long long pbase = (long long)wu.panel * I.ps;
-  const long long fs = I.fs;
-  const int t = threadIdx.x;
-  const int col = wu.cl0 + t;
-  const bool load_col = col < wu.cl1;
-  const T grav = I.grav;
-  static_assert(sizeof(T) == 8, "the FP32 form runs the TMA kernel");
-  const T ghs = I.ghs;
-  const ScaledInterior<ORD, T> ghs_c = scaled_interior<ORD, T>(ghs);
-
-  auto load_row = [&](int r) {
-    if (!load_col) return;
-    const long long idx = pbase + (long long)r * P + col;
-    const T h = I.in[idx], u = I.in[fs + idx], v = I.in[2 * fs + idx];
-    const T J = I.metric[MJ * fs + idx];
-    const T q1 = I.metric[MQI1 * fs + idx], q2 = I.metric[MQI2 * fs + idx],
-            q3 = I.metric[MQI3 * fs + idx];
-    const T ut = q1 * u + q2 * v;
-    const T vt = q2 * u + q3 * v;
-    T ke = (u * ut + v * vt) / T(2.0);
-    ke = ke + grav * h;
-    if (I.hs) ke = ke + grav * I.hs[idx];
-    // J ut and J vt serve the mass flux (times h) and the Coriolis term
-    const T jut = J * ut, jvt = J * vt;
-    const int s = r % RB, sx = r % RX1;
-    yring[s][RY_KE][t] = ke;
-    yring[s][RY_U][t] = u;
-    yring[s][RY_GV][t] = h * jvt;
-    xring[sx][RX_V][t] = v;
-    xring[sx][RX_GU][t] = h * jut;
-    xring[sx][RX_JUT][t] = jut;
-    xring[sx][RX_JVT][t] = jvt;
-  };
-
-  int loaded = wu.rl0;
-  {
-    const int target = min((int)wu.rl1, wu.j0 + RMAX + 1);
-    for (; loaded < target; ++loaded) load_row(loaded);
+  int p, i, j;
+  if (!point_node<ORD>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
+  const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
+  const T* __restrict__ K = I.der + DR_K2 * fs + x;
+  const T* __restrict__ GU = I.der + DR_GU * fs + x;
+  const T* __restrict__ GV = I.der + DR_GV * fs + x;
+  const T* __restrict__ U = I.in + fs + x;
+  const T* __restrict__ V = I.in + 2 * fs + x;
+  T rb[3] = {}, ra[3] = {}, rl[3] = {};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (needB) rb[c] = I.base[c * fs + x];
+    if (needA) ra[c] = I.acc ? I.acc[c * fs + x] : T(0);
   }
-  for (int j = wu.j0; j < wu.j1; ++j) {
-    if (j > wu.j0) {
-      __syncthreads();
-      const int target = min((int)wu.rl1, j + RMAX + 1);
-      for (; loaded < target; ++loaded) load_row(loaded);
-    }
-    __syncthreads();
-    if (col < wu.i0 || col >= wu.i1) continue;
-    const int sj = j % RB, sxj = j % RX1;
-    // x derivatives (along the row, neighbours are other threads' columns).
-    // For the 4/2 and 4/3 stencils the KE gradient's 1/(hx a) rides in the
-    // interior coefficients (measured on GB300: 2.8% faster FP64 steps at
-    // N=384 d42); for 6/3 that form measured 5% slower at N=1024, so it
-    // scales the derivative.
-    constexpr bool kScaledGrad = Ord<ORD>::H <= 2;
-    auto grad_ke = [&](int k, auto fa) {
-      if constexpr (kScaledGrad) return d_line_scaled<ORD, T>(k, n, fa, ghs_c, ghs);
-      else return d_line<ORD, T>(k, n, fa) * ghs;
-    };
-    const T gx = grad_ke(col, [&](int m) { return yring[sj][RY_KE][m - wu.cl0]; });
-    const T dxv = d_line<ORD, T>(col, n, [&](int m) { return xring[sxj][RX_V][m - wu.cl0]; });
-    const T dxgu = d_line<ORD, T>(col, n, [&](int m) { return xring[sxj][RX_GU][m - wu.cl0]; });
-    // y derivatives (along this thread's column)
-    auto ya = [&](int f) {
-      return d_line<ORD, T>(j, n, [&](int m) { return yring[m % RB][f][t]; });
-    };
-    const T gy = grad_ke(j, [&](int m) { return yring[m % RB][RY_KE][t]; });
-    const T dyu = ya(RY_U), dygv = ya(RY_GV);
-    const T rJ = I.metric[MRJ * fs + pbase + (long long)j * P + col];
-    const T zeta = (dxv - dyu) * rJ;
-    const T dv = (dxgu + dygv) * rJ;
-    const long long idx = pbase + (long long)j * P + col;
-    const bool bnd = (col == 0) | (col == n - 1) | (j == 0) | (j == n - 1);
-    if (bnd) {
-      T* E = I.edge + (long long)wu.panel * 16 * n;
-      // the four values one by one (an array of them was kept in local memory
-      // for every node, boundary or not)
+  T rJ = I.metric[MRJ * fs + x];
+  const T f = I.metric[MF * fs + x];
+  const T jut = I.der[DR_JUT * fs + x], jvt = I.der[DR_JVT * fs + x];
+  T gx, gy, zw, dw;   // zw, dw: the curl and the divergence before the factor rJ
+  const bool xin = i >= NE && i < n - NE, yin = j >= NE && j < n - NE;
+  if (xin && yin) {
+    gx = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o] - K[-o]; });
+    gy = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o * P] - K[-o * P]; });
+    zw = d_ratio<ORD, T>([&](int o) { return (V[o] - V[-o]) - (U[o * P] - U[-o * P]); });
+    dw = d_ratio<ORD, T>([&](int o) { return (GU[o] - GU[-o]) + (GV[o * P] - GV[-o * P]); });
+    rJ = rJ * T(d_coef<ORD>(1));
+  } else {
+    auto dx = [&](const T* q) { return d_line<ORD, T>(i, n, [&](int m) { return q[m - i]; }); };
+    auto dy = [&](const T* q) { return d_line<ORD, T>(j, n, [&](int m) { return q[(m - j) * P]; }); };
+    gx = dx(K) * I.ghs2;
+    gy = dy(K) * I.ghs2;
+    zw = dx(V) - dy(U);
+    dw = dx(GU) + dy(GV);
+    if (i == 0 || i == n - 1 || j == 0 || j == n - 1) {
+      const T zeta = zw * rJ, dv = dw * rJ;
+      T* E = I.edge + (long long)p * 16 * n;
       auto put = [&](int side, int k) {
         T* e = E + (side * 4) * n + k;
         e[0] = gx; e[n] = gy; e[2 * n] = zeta; e[3 * n] = dv;
       };
-      if (col == 0) put(SIDE_L, j);
-      if (col == n - 1) put(SIDE_R, j);
-      if (j == 0) put(SIDE_B, col);
-      if (j == n - 1) put(SIDE_T, col);
-      continue;
+      if (i == 0) put(SIDE_L, j);
+      if (i == n - 1) put(SIDE_R, j);
+      if (j == 0) put(SIDE_B, i);
+      if (j == n - 1) put(SIDE_T, i);
+      return;
     }
-    const T f = I.metric[MF * fs + idx];
-    T kh, ku, kv;
-    node_tendency_j<T>(gx, gy, zeta, dv, f, xring[sxj][RX_JUT][t], xring[sxj][RX_JVT][t], kh, ku, kv);
-    stage_epilogue<T>(I, mode, idx, kh, ku, kv);
   }
-  (void)NE;
+  const T fz = f + zw * rJ;
+  T y[3];
+  stage_epilogue_pre<T>(I, MODE, x, -(dw * rJ), fz * jvt - gx, -(fz * jut) - gy, rb, ra, rl, y);
+  if (needB && I.der_out)
+    derive_store<T>(I.der_out, fs, x, y[0], y[1], y[2], I.metric[MJ * fs + x], I.metric[MQI1 * fs + x],
+                    I.metric[MQI2 * fs + x], I.metric[MQI3 * fs + x], I.grav2, I.hs);
 }
 
-template <class T, int ORD>
-constexpr size_t stage_smem_bytes() {
-  return sizeof(T) * ((2 * Ord<ORD>::RMAX + 1) * RY_N + (Ord<ORD>::RMAX + 1) * RX_N) * STAGE_BW;
+// Stencil inputs of I.in, then (launch_point_stage) one stage from them, over
+// ninst instances whose largest edge has max_n nodes.
+template <class T>
+cudaError_t launch_point_derive(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,
+                                cudaStream_t st) {
+  point_derive_kernel<T><<<dim3((6 * max_n * max_n + PT_TPB - 1) / PT_TPB, ninst), PT_TPB, 0, st>>>(one, many);
+  return cudaGetLastError();
 }
-
 template <class T, int ORD>
-cudaError_t launch_stage_ord(const InstDev<T>& one, const InstDev<T>* many, const WorkUnit* units,
-                             int nunits, int mode, cudaStream_t st) {
-  constexpr size_t smem = stage_smem_bytes<T, ORD>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(stage_kernel<T, ORD>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
+cudaError_t launch_point_stage_ord(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,
+                                   int mode, cudaStream_t st) {
+  const dim3 g((6 * max_n * max_n + PT_TPB - 1) / PT_TPB, ninst);
+  switch (mode) {
+    case MODE_APPLY: point_stage_kernel<T, ORD, MODE_APPLY><<<g, PT_TPB, 0, st>>>(one, many); break;
+    case MODE_RK1: point_stage_kernel<T, ORD, MODE_RK1><<<g, PT_TPB, 0, st>>>(one, many); break;
+    case MODE_RK2: point_stage_kernel<T, ORD, MODE_RK2><<<g, PT_TPB, 0, st>>>(one, many); break;
+    case MODE_RK3: point_stage_kernel<T, ORD, MODE_RK3><<<g, PT_TPB, 0, st>>>(one, many); break;
+    case MODE_RK4: point_stage_kernel<T, ORD, MODE_RK4><<<g, PT_TPB, 0, st>>>(one, many); break;
+    default: return cudaErrorInvalidValue;
   }
-  if (nunits <= 0) return cudaSuccess;
-  stage_kernel<T, ORD><<<nunits, STAGE_BW, smem, st>>>(one, many, units, mode);
   return cudaGetLastError();
 }
 
@@ -519,7 +467,7 @@ __global__ void edge_kernel(InstDev<T> one, const InstDev<T>* many, Topology tp,
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     rb[c] = needB ? bsrc[c * fs + idx] : T(0);
-    ra[c] = needA ? I.acc[c * fs + idx] : T(0);
+    ra[c] = needA && I.acc ? I.acc[c * fs + idx] : T(0);
     rlo[c] = needL ? I.base_lo[c * fs + idx] : T(0);
   }
 
@@ -554,7 +502,11 @@ __global__ void edge_kernel(InstDev<T> one, const InstDev<T>* many, Topology tp,
   const T ut = q1 * u + q2 * v, vt = q2 * u + q3 * v;
   T kh, ku, kv;
   node_tendency<T>(gx, gy, zeta, dv, f, J, ut, vt, kh, ku, kv);
-  stage_epilogue_pre<T>(I, mode, idx, kh, ku, kv, rb, ra, rlo);
+  T y[3] = {};
+  stage_epilogue_pre<T>(I, mode, idx, kh, ku, kv, rb, ra, rlo, y);
+  if constexpr (sizeof(T) == 8)
+    if (mode != MODE_APPLY && mode != MODE_RK4 && I.der_out)
+      derive_store<T>(I.der_out, fs, idx, y[0], y[1], y[2], J, q1, q2, q3, I.grav2, I.hs);
 }
 
 }  // namespace swm

@@ -46,6 +46,41 @@ def test_apply_fp64_matches_oracle(cfg1, fused):
         assert rel_l2(a, b, J) < TOL_TENDENCY
 
 
+# The FP64 stage kernel numbers the closure columns first and the other nodes
+# after them: the smallest panel (5 inner columns for 6/3), panels around a
+# whole number of warps, with orography, as a tendency and through the stage
+# chain of two steps, whose stencil inputs pass from stage to stage.
+@pytest.mark.parametrize("order,N", [(42, 16), (43, 17), (63, 16), (42, 39), (63, 44), (42, 103)])
+def test_fp64_stage_matches_unfused_operators(order, N):
+    h, u, v, _ = initial.balanced_zonal(N, 5, 8)
+    geo = initial.ecs_geometry(N)
+    hs = 100.0 * geo["r"][..., 0] ** 2
+    op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=order))
+    op.set_orography(hs)
+    J = geo["J"]
+    x = _state(op, h, u, v)
+    want, got = x.create_similar(), x.create_similar()
+    op.apply_unfused(want, x)
+    op.apply(got, x)
+    for a, b in zip(got.download(), want.download()):
+        assert rel_l2(a, b, J) < TOL_TENDENCY
+    dt = 300.0 * 48 / N
+    ref, y, k, w = (x.create_similar() for _ in range(4))
+    ref.assign_s1v1(1.0, x)
+    for _ in range(2):
+        w.assign_s1v1(1.0, ref)
+        y.assign_s1v1(1.0, ref)
+        for c_in, c_acc in ((0.5, 1 / 6), (0.5, 1 / 3), (1.0, 1 / 3), (None, 1 / 6)):
+            op.apply_unfused(k, y)
+            w.update_s1v1(c_acc * dt, k)
+            if c_in:
+                y.assign_s1v1s2v2(1.0, ref, c_in * dt, k)
+        ref.assign_s1v1(1.0, w)
+    swm.RK4().step(x, op, dt, 2)
+    for a, b in zip(x.download(), ref.download()):
+        assert rel_l2(a, b, J) < 2 * TOL_STEP
+
+
 @pytest.mark.parametrize("order,N", [(43, 40), (63, 48)])
 def test_apply_other_orders_match_oracle(order, N):
     h, u, v, _ = initial.balanced_zonal(N, 9, 16)
