@@ -810,7 +810,7 @@ def diffusion_leg(w, h, u, v, local, steps, warmup):
 #   plus the stage epilogues of the three state components (2, 4, 2 and 3
 #   words in stages 1..4): 4 x 46 + 3 x 11 = 217 words per point and step.
 CGRID_WORDS_PER_POINT_STEP = 217
-CGRID_LAUNCHES_PER_STEP = 24          # 4 x 6 passes (the curl's corner sync rides in w2uv's reads)
+CGRID_LAUNCHES_PER_STEP = 16          # 4 x 4 passes (the curl's corner sync rides in the reads of the second)
 # The namelist's C-grid model step adds one explicit Euler step of the
 # hyperdiffusion (hordiff_c_biharm_curl_div, hordiff_scalar_C; 2/1
 # operators).  Words per point of its passes, inputs + outputs + metric:

@@ -4,19 +4,19 @@
 // epilogue, the SBP_C quadrature, the hyperdiffusion and the ECS halos of the
 // cell centres.
 //
-// One right-hand side (operator_swm_mod.f90:61-113 with the C-grid operators)
-// is six passes over the panels:
+// The fused right-hand side and its RK4 epilogue are in swm_cgrid_rhs.cuh; the
+// passes here serve the unfused operators and the hyperdiffusion:
 //   centre_a  p points   J Qi12 times the other covariant component
 //                        interpolated to the centres (co2contra, first half)
-//   faces_a   u, v       contravariant components, mass fluxes h*u^i, J*flux
-//                        and the kinetic-energy densities J u u^i / 2
+//   faces_a   u, v       contravariant components, mass fluxes h*u^i, J*flux,
+//                        kinetic-energy densities J u u^i / 2
 //   curl      q points   staggered differences + SAT penalties
-//   w2uv      u          the curl, with its Ah-type edge / corner average
-//                        taken as it is read, interpolated to the x-faces
-//   centre_b  p points   kinetic energy + g (h + hs), the divergence with its
-//                        SAT penalties (h tendency), the Coriolis terms
-//   faces_b   u, v       gradient with its SAT penalties + the Coriolis term
-//                        interpolated back (u, v tendencies)
+//   w2uv      u          the curl interpolated to the x-faces
+//   centre_b  p points   kinetic energy, divergence with its SAT penalties,
+//                        Coriolis terms
+//   faces_b   u, v       gradient with its SAT penalties, or the Coriolis
+//                        terms interpolated back
+//   gperp     u, v       grad_perp
 // The neighbours' points the SBP-SAT operators read across a panel edge come
 // straight from the neighbouring panel through a precomputed table (one GPU
 // holds all six panels, so the reference's halo exchange becomes an indexed
@@ -28,6 +28,7 @@
 #include <cmath>
 #include <cstdint>
 #include <initializer_list>
+#include <type_traits>
 #include <vector>
 
 namespace swm {
@@ -145,31 +146,29 @@ void fill_ops(int order, COps& o) {
 // GB300's FP64 pipe is narrow, so the divisions of the operators are taken
 // once on the host: reciprocal fields 1/J and 1/(J hx a), and J Qi12.  The
 // covariant metric (J Q12, Q11, Q22) and 1/(J hx a) on the faces serve the
-// contra2co transform and grad_perp of the hyperdiffusion.
+// contra2co transform and grad_perp of the hyperdiffusion.  The M_S* fields are
+// 1/J (faces), 1/(J hx a) (corners), 1/(2J) and 1/(J hx a) (centres) times the
+// stencil scales of the context's order (swm_cgrid_rhs.cuh).
 enum { M_JP = 0, M_QI2P, M_FP, M_RJP, M_RJPHA, M_JQI2P,  // centres
        M_JU, M_QI1U, M_RJU,                              // x-faces
        M_JV, M_QI3V, M_RJV,                              // y-faces
        M_JQ, M_RJQHA,                                    // corners
        M_JQ2P, M_Q1U, M_Q3V, M_RJUHA, M_RJVHA,           // covariant metric, face 1/(J hx a)
+       M_SJU, M_SJV, M_SJQ, M_SJP, M_SDIV,               // the fused passes' scaled fields
        M_COUNT };
-constexpr int kMetricMesh[M_COUNT] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 0, 1, 2, 1, 2};
+constexpr int kMetricMesh[M_COUNT] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 0, 1, 2, 1, 2, 1, 2, 3, 0, 0};
 enum { W_AP = 0, W_BP, W_UT, W_VT, W_HU, W_HV, W_GU, W_GV, W_KEU, W_KEV, W_CURL, W_FU, W_KE,
        W_CUP, W_CVP, W_COUNT };
 
 // kernel flags
 enum : int {
-  F_CO = 1,        // faces_a: contravariant components from the covariant ones
-  F_MF = 2,        // faces_a: mass fluxes
-  F_G = 4,         // faces_a: J * mass flux
-  F_KE = 8,        // faces_a: kinetic-energy densities; centre_b: kinetic energy
-  F_ADDGH = 16,    // centre_b: + g h + g hs
-  F_DIV = 32,      // centre_b: divergence
-  F_COR = 64,      // centre_b: Coriolis terms at the centres; faces_b: back to the faces
-  F_GRAD = 128,    // faces_b: gradient
-  F_SEP = 256,     // centre_b / faces_b: write the operator's own output, not a tendency
-  F_WUT = 512,     // faces_a: store the contravariant components (unfused co2contra)
-  F_WFLUX = 1024,  // faces_a: store the mass fluxes (unfused massflux; the 2/1 divergence)
-  F_QSYNC = 2048,  // w2uv: the curl is unsynced; average its edge and corner copies as it is read
+  F_CO = 1,    // faces_a: contravariant components from the covariant ones
+  F_MF = 2,    // faces_a: mass fluxes
+  F_G = 4,     // faces_a: J * mass flux
+  F_KE = 8,    // faces_a: kinetic-energy densities; centre_b: kinetic energy
+  F_DIV = 16,  // centre_b: divergence
+  F_COR = 32,  // centre_b: Coriolis terms at the centres; faces_b: back to the faces
+  F_GRAD = 64, // faces_b: gradient
 };
 
 template <class T>
@@ -198,13 +197,7 @@ struct CArgsT {
   const T *h, *u, *v, *hs, *ut_in, *vt_in, *hu_in, *hv_in, *ke_in, *curl_in;
   // intermediate and unfused outputs
   T *Ap, *Bp, *ut, *vt, *hu, *hv, *Gu, *Gv, *KEu, *KEv, *curl, *fu, *KE, *cup, *cvp;
-  T *o1, *o2;  // unfused outputs of centre_b (div) / faces_b (gx|cor_u, gy|cor_v)
-  // RK4 stage epilogue: mode 0 writes the tendency to tend, 1..4 the stages
-  // of rk4_mod.f90:20-42 (y0, Y, Kb, acc: 3 fields each, fs apart; FP32:
-  // y0 / lo the state pair, acc the running increment, no Kb)
-  int mode;
-  T hdt, dt, c3, c6;
-  T *tend, *y0, *Y, *Kb, *acc, *lo;
+  T *o1, *o2;  // outputs of centre_b (div) / faces_b (gx|cor_u, gy|cor_v)
 };
 
 // element offset within a field (fields stay below 2^31 elements)
@@ -257,42 +250,6 @@ __device__ __forceinline__ T halo_at(const CArgsT<T>& a, int mesh, int side, int
   return (c & 1) ? -x : x;
 }
 
-template <class T>
-__device__ __forceinline__ void rk_put(const CArgsT<T>& a, int comp, int e, T k) {
-  const int o = comp * (int)a.g.fs + e;
-  if constexpr (sizeof(T) == 8) {
-    // FP64: the reference's order, y = 1*y0 + c k and
-    // y0 = (y0 + dt/6 k1 + dt/3 k2) + dt/3 k3 + dt/6 k4
-    switch (a.mode) {
-      case 0: a.tend[o] = k; break;
-      case 1: a.Kb[o] = k; a.Y[o] = T(1.0) * a.y0[o] + a.hdt * k; break;
-      case 2: a.acc[o] = (a.y0[o] + a.c6 * a.Kb[o]) + a.c3 * k; a.Y[o] = T(1.0) * a.y0[o] + a.hdt * k; break;
-      case 3: a.Kb[o] = k; a.Y[o] = T(1.0) * a.y0[o] + a.dt * k; break;
-      default: a.y0[o] = (a.acc[o] + a.c3 * a.Kb[o]) + a.c6 * k; break;
-    }
-  } else {
-    // FP32 compensated form (as on the Ah grid): the stage increments add up
-    // apart from the state, and the last stage adds them to the (hi, lo)
-    // state pair with an exact two-sum
-    switch (a.mode) {
-      case 0: a.tend[o] = k; break;
-      case 1: a.Y[o] = a.y0[o] + a.hdt * k; a.acc[o] = a.c6 * k; break;
-      case 2: a.Y[o] = a.y0[o] + a.hdt * k; a.acc[o] = a.acc[o] + a.c3 * k; break;
-      case 3: a.Y[o] = a.y0[o] + a.dt * k; a.acc[o] = a.acc[o] + a.c3 * k; break;
-      default: {
-        const T d = a.acc[o] + a.c6 * k;
-        const T hi = a.y0[o], lo = a.lo[o];
-        const T t = lo + d;
-        const T s = hi + t;
-        const T bb = s - hi;
-        a.y0[o] = s;
-        a.lo[o] = (hi - (s - bb)) + (t - bb);
-        break;
-      }
-    }
-  }
-}
-
 #define SWM_C_INDEX(nx_, ny_)                                  \
   const int i = blockIdx.x * blockDim.x + threadIdx.x;        \
   const int j = blockIdx.y * blockDim.y + threadIdx.y;        \
@@ -328,14 +285,12 @@ __global__ void __launch_bounds__(256) faces_a_kernel(const __grid_constant__ CA
     if (a.flags & F_CO) {
       const T t = stag_at<W, T>(a.ops.wc2i, a.Ap + at(g, p, 0, j), 1, N + 1, i);
       ut = a.Qi1u[e] * a.u[e] + t * a.rJu[e];
-      if (a.flags & F_WUT) a.ut[e] = ut;
+      a.ut[e] = ut;
     } else {
       ut = a.ut_in ? a.ut_in[e] : T(0.0);
     }
     if (a.flags & F_MF) {
-      const T hu = ut * stag_at<W, T>(a.ops.wc2i, a.h + at(g, p, 0, j), 1, N + 1, i);
-      if (a.flags & F_WFLUX) a.hu[e] = hu;
-      if (a.flags & F_G) a.Gu[e] = hu * a.Ju[e];
+      a.hu[e] = ut * stag_at<W, T>(a.ops.wc2i, a.h + at(g, p, 0, j), 1, N + 1, i);
     } else if (a.flags & F_G) {
       a.Gu[e] = a.hu_in[e] * a.Ju[e];
     }
@@ -346,14 +301,12 @@ __global__ void __launch_bounds__(256) faces_a_kernel(const __grid_constant__ CA
     if (a.flags & F_CO) {
       const T t = stag_at<W, T>(a.ops.wc2i, a.Bp + at(g, p, i, 0), g.P, N + 1, j);
       vt = a.Qi3v[e] * a.v[e] + t * a.rJv[e];
-      if (a.flags & F_WUT) a.vt[e] = vt;
+      a.vt[e] = vt;
     } else {
       vt = a.vt_in ? a.vt_in[e] : T(0.0);
     }
     if (a.flags & F_MF) {
-      const T hv = vt * stag_at<W, T>(a.ops.wc2i, a.h + at(g, p, i, 0), g.P, N + 1, j);
-      if (a.flags & F_WFLUX) a.hv[e] = hv;
-      if (a.flags & F_G) a.Gv[e] = hv * a.Jv[e];
+      a.hv[e] = vt * stag_at<W, T>(a.ops.wc2i, a.h + at(g, p, i, 0), g.P, N + 1, j);
     } else if (a.flags & F_G) {
       a.Gv[e] = a.hv_in[e] * a.Jv[e];
     }
@@ -405,41 +358,13 @@ __global__ void __launch_bounds__(256) curl_kernel(const __grid_constant__ CArgs
 // tensor-product interpolations to the centres, x after y and y after x;
 // the 1-D operators act on different indices, so both are the same linear
 // map and one of them is evaluated (the results agree to round-off).
-//
-// With F_QSYNC the curl comes straight from curl_kernel, unsynced, and its
-// edge and corner points are averaged with the neighbours' copies here, as
-// they are read: the Ah-type sync of the corner mesh
-// (halo/halo_Ah_scalar_sync_mod.f90:38-93, in the order of the sync kernel),
-// with the copies from the corner mesh's cross-halo table.  That saves the
-// sync's two launches per stage in the fused step, where this pass is the
-// curl's only reader.
-template <class T>
-__device__ __forceinline__ T curl_synced(const CArgsT<T>& a, int p, int i, int j) {
-  const int N = a.N;
-  const T* c = a.curl_in;
-  const T own = c[at(a.g, p, i, j)];
-  if (i > 0 && i < N && j > 0 && j < N) return own;
-  auto H = [&](int side, int k) { return halo_at(a, 3, side, p, 1, k, c, c); };
-  if (i == 0 && j == 0) return (own + H(0, 0) + H(2, 0)) / T(3.0);
-  if (i == N && j == 0) return (own + H(1, 0) + H(2, N)) / T(3.0);
-  if (i == 0 && j == N) return (own + H(0, N) + H(3, 0)) / T(3.0);
-  if (i == N && j == N) return (own + H(1, N) + H(3, N)) / T(3.0);
-  if (i == 0) return T(0.5) * (H(0, j) + own);
-  if (i == N) return T(0.5) * (own + H(1, j));
-  if (j == 0) return T(0.5) * (own + H(2, i));
-  return T(0.5) * (own + H(3, i));
-}
-
 template <int ORD, class T>
 __global__ void __launch_bounds__(256) w2uv_kernel(const __grid_constant__ CArgsT<T> a) {
   constexpr int W = ORD == 42 ? 4 : 2;
   const int N = a.N;
   SWM_C_INDEX(N + 1, N)
   const FieldGeom& g = a.g;
-  if (a.flags & F_QSYNC)
-    a.fu[at(g, p, i, j)] = stag_at_f<W, T>(a.ops.wi2c, [&](int m) { return curl_synced(a, p, i, m); }, N, j);
-  else
-    a.fu[at(g, p, i, j)] = stag_at<W, T>(a.ops.wi2c, a.curl_in + at(g, p, i, 0), g.P, N, j);
+  a.fu[at(g, p, i, j)] = stag_at<W, T>(a.ops.wi2c, a.curl_in + at(g, p, i, 0), g.P, N, j);
 }
 
 // grad_perp_c_sbp (grad_perp/grad_perp_c_sbp_mod.f90:20-95): the staggered
@@ -870,8 +795,7 @@ __global__ void __launch_bounds__(256) laplace_ch_kernel(const __grid_constant__
   out[at(a.g, p, i, j)] = v;
 }
 
-// Centre pass: the kinetic energy (KE_Cgrid_mod.f90:60-75) plus g (h + hs)
-// (operator_swm_mod.f90:84-85), the divergence (div_c_sbp42_mod.f90:67-107,
+// Centre pass: the kinetic energy (KE_Cgrid_mod.f90:60-75), the divergence (div_c_sbp42_mod.f90:67-107,
 // div_c2_mod.f90:97-177) and the Coriolis terms at the centres
 // (coriolis_Cgrid_mod.f90:98-118).
 template <int ORD, class T>
@@ -883,14 +807,8 @@ __global__ void __launch_bounds__(256) centre_b_kernel(const __grid_constant__ C
   const COpsT<T>& o = a.ops;
   const int e = at(g, p, i, j);
   const int row = at(g, p, 0, j), col = at(g, p, i, 0);
-  // h of this point, read before the RK epilogue of stages 2 and 3 writes
-  // the new h in place over it
-  const T hh = (a.flags & (F_ADDGH | F_COR)) ? a.h[e] : T(0.0);
-  if (a.flags & F_KE) {
-    T ke = (stag_at<W, T>(o.wi2c, a.KEu + row, 1, N, i) + stag_at<W, T>(o.wi2c, a.KEv + col, g.P, N, j)) * a.rJp[e];
-    if (a.flags & F_ADDGH) ke = ke + a.grav * hh + a.grav * (a.hs ? a.hs[e] : T(0.0));
-    a.KE[e] = ke;
-  }
+  if (a.flags & F_KE)
+    a.KE[e] = (stag_at<W, T>(o.wi2c, a.KEu + row, 1, N, i) + stag_at<W, T>(o.wi2c, a.KEv + col, g.P, N, j)) * a.rJp[e];
   if (a.flags & F_DIV) {
     T dx, dy;
     if (ORD == 21) {
@@ -923,15 +841,13 @@ __global__ void __launch_bounds__(256) centre_b_kernel(const __grid_constant__ C
       if (j >= N - o.np)
         dy = dy + T(0.5) * o.pen_c[N - 1 - j] * (halo_at(a, 2, 3, p, 1, i, gv, gu) - gv[col + N * g.P]);
     }
-    const T dv = (dx + dy) * a.rJpha[e];
-    if (a.flags & F_SEP) a.o1[e] = dv;
-    else rk_put(a, 0, e, -T(1.0) * dv);
+    a.o1[e] = (dx + dy) * a.rJpha[e];
   }
   if (a.flags & F_COR) {
     const T gup = stag_at<W, T>(o.wi2c, a.Gu + row, 1, N, i);
     const T gvp = stag_at<W, T>(o.wi2c, a.Gv + col, g.P, N, j);
     const T cp = stag_at<W, T>(o.wi2c, a.fu + row, 1, N, i);  // the curl at the centre
-    const T q = (a.fp[e] + cp) / hh;  // one division per point
+    const T q = (a.fp[e] + cp) / a.h[e];  // one division per point
     a.cup[e] = q * gvp;
     a.cvp[e] = -q * gup;
   }
@@ -940,8 +856,8 @@ __global__ void __launch_bounds__(256) centre_b_kernel(const __grid_constant__ C
 // covariant gradient of the centre field f at face i (gradient_c_sbp42,
 // grad_c_sbp42_mod.f90:44-139; gradient_c_sbp21, grad_c2_ecs_mod.f90:234-293)
 // along a line: F(k) for 0 <= k < N from the panel, else the o halo.
-template <int ORD, class T, class Fn>
-__device__ __forceinline__ T grad_line(const CArgsT<T>& a, int N, int i, Fn F) {
+template <int ORD, class T, class A, class Fn>
+__device__ __forceinline__ T grad_line(const A& a, int N, int i, Fn F) {
   const COpsT<T>& o = a.ops;
   if (ORD == 21) {
     const T dx1 = a.dx1;
@@ -1000,9 +916,8 @@ __device__ __forceinline__ T grad_in(const CArgsT<T>& a, const T* __restrict__ f
   return s * a.dx1;
 }
 
-// Face pass: the gradient of the kinetic energy and the Coriolis term
-// interpolated from the centres (interpolator_p2uv_mod.f90:98-115), combined
-// into the u, v tendencies (operator_swm_mod.f90:95-96).
+// Face pass: the gradient of a centre field, or the Coriolis terms
+// interpolated from the centres (interpolator_p2uv_mod.f90:98-115).
 template <int ORD, class T>
 __global__ void __launch_bounds__(256) faces_b_kernel(const __grid_constant__ CArgsT<T> a) {
   constexpr int W = ORD == 42 ? 4 : 2;
@@ -1023,8 +938,7 @@ __global__ void __launch_bounds__(256) faces_b_kernel(const __grid_constant__ CA
         });
     }
     if (a.flags & F_COR) cu = stag_at<W, T>(a.ops.wc2i, a.cup + at(g, p, 0, j), 1, N + 1, i);
-    if (a.flags & F_SEP) a.o1[e] = (a.flags & F_GRAD) ? gx : cu;
-    else rk_put(a, 1, e, -T(1.0) * gx + T(1.0) * cu);
+    a.o1[e] = (a.flags & F_GRAD) ? gx : cu;
   }
   if (i < N) {  // v point
     T gy = T(0.0), cv = T(0.0);
@@ -1039,8 +953,7 @@ __global__ void __launch_bounds__(256) faces_b_kernel(const __grid_constant__ CA
         });
     }
     if (a.flags & F_COR) cv = stag_at<W, T>(a.ops.wc2i, a.cvp + at(g, p, i, 0), g.P, N + 1, j);
-    if (a.flags & F_SEP) a.o2[e] = (a.flags & F_GRAD) ? gy : cv;
-    else rk_put(a, 2, e, -T(1.0) * gy + T(1.0) * cv);
+    a.o2[e] = (a.flags & F_GRAD) ? gy : cv;
   }
 }
 
@@ -1100,6 +1013,8 @@ __global__ void cpack_kernel(FieldGeom g, int nx, int ny, const double* __restri
   dst[k] = lo ? (double)hi[e] + (double)lo[e] : d64[e];
 }
 
+#include "swm_cgrid_rhs.cuh"
+
 __global__ void mass_final_kernel(const double* part, int n, double* out) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
@@ -1118,6 +1033,7 @@ struct CGrid {
   COpsT<float> ops32{};
   COps ops21{};             // the 2/1 operators of the hyperdiffusion (any order)
   COpsT<float> ops21_32{};
+  ScaledOps<double> sops{};        // the fused FP64 passes' operators
   double* met = nullptr;   // M_COUNT fields
   float* met32 = nullptr;  // their FP32 copies (contexts of the FP32 form)
   double* wk = nullptr;    // W_COUNT fields
@@ -1209,25 +1125,47 @@ SWM_C_LAUNCH(run_gperp, gperp_kernel, c->N + 1, c->N + 1)
     if (e_ != cudaSuccess) return e_;           \
   } while (0)
 
-// One right-hand side of the state (h, u, v) with the epilogue of a.mode.
+// Arguments of the fused right-hand side in precision T.
 template <class T>
-cudaError_t rhs(const CGrid* c, CArgsT<T> a, const T* in, cudaStream_t st) {
+RhsArgs<T> rhs_args(const CGrid* c) {
+  RhsArgs<T> a{};
+  a.g = c->g; a.N = c->N; a.L = c->L;
+  a.halo = c->halo;
+  auto M = [&](int k) { return metric_t<T>(c, k); };
+  a.jq = M(M_JQI2P); a.fp = M(M_FP); a.Ju = M(M_JU); a.Jv = M(M_JV);
+  a.Qi1u = M(M_QI1U); a.Qi3v = M(M_QI3V);
+  if constexpr (sizeof(T) == 8) {
+    a.ops = c->sops;
+    a.sju = M(M_SJU); a.sjv = M(M_SJV); a.sjq = M(M_SJQ); a.sjp = M(M_SJP); a.sdiv = M(M_SDIV);
+  } else {
+    a.ops = c->ops32;
+    a.sju = M(M_RJU); a.sjv = M(M_RJV); a.sjq = M(M_RJQHA); a.sjp = M(M_RJP); a.sdiv = M(M_RJPHA);
+  }
+  auto Wk = [&](int k) { return reinterpret_cast<T*>(c->work(k)); };
+  a.Ap = Wk(W_AP); a.Bp = Wk(W_BP); a.Gu = Wk(W_GU); a.Gv = Wk(W_GV);
+  a.KEu = Wk(W_KEU); a.KEv = Wk(W_KEV); a.curl = Wk(W_CURL); a.fu = Wk(W_FU); a.KE = Wk(W_KE);
+  a.cup = Wk(W_CUP); a.cvp = Wk(W_CVP); a.hu = Wk(W_HU); a.hv = Wk(W_HV);
+  a.dx1 = T(1.0 / (c->radius * c->hx));
+  const double w = scale_w(c->order), d = scale_d(c->order);
+  a.grav = T(c->grav);
+  a.cg = T(d / (c->radius * c->hx));
+  a.cw = T(w * w * w);   // of Gu (w), its interpolation (w) and the one back to the faces (w)
+  a.cw2 = T(w * w);      // of the curl's two interpolations
+  return a;
+}
+
+// One right-hand side of the state (h, u, v) at `in` with the epilogue of
+// mode (rhs1..rhs4).
+template <class T>
+cudaError_t rhs(const CGrid* c, RhsArgs<T> a, int mode, const T* in, cudaStream_t st) {
   const long long fs = c->g.fs;
+  const int N = c->N;
   a.h = in; a.u = in + fs; a.v = in + 2 * fs;
-  a.flags = F_CO | F_MF | F_G | F_KE | (c->order == 21 ? F_WFLUX : 0);
-  CKE(run_centre_a(c, a, st));
-  CKE(run_faces_a(c, a, st));
-  CKE(run_curl(c, a, st));
-  // the corner sync of the curl rides in w2uv's reads (its only reader here)
-  a.curl_in = a.curl;
-  a.flags = F_QSYNC;
-  CKE(run_w2uv(c, a, st));
-  a.hu_in = a.hu; a.hv_in = a.hv;
-  a.flags = F_KE | F_ADDGH | F_DIV | F_COR;
-  CKE(run_centre_b(c, a, st));
-  a.ke_in = a.KE;
-  a.flags = F_GRAD | F_COR;
-  return run_faces_b(c, a, st);
+  dim3 grid((N - 2 * kRhsEdge + kRhsX) / kRhsX, (N + kRhsY) / kRhsY, 6);
+  const int blocks = 6 * ((N + kRhsX) / kRhsX), slab = grid.x * grid.y;
+  a.strips = (blocks + slab - 1) / slab;
+  grid.z += a.strips;
+  return c->order == 42 ? rhs_passes<42, T>(a, mode, grid, st) : rhs_passes<21, T>(a, mode, grid, st);
 }
 
 // ------------------------------------------------------------------ host
@@ -1236,8 +1174,7 @@ cudaError_t rhs(const CGrid* c, CArgsT<T> a, const T* in, cudaStream_t st) {
 struct MetricAt {
   double J, qi1, qi2, qi3, q1, q2, q3;
 };
-MetricAt metric_at(double al, double be) {
-  const double ta = std::tan(al), tb = std::tan(be);
+MetricAt metric_of_tan(double ta, double tb) {
   const double sg = std::sqrt(1.0 + ta * ta + tb * tb);
   const double s4 = sg * sg * sg * sg;
   MetricAt m;
@@ -1252,8 +1189,10 @@ MetricAt metric_at(double al, double be) {
   return m;
 }
 
-double coriolis_at(int p, double al, double be, double omega, const double ax[3]) {
-  const double ta = std::tan(al), tb = std::tan(be);
+MetricAt metric_at(double al, double be) { return metric_of_tan(std::tan(al), std::tan(be)); }
+
+// at the point of panel p with the tangents ta, tb of its angles
+double coriolis_at(int p, double ta, double tb, double omega, const double ax[3]) {
   const double d = std::sqrt(1.0 + ta * ta + tb * tb);
   const double v[3] = {ta / d, tb / d, 1.0 / d};
   double w[3];
@@ -1334,7 +1273,7 @@ cudaError_t transform(const CGrid* c, CArgsT<T> a, const T* x, const T* y, T* xo
     a.Qi3v = metric_t<T>(c, M_Q3V);
   }
   a.u = x; a.v = y; a.ut = xo; a.vt = yo;
-  a.flags = F_CO | F_WUT;
+  a.flags = F_CO;
   CKE(run_centre_a(c, a, st));
   return run_faces_a(c, a, st);
 }
@@ -1380,13 +1319,13 @@ cudaError_t diffusion(const CGrid* c, const Topology& tp, T* edge, int parts, do
   auto div = [&](const Branch& B, const T* x, const T* y, T* o) {
     CArgsT<T> b = B.a;
     b.hu_in = x; b.hv_in = y; b.o1 = o;
-    b.flags = F_DIV | F_SEP;
+    b.flags = F_DIV;
     return run_centre_b(c, b, B.st);
   };
   auto grad = [&](const Branch& B, const T* f, T* gx, T* gy) {
     CArgsT<T> b = B.a;
     b.ke_in = f; b.o1 = gx; b.o2 = gy;
-    b.flags = F_GRAD | F_SEP;
+    b.flags = F_GRAD;
     return run_faces_b(c, b, B.st);
   };
   auto curl = [&](const Branch& B, const T* x, const T* y, T* q) {
@@ -1576,6 +1515,7 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
   c->radius = radius; c->grav = grav;
   fill_ops(order, c->ops);
   c->ops32 = ops_cast<float>(c->ops);
+  c->sops = scaled_ops<double>(c->ops, order);
   fill_ops(21, c->ops21);
   c->ops21_32 = ops_cast<float>(c->ops21);
   const double an = std::sqrt(axis[0] * axis[0] + axis[1] * axis[1] + axis[2] * axis[2]);
@@ -1625,38 +1565,55 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
   if (e == cudaSuccess) {
     // metric of the four meshes (mesh_factory_mod.f90:25-133: alpha =
     // alpha0 + (i - 1 + shift_i) hx, shift 1/2 at centres, 0 on faces and
-    // corners), one field at a time through a host buffer
-    std::vector<double> hm(tables_only ? 0 : g.fs, 0.0);
-    for (int k = 0; k < (tables_only ? 0 : M_COUNT) && e == cudaSuccess; ++k) {
-      std::fill(hm.begin(), hm.end(), 0.0);
-      const int mesh = kMetricMesh[k];
+    // corners).  All but the Coriolis parameter are the same on every panel:
+    // one panel is formed and copied to the others on the device.
+    const double sw = scale_w(order), sd = scale_d(order);
+    std::vector<double> tn(N + 1), tc(N);   // tangents at the nodes and centres of a line
+    for (int i = 0; i <= N; ++i) tn[i] = std::tan(-0.25 * kPiC + (i + 0.0) * c->hx);
+    for (int i = 0; i < N; ++i) tc[i] = std::tan(-0.25 * kPiC + (i + 0.5) * c->hx);
+    std::vector<double> hm(tables_only ? 0 : g.ps, 0.0);
+    std::vector<MetricAt> mm(tables_only ? 0 : (size_t)(N + 1) * (N + 1));
+    for (int mesh = 0; mesh < (tables_only ? 0 : 4) && e == cudaSuccess; ++mesh) {
       const bool ci = mesh == 0 || mesh == 2;  // centred in alpha
       const bool cj = mesh == 0 || mesh == 1;  // centred in beta
       const int nx = ci ? N : N + 1, ny = cj ? N : N + 1;
-      for (int p = 0; p < 6; ++p)
-        for (int j = 0; j < ny; ++j)
-          for (int i = 0; i < nx; ++i) {
-            const double al = -0.25 * kPiC + (i + (ci ? 0.5 : 0.0)) * c->hx;
-            const double be = -0.25 * kPiC + (j + (cj ? 0.5 : 0.0)) * c->hx;
-            const MetricAt m = metric_at(al, be);
-            const double J = m.J, jha = J * c->hx * radius;
-            double x;
-            switch (k) {
-              case M_QI2P: x = m.qi2; break;
-              case M_FP: x = coriolis_at(p, al, be, omega, ax); break;
-              case M_RJP: case M_RJU: case M_RJV: x = 1.0 / J; break;
-              case M_RJPHA: case M_RJQHA: case M_RJUHA: case M_RJVHA: x = 1.0 / jha; break;
-              case M_JQI2P: x = J * m.qi2; break;
-              case M_QI1U: x = m.qi1; break;
-              case M_QI3V: x = m.qi3; break;
-              case M_JQ2P: x = J * m.q2; break;
-              case M_Q1U: x = m.q1; break;
-              case M_Q3V: x = m.q3; break;
-              default: x = J; break;
+      const std::vector<double>&ta = ci ? tc : tn, &tb = cj ? tc : tn;
+      for (int j = 0; j < ny; ++j)
+        for (int i = 0; i < nx; ++i) mm[(size_t)j * nx + i] = metric_of_tan(ta[i], tb[j]);
+      for (int k = 0; k < M_COUNT && e == cudaSuccess; ++k) {
+        if (kMetricMesh[k] != mesh) continue;
+        std::fill(hm.begin(), hm.end(), 0.0);
+        double* dst = c->met + (size_t)k * g.fs;
+        for (int p = 0; p < (k == M_FP ? 6 : 1); ++p) {
+          for (int j = 0; j < ny; ++j)
+            for (int i = 0; i < nx; ++i) {
+              const MetricAt& m = mm[(size_t)j * nx + i];
+              const double J = m.J, jha = J * c->hx * radius;
+              double x;
+              switch (k) {
+                case M_QI2P: x = m.qi2; break;
+                case M_FP: x = coriolis_at(p, ta[i], tb[j], omega, ax); break;
+                case M_RJP: case M_RJU: case M_RJV: x = 1.0 / J; break;
+                case M_RJPHA: case M_RJQHA: case M_RJUHA: case M_RJVHA: x = 1.0 / jha; break;
+                case M_JQI2P: x = J * m.qi2; break;
+                case M_QI1U: x = m.qi1; break;
+                case M_QI3V: x = m.qi3; break;
+                case M_JQ2P: x = J * m.q2; break;
+                case M_Q1U: x = m.q1; break;
+                case M_Q3V: x = m.q3; break;
+                case M_SJU: case M_SJV: x = sw * sw / J; break;
+                case M_SJQ: x = sd / jha; break;
+                case M_SJP: x = 0.5 * sw / J; break;
+                case M_SDIV: x = sd * sw / jha; break;
+                default: x = J; break;
+              }
+              hm[(size_t)j * g.P + i] = x;
             }
-            hm[(size_t)p * g.ps + (size_t)j * g.P + i] = x;
-          }
-      ok(cudaMemcpy(c->met + (size_t)k * g.fs, hm.data(), fb, cudaMemcpyHostToDevice));
+          ok(cudaMemcpy(dst + p * g.ps, hm.data(), sizeof(double) * g.ps, cudaMemcpyHostToDevice));
+        }
+        for (int p = 1; p < 6 && k != M_FP; ++p)
+          ok(cudaMemcpyAsync(dst + p * g.ps, dst, sizeof(double) * g.ps, cudaMemcpyDeviceToDevice, st));
+      }
     }
     if (!tables_only) {
       ok(cudaMemsetAsync(c->wk, 0, W_COUNT * fb, st));
@@ -1720,7 +1677,7 @@ void cgrid_mesh_dims(const CGrid* c, int mesh, int* nx, int* ny) {
 cudaError_t cgrid_co2contra(CGrid* c, const double* u, const double* v, double* ut, double* vt, cudaStream_t st) {
   CArgsT<double> a = base_args<double>(c);
   a.u = u; a.v = v; a.ut = ut; a.vt = vt;
-  a.flags = F_CO | F_WUT;
+  a.flags = F_CO;
   CKE(run_centre_a(c, a, st));
   return run_faces_a(c, a, st);
 }
@@ -1729,7 +1686,7 @@ cudaError_t cgrid_massflux(CGrid* c, const double* h, const double* ut, const do
                            cudaStream_t st) {
   CArgsT<double> a = base_args<double>(c);
   a.h = h; a.ut_in = ut; a.vt_in = vt; a.hu = hu; a.hv = hv;
-  a.flags = F_MF | F_WFLUX;
+  a.flags = F_MF;
   return run_faces_a(c, a, st);
 }
 
@@ -1745,7 +1702,7 @@ cudaError_t cgrid_ke(CGrid* c, const double* u, const double* v, const double* u
 cudaError_t cgrid_grad(CGrid* c, const double* f, double* gx, double* gy, cudaStream_t st) {
   CArgsT<double> a = base_args<double>(c);
   a.ke_in = f; a.o1 = gx; a.o2 = gy;
-  a.flags = F_GRAD | F_SEP;
+  a.flags = F_GRAD;
   return run_faces_b(c, a, st);
 }
 
@@ -1756,7 +1713,7 @@ cudaError_t cgrid_div(CGrid* c, const double* hu, const double* hv, double* div,
     a.flags = F_G;
     CKE(run_faces_a(c, a, st));
   }
-  a.flags = F_DIV | F_SEP;
+  a.flags = F_DIV;
   return run_centre_b(c, a, st);
 }
 
@@ -1778,27 +1735,25 @@ cudaError_t cgrid_coriolis(CGrid* c, const double* hu, const double* hv, const d
   a.flags = F_COR;
   CKE(run_centre_b(c, a, st));
   a.o1 = cor_u; a.o2 = cor_v;
-  a.flags = F_COR | F_SEP;
+  a.flags = F_COR;
   return run_faces_b(c, a, st);
 }
 
 cudaError_t cgrid_apply(CGrid* c, const Topology& tp, double* edge, const double* hs, const double* in, double* out,
                         cudaStream_t st) {
-  CArgsT<double> a = base_args<double>(c);
+  RhsArgs<double> a = rhs_args<double>(c);
   a.hs = hs;
-  a.mode = 0;
   a.tend = out;
-  return rhs(c, a, in, st);
+  return rhs(c, a, 0, in, st);
 }
 
 cudaError_t cgrid_apply32(CGrid* c, const Topology& tp, float* edge, const float* hs, const float* in, float* out,
                           cudaStream_t st) {
   if (!c->met32) return cudaErrorInvalidValue;
-  CArgsT<float> a = base_args<float>(c);
+  RhsArgs<float> a = rhs_args<float>(c);
   a.hs = hs;
-  a.mode = 0;
   a.tend = out;
-  return rhs(c, a, in, st);
+  return rhs(c, a, 0, in, st);
 }
 
 // The FP32 form: stage inputs are the state's high part (stage 1) or Y in
@@ -1807,38 +1762,32 @@ cudaError_t cgrid_apply32(CGrid* c, const Topology& tp, float* edge, const float
 cudaError_t cgrid_rk4_32(CGrid* c, const Topology& tp, float* edge, const float* hs, float* hi, float* lo, double dt,
                          cudaStream_t st) {
   if (!c->met32) return cudaErrorInvalidValue;
-  CArgsT<float> a = base_args<float>(c);
+  RhsArgs<float> a = rhs_args<float>(c);
   a.hs = hs;
   a.dt = float(dt); a.hdt = float(0.5 * dt); a.c6 = float(dt / 6.0); a.c3 = float(dt / 3.0);
   a.y0 = hi;
   a.lo = lo;
   a.Y = reinterpret_cast<float*>(c->rk);
   a.acc = a.Y + 3 * c->g.fs;
-  for (int s = 1; s <= 4; ++s) {
-    a.mode = s;
-    CKE(rhs(c, a, s == 1 ? static_cast<const float*>(hi) : a.Y, st));
-  }
+  for (int s = 1; s <= 4; ++s) CKE(rhs(c, a, s, s == 1 ? static_cast<const float*>(hi) : a.Y, st));
   return cudaSuccess;
 }
 
 // Stage 1 reads y0 and writes Y; stages 2 and 3 read Y and write Y in place;
 // stage 4 reads Y and writes y0.  In place is safe: the passes that read the
-// stage input at neighbouring points (centre_a, faces_a, curl) run before the
-// two that write it (centre_b, faces_b), and those read only their own point
-// of it, before writing it.
+// stage input at neighbouring points (rhs1, rhs2) run before the two that
+// write it (rhs3 h, rhs4 u and v), and of it those read only h at their own
+// point (rhs3), before writing it.
 cudaError_t cgrid_rk4(CGrid* c, const Topology& tp, double* edge, const double* hs, double* y0, double dt,
                       cudaStream_t st) {
-  CArgsT<double> a = base_args<double>(c);
+  RhsArgs<double> a = rhs_args<double>(c);
   a.hs = hs;
   a.dt = dt; a.hdt = 0.5 * dt; a.c6 = dt / 6.0; a.c3 = dt / 3.0;
   a.y0 = y0;
   a.Y = c->rk;
   a.Kb = c->rk + 3 * c->g.fs;
   a.acc = c->rk + 6 * c->g.fs;
-  for (int s = 1; s <= 4; ++s) {
-    a.mode = s;
-    CKE(rhs(c, a, s == 1 ? y0 : a.Y, st));
-  }
+  for (int s = 1; s <= 4; ++s) CKE(rhs(c, a, s, s == 1 ? static_cast<const double*>(y0) : a.Y, st));
   return cudaSuccess;
 }
 

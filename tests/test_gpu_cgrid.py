@@ -264,6 +264,24 @@ def test_apply_fused_and_unfused_match_oracle(order):
             assert _rel(a, b) < 1e-10, (apply.__name__, _rel(a, b))
 
 
+# The fused passes run the four columns of either side as warps along the
+# column and the columns between in tiles of 32: the smallest panel, panels
+# whose inner columns are one below, at and one above a whole number of tiles,
+# and one whose rows leave a partial block, with orography.
+@pytest.mark.parametrize("order", [42, 21])
+@pytest.mark.parametrize("N", [16, 17, 38, 39, 40, 72])
+def test_fused_passes_match_unfused_operators(order, N):
+    op = c_op(N, order)
+    op.set_orography(50.0 * np.cos(np.arange(N) * 0.3)[None, None, :] * np.ones(op.shape))
+    x = op.create_stvec()
+    x.upload(*_state(N))
+    a, b = x.create_similar(), x.create_similar()
+    op.apply(a, x)
+    op.apply_unfused(b, x)
+    for f, g in zip(a.download(), b.download()):
+        assert _rel(f, g) < 1e-10, _rel(f, g)
+
+
 @pytest.mark.parametrize("order,N,steps", [(42, 40, 1), (42, 40, 24), (21, 40, 24), (42, 96, 2)])
 def test_rk4_matches_oracle(order, N, steps):
     op, od = c_op(N, order), oracle.OracleCDomain(N, order)
