@@ -158,26 +158,28 @@ __device__ __forceinline__ void node_tendency(T gx, T gy, T zeta, T dv, T f, T J
 // ---------------------------------------------------------------------------
 constexpr int PT_TPB = 128;
 
-// Node of thread tid: first the closure columns (along the column), then
-// the others (along the row).  False past the last node.
-template <int ORD>
-__host__ __device__ inline bool point_node(int n, int tid, int& p, int& i, int& j) {
-  constexpr int NE = Ord<ORD>::NE;
-  const int nclosed = 12 * NE * n, ni = n - 2 * NE;
+// Node of thread tid: first the E columns at either panel side (threads along
+// the column), then the others (along the row).  False past the last node.
+// Panels of fewer than 2 E columns split in the middle: the columns between
+// are then not free of closures, so kernels test the node, not the thread.
+template <int E>
+__device__ __forceinline__ bool point_node(int n, int tid, int& p, int& i, int& j) {
+  const int ne = min(E, n / 2), nclosed = 12 * ne * n, ni = n - 2 * ne;
   if (tid < nclosed) {
     const int r = tid / n;
     j = tid - r * n;
-    const int c = r % NE, s = r / NE;
+    const int s = r / ne, c = r - s * ne;
     i = (s & 1) ? n - 1 - c : c;
     p = s >> 1;
     return true;
   }
-  const int t = tid - nclosed, row = t / ni;
+  const int t = tid - nclosed, row = ni > 0 ? t / ni : 6 * n;
   p = row / n;
   j = row - p * n;
-  i = NE + t - row * ni;
+  i = ne + t - row * ni;
   return p < 6;
 }
+
 // Stencil inputs of a node with state (h, u, v).
 template <class T>
 __device__ __forceinline__ void derive_store(T* der, long long fs, long long idx, T h, T u, T v, T J,
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(PT_TPB)
   const InstDev<T>& I = many ? many[blockIdx.y] : one;
   const int n = I.n, P = I.P;
   int p, i, j;
-  if (!point_node<ORD>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
+  if (!point_node<NE>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
   const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
   const T* __restrict__ K = I.der + DR_K2 * fs + x;
   const T* __restrict__ GU = I.der + DR_GU * fs + x;

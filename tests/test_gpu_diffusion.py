@@ -48,6 +48,20 @@ def test_laplace_matches_oracle(narrow, N):
     assert rel_l2(fi.download(), ref, J) <= 1e-12
 
 
+# The FP64 kernels number the closure columns first: panels of closure columns
+# only (6/3 at N=17) and of one and a few inner columns, and of one node more
+# than whole warps.
+@pytest.mark.parametrize("narrow,N", [(63, 17), (63, 18), (63, 26), (42, 16), (42, 43), (42, 44), (21, 16)])
+def test_laplace_small_panels_match_oracle(narrow, N):
+    op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=42, precision="fp64"))
+    od = oracle.OracleDomain(N, 42)
+    f = _state(N)[0]
+    fi, fo = op.create_field(), op.create_field()
+    fi.upload(f)
+    op.laplace(fo, fi, narrow)
+    assert rel_l2(fo.download(), od.laplace(f, narrow), od.geometry()["J"]) <= 1e-12
+
+
 @pytest.mark.parametrize("uv_narrow,h_narrow", [(42, 42), (63, 63), (63, 42), (21, 21), (42, 21)])
 def test_diffusion_operator_matches_oracle(uv_narrow, h_narrow):
     N = 32
