@@ -514,7 +514,7 @@ int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode, bool derive = true) {
   }
   if constexpr (sizeof(T) == 8) {
     if (derive) CK(launch_derive64(I, nullptr, 1, ctx->n, ctx->st), "stencil inputs");
-    CK(launch_stage64(ctx->order, I, nullptr, 1, ctx->n, mode, ctx->st), "stage kernel");
+    CK(launch_stage64(ctx->order, I, nullptr, 1, ctx->n, ctx->topo, mode, ctx->st), "stage kernel");
   } else {
     CK(launch_stage<T>(ctx->order, ctx->shape.cols, ctx->shape.fixbw != 0, &maps, I, nullptr, ctx->units,
                        ctx->nunits, mode, ctx->shape.boxw, ctx->stage_grid, ctx->derr, ctx->st),
@@ -523,13 +523,17 @@ int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode, bool derive = true) {
   if (ctx->timing) {
     CK(cudaEventRecord(b, ctx->st), "event record");
     ctx->ev_stage.emplace_back(a, b);
-    CK(cudaEventCreate(&a), "event"); CK(cudaEventCreate(&b), "event");
-    CK(cudaEventRecord(a, ctx->st), "event record");
   }
-  CK(launch_edge<T>(I, nullptr, 1, ctx->n, ctx->topo, mode, ctx->st), "edge kernel");
-  if (ctx->timing) {
-    CK(cudaEventRecord(b, ctx->st), "event record");
-    ctx->ev_edge.emplace_back(a, b);
+  if constexpr (sizeof(T) == 4) {   // the FP64 stage kernel finishes the boundary nodes itself
+    if (ctx->timing) {
+      CK(cudaEventCreate(&a), "event"); CK(cudaEventCreate(&b), "event");
+      CK(cudaEventRecord(a, ctx->st), "event record");
+    }
+    CK(launch_edge32(I, nullptr, 1, ctx->n, ctx->topo, mode, ctx->st), "edge kernel");
+    if (ctx->timing) {
+      CK(cudaEventRecord(b, ctx->st), "event record");
+      ctx->ev_edge.emplace_back(a, b);
+    }
   }
   return SWM_OK;
 }
@@ -2473,15 +2477,14 @@ int ens_capture(swm_ensemble* ens) {
     if constexpr (sizeof(T) == 8) {
       if (i == 0) e = launch_derive64(InstDev<T>{}, I, ens->nmem, ens->max_n, ens->st);
       if (e == cudaSuccess)
-        e = launch_stage64(ens->order, InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, MODE_RK1 + i,
+        e = launch_stage64(ens->order, InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i,
                            ens->st);
     } else {
       e = launch_stage<T>(ens->order, ens->cols, ens->fixbw, nullptr, InstDev<T>{}, I + i * ens->nmem,
                           ens->dunits, ens->nunits, MODE_RK1 + i, ens->boxw, ens->grid, derr, ens->st);
+      if (e == cudaSuccess)
+        e = launch_edge32(InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i, ens->st);
     }
-    if (e == cudaSuccess)
-      e = launch_edge<T>(InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i,
-                         ens->st);
   }
   cudaError_t ec = cudaStreamEndCapture(ens->st, &g);
   if (e != cudaSuccess) { if (ec == cudaSuccess) cudaGraphDestroy(g); ECK(e, "ensemble stage launch"); }

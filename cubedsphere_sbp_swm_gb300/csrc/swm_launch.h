@@ -48,10 +48,9 @@ cudaError_t stage_f32_prepare(int order);
 cudaError_t launch_derive64(const InstDev<double>& one, const InstDev<double>* many, int ninst,
                             int max_n, cudaStream_t st);
 cudaError_t launch_stage64(int order, const InstDev<double>& one, const InstDev<double>* many,
-                           int ninst, int max_n, int mode, cudaStream_t st);
-// Cube-edge kernel over ninst instances whose largest edge has max_n nodes.
-template <class T>
-cudaError_t launch_edge(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,
-                        const Topology& tp, int mode, cudaStream_t st);
+                           int ninst, int max_n, const Topology& tp, int mode, cudaStream_t st);
+// FP32 cube-edge kernel over ninst instances whose largest edge has max_n nodes.
+cudaError_t launch_edge32(const InstDev<float>& one, const InstDev<float>* many, int ninst, int max_n,
+                          const Topology& tp, int mode, cudaStream_t st);
 
 }  // namespace swm

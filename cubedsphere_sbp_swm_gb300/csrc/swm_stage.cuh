@@ -1,6 +1,6 @@
 // swm_stage.cuh -- SBP derivatives, the RHS tendency and RK stage epilogue,
 // the FP64 stage kernels, and the cube-edge pass that finishes the
-// panel-boundary nodes (both precisions; the FP32 stage kernel is in
+// panel-boundary nodes of an FP32 stage (whose stage kernel is in
 // swm_stage_tma.cuh).
 //
 // One FP64 RK stage:
@@ -8,16 +8,17 @@
 //                        inputs of the state: 2(KE + g(h+hs)), J h ut, J h vt,
 //                        J ut, J vt
 //   point_stage_kernel   every node: SBP grad(KE), curl and div(h u) with
-//                        their one-sided closures from those fields; interior
-//                        nodes then get Coriolis, the tendency, the RK stage
-//                        combination and the next stage's stencil inputs;
-//                        panel-boundary nodes write their pre-sync
-//                        (gx, gy, zeta, div) to the edge buffer.
-//   edge_kernel          every panel-boundary node: the reference's cube-edge
-//                        syncs (2-way average on edges, 3-way at cube
-//                        corners, metric-weighted for the covariant
-//                        gradient), then the same tendency, RK epilogue and
-//                        (FP64) next stencil inputs.
+//                        their one-sided closures from those fields, the
+//                        cube-edge syncs at panel-boundary nodes, Coriolis,
+//                        the tendency, the RK stage combination and the next
+//                        stage's stencil inputs.
+// An FP32 stage is its stage kernel and the
+//   edge_kernel          every panel-boundary node, from the pre-sync
+//                        (gx, gy, zeta, div) of the stage kernel: the
+//                        reference's cube-edge syncs (2-way average on edges,
+//                        3-way at cube corners, metric-weighted for the
+//                        covariant gradient), then the tendency and the RK
+//                        epilogue.
 // Reference: operator_swm_mod.f90:61-113, rk4_mod.f90:20-42,
 // sbp_operator_mod.f90:152-228, div_ah_sbp_mod.f90:46-96,
 // grad_ah_sbp_mod.f90:51-88, curl_div_based_mod.f90:26-66,
@@ -147,14 +148,20 @@ __device__ __forceinline__ void node_tendency(T gx, T gy, T zeta, T dv, T f, T J
 //     warps that run along the column, so that a warp's closure row is
 //     uniform and the other warps never meet one (in warps along the row, 2
 //     of 13 at N=384 ran closures and interior one after the other);
+//   - panel-boundary nodes form their neighbours' pre-sync terms themselves, a
+//     lane for their own panel and one for the neighbour's, in warps that start
+//     first, instead of a second launch that exchanges them (one lane for
+//     both: 0.126 against 0.073 ms a step at N=48);
 //   - differences are taken before they are scaled, and the constants come
 //     from the host: 32 FP64 instructions a node and 11 for the stencil inputs
 //     (4/2), against 58; with constants formed per thread 50 instead of 45
 //     (0.343 against 0.306 ms a step).
-// Measured, RK4 steps d42: N=48 0.239 -> 0.090 ms, N=192 0.251 -> 0.139 ms,
-// N=384 0.451 -> 0.306 ms (N=48, 192 one instance alone; the FP64 pipe is 82%
-// busy in a lone launch).  Blocks of 64 and 256 threads measured within 1% of
-// 128; 12 blocks a SM by capping the registers 1.5% slower.
+// Measured, RK4 steps d42 of one instance: N=48 0.239 -> 0.073 ms, N=192 0.251
+// -> 0.125 ms, N=384 0.560 -> 0.342 ms (0.090, 0.139 and 0.371 with the
+// boundary nodes in a launch of their own).  The FP64 pipe is 82% busy in a
+// launch at N=384.  Blocks of 64 and 256 threads measured within 1% of 128;
+// registers capped for 6, 7 or 8 blocks an SM (96 uncapped, 5 blocks) are 0.7%
+// faster at N=384 with three instances, 9 to 17% slower at N <= 201.
 // ---------------------------------------------------------------------------
 constexpr int PT_TPB = 128;
 
@@ -178,6 +185,15 @@ __device__ __forceinline__ bool point_node(int n, int tid, int& p, int& i, int& 
   j = row - p * n;
   i = ne + t - row * ni;
   return p < 6;
+}
+
+// boundary node b of a panel (0 <= b < 4n-4) -> (i, j); bottom and top rows
+// own the corners.
+__device__ __forceinline__ void boundary_node(int b, int n, int& i, int& j) {
+  if (b < n) { i = b; j = 0; }
+  else if (b < 2 * n) { i = b - n; j = n - 1; }
+  else if (b < 3 * n - 2) { i = 0; j = b - 2 * n + 1; }
+  else { i = n - 1; j = b - (3 * n - 2) + 1; }
 }
 
 // Stencil inputs of a node with state (h, u, v).
@@ -229,63 +245,151 @@ __device__ __forceinline__ T d_scaled(const T (&c)[3], F dif) {
   return s;
 }
 
+// Pre-sync gx, gy, curl and divergence of a node from the stencil inputs.
+template <int ORD, class T>
+__device__ __forceinline__ void raw_terms(const InstDev<T>& I, int p, int i, int j, T& gx, T& gy, T& zeta,
+                                          T& dv) {
+  const int n = I.n, P = I.P;
+  const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
+  auto dx = [&](const T* q) { return d_line<ORD, T>(i, n, [&](int m) { return q[x + (m - i)]; }); };
+  auto dy = [&](const T* q) { return d_line<ORD, T>(j, n, [&](int m) { return q[x + (m - j) * P]; }); };
+  const T rJ = I.metric[MRJ * fs + x];
+  const T* K = I.der + DR_K2 * fs;
+  gx = dx(K) * I.ghs2;
+  gy = dy(K) * I.ghs2;
+  zeta = (dx(I.in + 2 * fs) - dy(I.in + fs)) * rJ;
+  dv = (dx(I.der + DR_GU * fs) + dy(I.der + DR_GV * fs)) * rJ;
+}
+
+// Threads of one instance: the panel-boundary nodes (two lanes each), the
+// other closure columns, the other nodes, each padded to whole blocks.
+struct PointRanges {
+  int nb, closed, total;
+};
+template <int ORD>
+__host__ __device__ inline PointRanges point_ranges(int n) {
+  auto pad = [](int k) { return (k + PT_TPB - 1) / PT_TPB * PT_TPB; };
+  constexpr int NE = Ord<ORD>::NE;
+  PointRanges r;
+  r.nb = pad(2 * 6 * (4 * n - 4));
+  r.closed = r.nb + pad(12 * (NE - 1) * (n - 2));
+  r.total = r.closed + pad(6 * (n - 2 * NE) * (n - 2));
+  return r;
+}
+
 template <class T, int ORD, int MODE>
 __global__ void __launch_bounds__(PT_TPB)
-    point_stage_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many) {
+    point_stage_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many,
+                       const __grid_constant__ Topology tp) {
   constexpr int NE = Ord<ORD>::NE;
   constexpr bool needB = MODE == MODE_RK1 || MODE == MODE_RK2 || MODE == MODE_RK3;
   constexpr bool needA = MODE == MODE_RK2 || MODE == MODE_RK3 || MODE == MODE_RK4;
   const InstDev<T>& I = many ? many[blockIdx.y] : one;
-  const int n = I.n, P = I.P;
+  const int n = I.n, P = I.P, tid = blockIdx.x * PT_TPB + threadIdx.x;
+  const PointRanges rg = point_ranges<ORD>(n);
   int p, i, j;
-  if (!point_node<NE>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
+  if (tid < rg.nb) {
+    const int nb = 4 * n - 4, t = min(tid >> 1, 6 * nb - 1);   // surplus lanes stay for the shuffles
+    p = t / nb;
+    boundary_node(t - p * nb, n, i, j);
+  } else if (tid < rg.closed) {   // along the column: rows 1..n-2
+    const int t = tid - rg.nb, r = t / (n - 2);
+    if (r >= 12 * (NE - 1)) return;
+    j = 1 + t - r * (n - 2);
+    const int s = r / (NE > 1 ? NE - 1 : 1), c = 1 + r - s * (NE - 1);
+    i = (s & 1) ? n - 1 - c : c;
+    p = s >> 1;
+  } else {
+    const int t = tid - rg.closed, ni = n - 2 * NE, row = t / ni;
+    p = row / (n - 2);
+    if (p >= 6) return;
+    j = 1 + row - p * (n - 2);
+    i = NE + t - row * ni;
+  }
   const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
-  const T* __restrict__ K = I.der + DR_K2 * fs + x;
-  const T* __restrict__ GU = I.der + DR_GU * fs + x;
-  const T* __restrict__ GV = I.der + DR_GV * fs + x;
-  const T* __restrict__ U = I.in + fs + x;
-  const T* __restrict__ V = I.in + 2 * fs + x;
   T rb[3] = {}, ra[3] = {}, rl[3] = {};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     if (needB) rb[c] = I.base[c * fs + x];
     if (needA) ra[c] = I.acc ? I.acc[c * fs + x] : T(0);
   }
-  T rJ = I.metric[MRJ * fs + x];
   const T f = I.metric[MF * fs + x];
   const T jut = I.der[DR_JUT * fs + x], jvt = I.der[DR_JVT * fs + x];
-  T gx, gy, zw, dw;   // zw, dw: the curl and the divergence before the factor rJ
-  const bool xin = i >= NE && i < n - NE, yin = j >= NE && j < n - NE;
-  if (xin && yin) {
-    gx = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o] - K[-o]; });
-    gy = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o * P] - K[-o * P]; });
-    zw = d_ratio<ORD, T>([&](int o) { return (V[o] - V[-o]) - (U[o * P] - U[-o * P]); });
-    dw = d_ratio<ORD, T>([&](int o) { return (GU[o] - GU[-o]) + (GV[o * P] - GV[-o * P]); });
-    rJ = rJ * T(d_coef<ORD>(1));
-  } else {
-    auto dx = [&](const T* q) { return d_line<ORD, T>(i, n, [&](int m) { return q[m - i]; }); };
-    auto dy = [&](const T* q) { return d_line<ORD, T>(j, n, [&](int m) { return q[(m - j) * P]; }); };
-    gx = dx(K) * I.ghs2;
-    gy = dy(K) * I.ghs2;
-    zw = dx(V) - dy(U);
-    dw = dx(GU) + dy(GV);
-    if (i == 0 || i == n - 1 || j == 0 || j == n - 1) {
-      const T zeta = zw * rJ, dv = dw * rJ;
-      T* E = I.edge + (long long)p * 16 * n;
-      auto put = [&](int side, int k) {
-        T* e = E + (side * 4) * n + k;
-        e[0] = gx; e[n] = gy; e[2 * n] = zeta; e[3 * n] = dv;
-      };
-      if (i == 0) put(SIDE_L, j);
-      if (i == n - 1) put(SIDE_R, j);
-      if (j == 0) put(SIDE_B, i);
-      if (j == n - 1) put(SIDE_T, i);
-      return;
+  T kh, ku, kv;
+  if (tid < rg.nb) {
+    // A boundary node: one lane forms the raw terms of its own panel, the other
+    // those of the panels that hold copies of it (formed here again rather
+    // than exchanged); then their sync (2-way average on edges, 3-way at cube
+    // corners; the covariant gradient with the metric weights;
+    // halo_Ah_scalar_sync_mod.f90:38-93, ecs_Ah_vec_sync_mod.f90:62-125).
+    const int e = n - 1;
+    const bool lr = (i == 0) | (i == e), bt = (j == 0) | (j == e);
+    T sgx = T(0), sgy = T(0), sz = T(0), sd = T(0);
+    const bool own = (tid & 1) == 0;
+    const int copies = !own && lr && bt ? 2 : 1;
+#pragma unroll 1
+    for (int s = 0; s < copies; ++s) {
+      const bool side_lr = lr && s == 0;
+      int q = p, iq = i, jq = j;
+      EdgeLink L{};
+      if (!own) {
+        L = tp.link[p][side_lr ? (i == 0 ? SIDE_L : SIDE_R) : (j == 0 ? SIDE_B : SIDE_T)];
+        const int k = side_lr ? j : i, kk = L.rev ? e - k : k;
+        q = L.q;
+        iq = L.side_q == SIDE_L ? 0 : L.side_q == SIDE_R ? e : kk;
+        jq = L.side_q == SIDE_B ? 0 : L.side_q == SIDE_T ? e : kk;
+      }
+      T gx, gy, z, d;
+      raw_terms<ORD, T>(I, q, iq, jq, gx, gy, z, d);
+      if (!own) {   // the neighbour's components in this panel's frame
+        const T a = L.dim_i ? T(L.istep) * gx : T(L.jstep) * gy;
+        const T b = L.dim_i ? T(L.jstep) * gy : T(L.istep) * gx;
+        gx = a;
+        gy = b;
+        if (side_lr) gx += I.qw[(i == 0 ? 2 : 3) * n + j] * b;
+        else gy += I.qw[(j == 0 ? 0 : 1) * n + i] * a;
+      }
+      sgx += gx; sgy += gy; sz += z; sd += d;
     }
+    sgx += __shfl_xor_sync(0xffffffffu, sgx, 1);
+    sgy += __shfl_xor_sync(0xffffffffu, sgy, 1);
+    sz += __shfl_xor_sync(0xffffffffu, sz, 1);
+    sd += __shfl_xor_sync(0xffffffffu, sd, 1);
+    if (!own || (tid >> 1) >= 6 * (4 * n - 4)) return;
+    const T w = lr && bt ? T(1.0 / 3.0) : T(0.5);
+    const T fz = f + w * sz;
+    kh = -(w * sd);
+    ku = fz * jvt - w * sgx;
+    kv = -(fz * jut) - w * sgy;
+  } else {
+    const T* __restrict__ K = I.der + DR_K2 * fs + x;
+    const T* __restrict__ GU = I.der + DR_GU * fs + x;
+    const T* __restrict__ GV = I.der + DR_GV * fs + x;
+    const T* __restrict__ U = I.in + fs + x;
+    const T* __restrict__ V = I.in + 2 * fs + x;
+    T rJ = I.metric[MRJ * fs + x];
+    T gx, gy, zw, dw;   // zw, dw: the curl and the divergence before the factor rJ
+    if (i >= NE && i < n - NE && j >= NE && j < n - NE) {
+      gx = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o] - K[-o]; });
+      gy = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o * P] - K[-o * P]; });
+      zw = d_ratio<ORD, T>([&](int o) { return (V[o] - V[-o]) - (U[o * P] - U[-o * P]); });
+      dw = d_ratio<ORD, T>([&](int o) { return (GU[o] - GU[-o]) + (GV[o * P] - GV[-o * P]); });
+      rJ = rJ * T(d_coef<ORD>(1));
+    } else {
+      auto dx = [&](const T* q) { return d_line<ORD, T>(i, n, [&](int m) { return q[m - i]; }); };
+      auto dy = [&](const T* q) { return d_line<ORD, T>(j, n, [&](int m) { return q[(m - j) * P]; }); };
+      gx = dx(K) * I.ghs2;
+      gy = dy(K) * I.ghs2;
+      zw = dx(V) - dy(U);
+      dw = dx(GU) + dy(GV);
+    }
+    const T fz = f + zw * rJ;
+    kh = -(dw * rJ);
+    ku = fz * jvt - gx;
+    kv = -(fz * jut) - gy;
   }
-  const T fz = f + zw * rJ;
   T y[3];
-  stage_epilogue_pre<T>(I, MODE, x, -(dw * rJ), fz * jvt - gx, -(fz * jut) - gy, rb, ra, rl, y);
+  stage_epilogue_pre<T>(I, MODE, x, kh, ku, kv, rb, ra, rl, y);
   if (needB && I.der_out)
     derive_store<T>(I.der_out, fs, x, y[0], y[1], y[2], I.metric[MJ * fs + x], I.metric[MQI1 * fs + x],
                     I.metric[MQI2 * fs + x], I.metric[MQI3 * fs + x], I.grav2, I.hs);
@@ -301,14 +405,14 @@ cudaError_t launch_point_derive(const InstDev<T>& one, const InstDev<T>* many, i
 }
 template <class T, int ORD>
 cudaError_t launch_point_stage_ord(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,
-                                   int mode, cudaStream_t st) {
-  const dim3 g((6 * max_n * max_n + PT_TPB - 1) / PT_TPB, ninst);
+                                   const Topology& tp, int mode, cudaStream_t st) {
+  const dim3 g(point_ranges<ORD>(max_n).total / PT_TPB, ninst);
   switch (mode) {
-    case MODE_APPLY: point_stage_kernel<T, ORD, MODE_APPLY><<<g, PT_TPB, 0, st>>>(one, many); break;
-    case MODE_RK1: point_stage_kernel<T, ORD, MODE_RK1><<<g, PT_TPB, 0, st>>>(one, many); break;
-    case MODE_RK2: point_stage_kernel<T, ORD, MODE_RK2><<<g, PT_TPB, 0, st>>>(one, many); break;
-    case MODE_RK3: point_stage_kernel<T, ORD, MODE_RK3><<<g, PT_TPB, 0, st>>>(one, many); break;
-    case MODE_RK4: point_stage_kernel<T, ORD, MODE_RK4><<<g, PT_TPB, 0, st>>>(one, many); break;
+    case MODE_APPLY: point_stage_kernel<T, ORD, MODE_APPLY><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
+    case MODE_RK1: point_stage_kernel<T, ORD, MODE_RK1><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
+    case MODE_RK2: point_stage_kernel<T, ORD, MODE_RK2><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
+    case MODE_RK3: point_stage_kernel<T, ORD, MODE_RK3><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
+    case MODE_RK4: point_stage_kernel<T, ORD, MODE_RK4><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -410,14 +514,6 @@ __device__ void sync_vector_node(const EdgeView<T>& ev, const Topology& tp, cons
   }
 }
 
-// boundary node b of a panel (0 <= b < 4n-4) -> (i, j); bottom and top rows
-// own the corners.
-__device__ __forceinline__ void boundary_node(int b, int n, int& i, int& j) {
-  if (b < n) { i = b; j = 0; }
-  else if (b < 2 * n) { i = b - n; j = n - 1; }
-  else if (b < 3 * n - 2) { i = 0; j = b - 2 * n + 1; }
-  else { i = n - 1; j = b - (3 * n - 2) + 1; }
-}
 
 // ---------------------------------------------------------------------------
 // Edge kernel: finishes every panel-boundary node of every instance.
@@ -469,7 +565,7 @@ __global__ void edge_kernel(InstDev<T> one, const InstDev<T>* many, Topology tp,
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     rb[c] = needB ? bsrc[c * fs + idx] : T(0);
-    ra[c] = needA && I.acc ? I.acc[c * fs + idx] : T(0);
+    ra[c] = needA ? I.acc[c * fs + idx] : T(0);
     rlo[c] = needL ? I.base_lo[c * fs + idx] : T(0);
   }
 
@@ -506,9 +602,6 @@ __global__ void edge_kernel(InstDev<T> one, const InstDev<T>* many, Topology tp,
   node_tendency<T>(gx, gy, zeta, dv, f, J, ut, vt, kh, ku, kv);
   T y[3] = {};
   stage_epilogue_pre<T>(I, mode, idx, kh, ku, kv, rb, ra, rlo, y);
-  if constexpr (sizeof(T) == 8)
-    if (mode != MODE_APPLY && mode != MODE_RK4 && I.der_out)
-      derive_store<T>(I.der_out, fs, idx, y[0], y[1], y[2], J, q1, q2, q3, I.grav2, I.hs);
 }
 
 }  // namespace swm

@@ -65,9 +65,8 @@ cudaError_t prepare_stage<float>(int order, StageShape* shape) {
   return cudaGetLastError();
 }
 
-template <>
-cudaError_t launch_edge<float>(const InstDev<float>& one, const InstDev<float>* many, int ninst,
-                               int max_n, const Topology& tp, int mode, cudaStream_t st) {
+cudaError_t launch_edge32(const InstDev<float>& one, const InstDev<float>* many, int ninst,
+                          int max_n, const Topology& tp, int mode, cudaStream_t st) {
   const int nodes = 6 * (4 * max_n - 4);
   dim3 grid((nodes + 127) / 128, ninst);
   edge_kernel<float><<<grid, 128, 0, st>>>(one, many, tp, mode);

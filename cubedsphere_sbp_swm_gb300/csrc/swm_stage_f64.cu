@@ -1,5 +1,4 @@
-// swm_stage_f64.cu -- double instantiation of the FP64 stage kernels and the
-// cube-edge kernel.
+// swm_stage_f64.cu -- double instantiation of the FP64 stage kernels.
 #include "swm_launch.h"
 #include "swm_stage.cuh"
 
@@ -14,12 +13,12 @@ cudaError_t launch_derive64(const InstDev<double>& one, const InstDev<double>* m
 }
 
 cudaError_t launch_stage64(int order, const InstDev<double>& one, const InstDev<double>* many,
-                           int ninst, int max_n, int mode, cudaStream_t st) {
+                           int ninst, int max_n, const Topology& tp, int mode, cudaStream_t st) {
   switch (order) {
-    case 21: return launch_point_stage_ord<double, 21>(one, many, ninst, max_n, mode, st);
-    case 42: return launch_point_stage_ord<double, 42>(one, many, ninst, max_n, mode, st);
-    case 43: return launch_point_stage_ord<double, 43>(one, many, ninst, max_n, mode, st);
-    case 63: return launch_point_stage_ord<double, 63>(one, many, ninst, max_n, mode, st);
+    case 21: return launch_point_stage_ord<double, 21>(one, many, ninst, max_n, tp, mode, st);
+    case 42: return launch_point_stage_ord<double, 42>(one, many, ninst, max_n, tp, mode, st);
+    case 43: return launch_point_stage_ord<double, 43>(one, many, ninst, max_n, tp, mode, st);
+    case 63: return launch_point_stage_ord<double, 63>(one, many, ninst, max_n, tp, mode, st);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -48,15 +47,6 @@ int stage_occupancy<double>(int order, int boxw, int cols, bool fixbw) {
   (void)cols;
   (void)fixbw;
   return 1;
-}
-
-template <>
-cudaError_t launch_edge<double>(const InstDev<double>& one, const InstDev<double>* many, int ninst,
-                                int max_n, const Topology& tp, int mode, cudaStream_t st) {
-  const int nodes = 6 * (4 * max_n - 4);
-  dim3 grid((nodes + 127) / 128, ninst);
-  edge_kernel<double><<<grid, 128, 0, st>>>(one, many, tp, mode);
-  return cudaGetLastError();
 }
 
 }  // namespace swm
