@@ -2851,17 +2851,23 @@ int tl_apply(swm_ctx* ctx, const double* y, const double* dx, double* dk) {
 template <class T>
 int ad_stage(swm_ctx* ctx, const T* y, const T* lam, const T* mu_in, double alpha, double beta,
              T* mu_out, const T* acc_in, T* acc_out) {
-  T* C = (T*)ctx->adC;
-  T* Zedge = C + 16LL * 6 * ctx->n;   // edge values of the base curl
-  const T* m = metric_of<T>(ctx);
-  CK(launch_zeta_pre<T>(ctx->g, ctx->order, m, y, adf<T>(ctx, 9), Zedge, ctx->st), "ad curl");
-  CK(launch_ad_pre<T>(ctx->g, ctx->topo, ctx->qw, m, y, adf<T>(ctx, 9), Zedge, lam, mu_in, (T)alpha,
-                      (T)beta, adf<T>(ctx, 0), C, ctx->st),
-     "ad pre");
-  CK(launch_adsync_gather<T>(ctx->g, ctx->topo, m, C, adf<T>(ctx, 0), ctx->st), "ad syncs");
-  CK(launch_ad_main<T>(ctx->g, ctx->order, ctx->sbpT, m, (T)ctx->ghs, (T)ctx->cfg.grav, y,
-                       adf<T>(ctx, 0), mu_out, acc_in, acc_out, ctx->st),
-     "ad main");
+  if constexpr (sizeof(T) == 8) {
+    CK(launch_ad_stage64(ctx->g, ctx->order, ctx->topo, ctx->sbpT, ctx->qw, ctx->m64, ctx->ghs, ctx->cfg.grav, y,
+                         lam, mu_in, alpha, beta, adf<T>(ctx, 0), mu_out, acc_in, acc_out, ctx->st),
+       "ad stage");
+  } else {
+    T* C = (T*)ctx->adC;
+    T* Zedge = C + 16LL * 6 * ctx->n;   // edge values of the base curl
+    const T* m = metric_of<T>(ctx);
+    CK(launch_zeta_pre<T>(ctx->g, ctx->order, m, y, adf<T>(ctx, 9), Zedge, ctx->st), "ad curl");
+    CK(launch_ad_pre<T>(ctx->g, ctx->topo, ctx->qw, m, y, adf<T>(ctx, 9), Zedge, lam, mu_in, (T)alpha,
+                        (T)beta, adf<T>(ctx, 0), C, ctx->st),
+       "ad pre");
+    CK(launch_adsync_gather<T>(ctx->g, ctx->topo, m, C, adf<T>(ctx, 0), ctx->st), "ad syncs");
+    CK(launch_ad_main<T>(ctx->g, ctx->order, ctx->sbpT, m, (T)ctx->ghs, (T)ctx->cfg.grav, y,
+                         adf<T>(ctx, 0), mu_out, acc_in, acc_out, ctx->st),
+       "ad main");
+  }
   return SWM_OK;
 }
 

@@ -15,6 +15,15 @@
 // (SbpT), Ss^T = Ss (the sync averages each class of duplicated edge nodes
 // with equal weights, a symmetric projection) and Sv^T in two deterministic
 // passes (pull back onto the neighbour values each node read, then gather).
+//
+// FP64 has AD kernels of its own (ad_pre64_kernel, ad_main64_kernel): GB300's
+// FP64 rate bounds them, so they are built like the FP64 stage kernel.  The
+// base curl is formed where it is used, boundary nodes form their neighbours'
+// terms themselves (two lanes a node), so a stage is two launches, closure
+// columns are warps of their own, and differences are taken before scaling:
+// 26 + 42 FP64 instructions a node (4/2) against about 190 in the four kernels
+// of the FP32 form.  Gradient of 24 steps at N=192 (6 snapshots): 16.1 ->
+// 13.0 ms.
 #include "swm_ops.cuh"
 #include "swm_stage.cuh"
 
@@ -310,6 +319,204 @@ __global__ void adsync_gather_kernel(FieldGeom g, Topology tp, const T* m, const
   s2[x] = d * rJ;
 }
 
+// ------------------------------------------------------------- FP64 adjoint
+// One FP64 adjoint stage.  Fields of A, c the leading interior coefficient of
+// D: 0, 1 the transposed-synced cotangents of -GX, -GY; 2 and 3 c times those of
+// rJ DIV and rJ Z (J hx a rJ = 1 takes J out of the latter); 4, 5 the l_ut and
+// l_vt parts.
+struct Ad64 {
+  FieldGeom g;
+  const double *qw, *m, *y;
+  double ghs;
+};
+
+// cotangents of (h, u, v): alpha lam + beta mu
+template <bool MU>
+__device__ __forceinline__ void ad_cot(const Ad64& a, long long x, const double* lam, const double* mu,
+                                       double alpha, double beta, double& lh, double& lu, double& lv) {
+  const long long fs = a.g.fs;
+  lh = alpha * lam[x];
+  lu = alpha * lam[fs + x];
+  lv = alpha * lam[2 * fs + x];
+  if (MU) {
+    lh += beta * mu[x];
+    lu += beta * mu[fs + x];
+    lv += beta * mu[2 * fs + x];
+  }
+}
+// contravariant components of the base state
+__device__ __forceinline__ void ad_contra(const Ad64& a, long long x, double& ut, double& vt) {
+  const long long fs = a.g.fs;
+  const double u = a.y[fs + x], v = a.y[2 * fs + x], q2 = a.m[MQI2 * fs + x];
+  ut = a.m[MQI1 * fs + x] * u + q2 * v;
+  vt = q2 * u + a.m[MQI3 * fs + x] * v;
+}
+
+template <int ORD, bool MU>
+__global__ void __launch_bounds__(PT_TPB, 5)
+    ad_pre64_kernel(const __grid_constant__ Ad64 a, const __grid_constant__ Topology tp,
+                    const double* __restrict__ lam, const double* __restrict__ mu, double alpha,
+                    double beta, double* __restrict__ A) {
+  constexpr int NE = Ord<ORD>::NE;
+  constexpr double c1 = d_coef<ORD>(1);
+  const FieldGeom& g = a.g;
+  const int n = g.n, P = g.P, tid = blockIdx.x * PT_TPB + threadIdx.x;
+  const long long fs = g.fs;
+  PointAt at;
+  if (!point_at<ORD>(n, tid, at)) return;
+  const int p = at.p, i = at.i, j = at.j;
+  const long long x = (long long)p * g.ps + (long long)j * P + i;
+  const double rJ = a.m[MRJ * fs + x], J = a.m[MJ * fs + x], f = a.m[MF * fs + x];
+  const double* U = a.y + fs;
+  const double* V = a.y + 2 * fs;
+  // pre-sync curl at any node
+  auto curl = [&](long long xx, int ii, int jj) {
+    const double dv = taps_sum<ORD>(taps_of<ORD>(ii, n), V + xx, ii, 1);
+    const double du = taps_sum<ORD>(taps_of<ORD>(jj, n), U + xx, jj, P);
+    return (dv - du) * a.m[MRJ * fs + xx];
+  };
+  double lh, lu, lv, ut, vt, fz, w4, sh, su, sv;
+  if (at.boundary) {
+    const int e = n - 1;
+    const bool lr = (i == 0) | (i == e), bt = (j == 0) | (j == e), own = (tid & 1) == 0;
+    const double w = lr && bt ? 1.0 / 3.0 : 0.5;
+    double z = 0.0, l4 = 0.0;
+    sh = su = sv = 0.0;
+    lh = lu = lv = 0.0;
+    const int copies = !own && lr && bt ? 2 : 1;
+#pragma unroll 1
+    for (int s = 0; s < copies; ++s) {
+      const bool slr = lr && s == 0;
+      int q = p, iq = i, jq = j;
+      if (!own) {
+        const EdgeLink L = tp.link[p][slr ? (i == 0 ? SIDE_L : SIDE_R) : (j == 0 ? SIDE_B : SIDE_T)];
+        const int k = slr ? j : i, kk = L.rev ? e - k : k;
+        q = L.q;
+        iq = L.side_q == SIDE_L ? 0 : L.side_q == SIDE_R ? e : kk;
+        jq = L.side_q == SIDE_B ? 0 : L.side_q == SIDE_T ? e : kk;
+        const long long xx = (long long)q * g.ps + (long long)jq * P + iq;
+        double h1, u1, v1, ut1, vt1;
+        ad_cot<MU>(a, xx, lam, mu, alpha, beta, h1, u1, v1);
+        ad_contra(a, xx, ut1, vt1);
+        z += curl(xx, iq, jq);
+        sh += h1;
+        l4 += vt1 * u1 - ut1 * v1;
+        // what that node's sync read of this one (put_ring at the neighbour's
+        // side, whose link leads back here)
+        const EdgeLink B = tp.link[q][L.side_q];
+        const bool qlr = L.side_q == SIDE_L || L.side_q == SIDE_R;
+        const double* qq = a.qw + (L.side_q == SIDE_L ? 2 : L.side_q == SIDE_R ? 3 : L.side_q == SIDE_B ? 0 : 1) * n;
+        const double rx = qlr ? u1 : u1 + qq[iq] * v1, ry = qlr ? v1 + qq[jq] * u1 : v1;
+        su += B.dim_i ? B.istep * rx : B.istep * ry;
+        sv += B.dim_i ? B.jstep * ry : B.jstep * rx;
+      } else {
+        ad_cot<MU>(a, x, lam, mu, alpha, beta, lh, lu, lv);
+        z += curl(x, i, j);
+        sh += lh;
+        su += lu;
+        sv += lv;
+      }
+    }
+    ad_contra(a, x, ut, vt);
+    if (own) l4 = vt * lu - ut * lv;
+    z += __shfl_xor_sync(0xffffffffu, z, 1);
+    l4 += __shfl_xor_sync(0xffffffffu, l4, 1);
+    sh += __shfl_xor_sync(0xffffffffu, sh, 1);
+    su += __shfl_xor_sync(0xffffffffu, su, 1);
+    sv += __shfl_xor_sync(0xffffffffu, sv, 1);
+    if (!own || !at.live) return;
+    fz = f + w * z;
+    w4 = w * l4;
+    sh *= w; su *= w; sv *= w;
+    const double ws = -(c1 * rJ) * sh;
+    A[2 * fs + x] = ws;
+  } else {
+    ad_cot<MU>(a, x, lam, mu, alpha, beta, lh, lu, lv);
+    ad_contra(a, x, ut, vt);
+    const double rc = rJ * c1;
+    if (i >= NE && i < n - NE && j >= NE && j < n - NE)
+      fz = f + rc * d_ratio<ORD, double>([&](int o) {
+             return (V[x + o] - V[x - o]) - (U[x + o * P] - U[x - o * P]);
+           });
+    else
+      fz = f + curl(x, i, j);
+    w4 = vt * lu - ut * lv;
+    su = lu;
+    sv = lv;
+    A[2 * fs + x] = -rc * lh;
+  }
+  const double fj = fz * J;
+  A[x] = su;
+  A[fs + x] = sv;
+  A[3 * fs + x] = (c1 * a.ghs) * w4;
+  A[4 * fs + x] = -fj * lv;
+  A[5 * fs + x] = fj * lu;
+}
+
+// mu = F'(y)^T lk from A; also acc_out = acc_in + mu (see ad_main_kernel)
+template <int ORD>
+__global__ void __launch_bounds__(PT_TPB)
+    ad_main64_kernel(const __grid_constant__ Ad64 a, const __grid_constant__ SbpT t, double grav2,
+                     const double* __restrict__ A, double* out, const double* acc_in, double* acc_out) {
+  constexpr int CT = AdOrd<ORD>::CT;
+  constexpr double c1 = d_coef<ORD>(1);
+  const FieldGeom& g = a.g;
+  const int n = g.n, P = g.P;
+  int p, i, j;
+  if (!point_node<CT>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
+  const long long fs = g.fs, x = (long long)p * g.ps + (long long)j * P + i;
+  double ain[3] = {};
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    if (acc_out) ain[c] = acc_in[c * fs + x];
+  const double h = a.y[x], u = a.y[fs + x], v = a.y[2 * fs + x];
+  const double q1 = a.m[MQI1 * fs + x], q2 = a.m[MQI2 * fs + x], q3 = a.m[MQI3 * fs + x];
+  const double J = a.m[MJ * fs + x];
+  const double *A0 = A + x, *A1 = A + fs + x, *W3 = A + 2 * fs + x, *W4 = A + 3 * fs + x;
+  const bool xin = i >= CT && i < n - CT, yin = j >= CT && j < n - CT;
+  // hK: half the cotangent of K; gu, gv those of J h ut, J h vt
+  double hK, gu, gv, dx4, dy4;
+  if (xin && yin) {
+    hK = (0.5 * c1 * a.ghs) *
+         d_ratio<ORD, double>([&](int o) { return (A0[o] - A0[-o]) + (A1[o * P] - A1[-o * P]); });
+    gu = -d_ratio<ORD, double>([&](int o) { return W3[o] - W3[-o]; });
+    gv = -d_ratio<ORD, double>([&](int o) { return W3[o * P] - W3[-o * P]; });
+    dx4 = -d_ratio<ORD, double>([&](int o) { return W4[o] - W4[-o]; });
+    dy4 = -d_ratio<ORD, double>([&](int o) { return W4[o * P] - W4[-o * P]; });
+  } else {
+    auto tx = [&](const double* q) { return dT_line<ORD, double>(t, n, i, [&](int m) { return q[m - i]; }); };
+    auto ty = [&](const double* q) { return dT_line<ORD, double>(t, n, j, [&](int m) { return q[(m - j) * P]; }); };
+    hK = -(0.5 * a.ghs) * (tx(A0) + ty(A1));
+    constexpr double ic = 1.0 / c1;
+    gu = ic * tx(W3);
+    gv = ic * ty(W3);
+    dx4 = ic * tx(W4);
+    dy4 = ic * ty(W4);
+  }
+  const double ut = q1 * u + q2 * v, vt = q2 * u + q3 * v, jh = J * h;
+  const double lut = A[4 * fs + x] + jh * gu + u * hK;
+  const double lvt = A[5 * fs + x] + jh * gv + v * hK;
+  const double r[3] = {J * (ut * gu + vt * gv) + grav2 * hK, ut * hK + q1 * lut + q2 * lvt - dy4,
+                       vt * hK + q2 * lut + q3 * lvt + dx4};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (out) out[c * fs + x] = r[c];
+    if (acc_out) acc_out[c * fs + x] = ain[c] + r[c];
+  }
+}
+
+template <int ORD>
+cudaError_t ad_stage64(const Ad64& a, const Topology& tp, const SbpT& t, double grav, const double* lam,
+                       const double* mu, double alpha, double beta, double* A, double* out,
+                       const double* acc_in, double* acc_out, cudaStream_t st) {
+  const int n = a.g.n, pre = point_ranges<ORD>(n).total / PT_TPB;
+  if (mu) ad_pre64_kernel<ORD, true><<<pre, PT_TPB, 0, st>>>(a, tp, lam, mu, alpha, beta, A);
+  else ad_pre64_kernel<ORD, false><<<pre, PT_TPB, 0, st>>>(a, tp, lam, mu, alpha, beta, A);
+  ad_main64_kernel<ORD><<<(6 * n * n + PT_TPB - 1) / PT_TPB, PT_TPB, 0, st>>>(a, t, 2.0 * grav, A, out, acc_in,
+                                                                            acc_out);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_tl_pre(const FieldGeom& g, const double* m64, double grav, const double* y,
@@ -373,6 +580,21 @@ cudaError_t launch_ad_main(const FieldGeom& g, int order, const SbpT& t, const T
   return cudaGetLastError();
 }
 
+// mu_out = F'(y)^T (alpha lam + beta mu), acc_out = acc_in + mu_out
+cudaError_t launch_ad_stage64(const FieldGeom& g, int order, const Topology& tp, const SbpT& t,
+                              const double* qw, const double* m, double ghs, double grav, const double* y,
+                              const double* lam, const double* mu, double alpha, double beta, double* A,
+                              double* out, const double* acc_in, double* acc_out, cudaStream_t st) {
+  const Ad64 a{g, qw, m, y, ghs};
+  switch (order) {
+    case 21: return ad_stage64<21>(a, tp, t, grav, lam, mu, alpha, beta, A, out, acc_in, acc_out, st);
+    case 42: return ad_stage64<42>(a, tp, t, grav, lam, mu, alpha, beta, A, out, acc_in, acc_out, st);
+    case 43: return ad_stage64<43>(a, tp, t, grav, lam, mu, alpha, beta, A, out, acc_in, acc_out, st);
+    case 63: return ad_stage64<63>(a, tp, t, grav, lam, mu, alpha, beta, A, out, acc_in, acc_out, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 #define SWM_AD_INSTANTIATE(T)                                                                    \
   template cudaError_t launch_zeta_pre<T>(const FieldGeom&, int, const T*, const T*, T*, T*,      \
                                           cudaStream_t);                                          \
@@ -384,7 +606,6 @@ cudaError_t launch_ad_main(const FieldGeom& g, int order, const SbpT& t, const T
   template cudaError_t launch_ad_main<T>(const FieldGeom&, int, const SbpT&, const T*, T, T,     \
                                          const T*, const T*, T*, const T*, T*, cudaStream_t);
 SWM_AD_INSTANTIATE(float)
-SWM_AD_INSTANTIATE(double)
 #undef SWM_AD_INSTANTIATE
 
 int adjoint_table_ct(int order) {

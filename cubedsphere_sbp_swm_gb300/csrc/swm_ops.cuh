@@ -82,7 +82,13 @@ cudaError_t launch_tl_post(const FieldGeom& g, const double* m64, const double* 
                            const double* zeta, const double* w, const double* dgx,
                            const double* dgy, const double* dz, const double* ddiv, double* dk,
                            cudaStream_t st);
-// Adjoint stage pieces, FP64 or FP32 (order = SBP order of the context;
+// One FP64 adjoint stage: out = F'(y)^T (alpha lam + beta mu) (mu and out
+// nullable), acc_out = acc_in + out (both nullable, may alias); A: 6 work fields.
+cudaError_t launch_ad_stage64(const FieldGeom& g, int order, const Topology& tp, const SbpT& t,
+                              const double* qw, const double* m, double ghs, double grav, const double* y,
+                              const double* lam, const double* mu, double alpha, double beta, double* A,
+                              double* out, const double* acc_in, double* acc_out, cudaStream_t st);
+// Adjoint stage pieces of the FP32 form (order = SBP order of the context;
 // m = metric of the element type; qw = FP64 sync weights):
 // zeta = pre-sync curl rJ (Dx v - Dy u) of the state y, boundary values also
 // into the EV_ZETA slots of the edge buffer Z;

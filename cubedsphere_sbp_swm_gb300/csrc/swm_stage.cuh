@@ -151,17 +151,16 @@ __device__ __forceinline__ void node_tendency(T gx, T gy, T zeta, T dv, T f, T J
 //   - panel-boundary nodes form their neighbours' pre-sync terms themselves, a
 //     lane for their own panel and one for the neighbour's, in warps that start
 //     first, instead of a second launch that exchanges them (one lane for
-//     both: 0.126 against 0.073 ms a step at N=48);
+//     both: 0.126 against 0.073 ms a step at N=48, before the Taps);
 //   - differences are taken before they are scaled, and the constants come
 //     from the host: 32 FP64 instructions a node and 11 for the stencil inputs
 //     (4/2), against 58; with constants formed per thread 50 instead of 45
 //     (0.343 against 0.306 ms a step).
-// Measured, RK4 steps d42 of one instance: N=48 0.239 -> 0.073 ms, N=192 0.251
-// -> 0.125 ms, N=384 0.560 -> 0.342 ms (0.090, 0.139 and 0.371 with the
-// boundary nodes in a launch of their own).  The FP64 pipe is 82% busy in a
-// launch at N=384.  Blocks of 64 and 256 threads measured within 1% of 128;
-// registers capped for 6, 7 or 8 blocks an SM (96 uncapped, 5 blocks) are 0.7%
-// faster at N=384 with three instances, 9 to 17% slower at N <= 201.
+// Measured, RK4 steps d42 of one instance: N=48 0.239 -> 0.052 ms, N=192 0.251
+// -> 0.112 ms, N=384 0.560 -> 0.351 ms.  The FP64 pipe is 82% busy in a launch
+// at N=384.  Blocks of 64 and 256 threads measured within 1% of 128; compiled
+// for 4 blocks an SM 4% slower at N=384 and 8% faster at N=48 than for 5, for 7
+// the reverse.
 // ---------------------------------------------------------------------------
 constexpr int PT_TPB = 128;
 
@@ -245,20 +244,68 @@ __device__ __forceinline__ T d_scaled(const T (&c)[3], F dif) {
   return s;
 }
 
-// Pre-sync gx, gy, curl and divergence of a node from the stencil inputs.
+// The SBP derivative at line index k as one row of taps: sum_m c[m] f(s + m),
+// closure or interior alike, zero past the row.  No branch separates the loads
+// of one derivative from the next, so a panel-boundary node waits for memory
+// once a direction and not once a derivative (with d_line in its place the RK4
+// step took 0.085 ms at N=48 and 0.141 at N=192, against 0.052 and 0.112).
+template <int ORD>
+struct Taps {
+  static constexpr int NT = Ord<ORD>::NW > 2 * Ord<ORD>::H + 1 ? Ord<ORD>::NW : 2 * Ord<ORD>::H + 1;
+  int s;
+  double c[NT];
+};
+template <int ORD>
+__device__ __forceinline__ Taps<ORD> taps_of(int k, int n) {
+  constexpr int NE = Ord<ORD>::NE, NT = Taps<ORD>::NT, ID = Ord<ORD>::idx, H = Ord<ORD>::H;
+  Taps<ORD> t;
+  const bool left = k < NE, right = k >= n - NE;
+  const int r = left ? k : right ? n - 1 - k : 0, last = c_sbp[ID].last[r];
+  t.s = left ? 0 : right ? n - NT : k - H;
+#pragma unroll
+  for (int m = 0; m < NT; ++m) {
+    const int mm = right ? NT - 1 - m : m;
+    const double q = mm < last && mm < MAXNW ? c_sbp[ID].Ql[r * MAXNW + mm] : 0.0;
+    t.c[m] = left ? q : right ? -q : m <= 2 * H ? c_sbp[ID].Qin[m <= 2 * H ? m : 0] : 0.0;
+  }
+  return t;
+}
+// f at the node, st the stride along the line, k the node's line index
+template <int ORD>
+__device__ __forceinline__ double taps_sum(const Taps<ORD>& t, const double* __restrict__ f, int k, int st) {
+  const double* q = f + (long long)(t.s - k) * st;
+  double v[Taps<ORD>::NT], s = 0.0;
+#pragma unroll
+  for (int m = 0; m < Taps<ORD>::NT; ++m) v[m] = __ldg(q + m * st);
+#pragma unroll
+  for (int m = 0; m < Taps<ORD>::NT; ++m) s += t.c[m] * v[m];
+  return s;
+}
+
+// Pre-sync gx, gy, curl and divergence of any node from the stencil inputs.
 template <int ORD, class T>
 __device__ __forceinline__ void raw_terms(const InstDev<T>& I, int p, int i, int j, T& gx, T& gy, T& zeta,
                                           T& dv) {
   const int n = I.n, P = I.P;
   const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
-  auto dx = [&](const T* q) { return d_line<ORD, T>(i, n, [&](int m) { return q[x + (m - i)]; }); };
-  auto dy = [&](const T* q) { return d_line<ORD, T>(j, n, [&](int m) { return q[x + (m - j) * P]; }); };
   const T rJ = I.metric[MRJ * fs + x];
-  const T* K = I.der + DR_K2 * fs;
-  gx = dx(K) * I.ghs2;
-  gy = dy(K) * I.ghs2;
-  zeta = (dx(I.in + 2 * fs) - dy(I.in + fs)) * rJ;
-  dv = (dx(I.der + DR_GU * fs) + dy(I.der + DR_GV * fs)) * rJ;
+  const T *K = I.der + DR_K2 * fs + x, *GU = I.der + DR_GU * fs + x, *GV = I.der + DR_GV * fs + x;
+  const T *U = I.in + fs + x, *V = I.in + 2 * fs + x;
+  T z, d;
+  {
+    const Taps<ORD> t = taps_of<ORD>(i, n);
+    gx = taps_sum<ORD>(t, K, i, 1) * I.ghs2;
+    z = taps_sum<ORD>(t, V, i, 1);
+    d = taps_sum<ORD>(t, GU, i, 1);
+  }
+  {
+    const Taps<ORD> t = taps_of<ORD>(j, n);
+    gy = taps_sum<ORD>(t, K, j, P) * I.ghs2;
+    z -= taps_sum<ORD>(t, U, j, P);
+    d += taps_sum<ORD>(t, GV, j, P);
+  }
+  zeta = z * rJ;
+  dv = d * rJ;
 }
 
 // Threads of one instance: the panel-boundary nodes (two lanes each), the
@@ -277,8 +324,44 @@ __host__ __device__ inline PointRanges point_ranges(int n) {
   return r;
 }
 
+// Node of thread tid of these ranges; false where it has none.  The lanes of
+// boundary blocks past the last node stay (live false) for the shuffles of the
+// pairs; the even lane of a pair is the node's own.
+struct PointAt {
+  int p, i, j;
+  bool boundary, live;
+};
+template <int ORD>
+__device__ __forceinline__ bool point_at(int n, int tid, PointAt& o) {
+  constexpr int NE = Ord<ORD>::NE;
+  const PointRanges rg = point_ranges<ORD>(n);
+  o.live = true;
+  o.boundary = tid < rg.nb;
+  if (o.boundary) {
+    const int nb = 4 * n - 4, t = min(tid >> 1, 6 * nb - 1);
+    o.live = (tid >> 1) < 6 * nb;
+    o.p = t / nb;
+    boundary_node(t - o.p * nb, n, o.i, o.j);
+    return true;
+  }
+  if (tid < rg.closed) {   // along the column: rows 1..n-2
+    const int t = tid - rg.nb, r = t / (n - 2);
+    if (r >= 12 * (NE - 1)) return false;
+    o.j = 1 + t - r * (n - 2);
+    const int s = r / (NE > 1 ? NE - 1 : 1), c = 1 + r - s * (NE - 1);
+    o.i = (s & 1) ? n - 1 - c : c;
+    o.p = s >> 1;
+    return true;
+  }
+  const int t = tid - rg.closed, ni = n - 2 * NE, row = t / ni;
+  o.p = row / (n - 2);
+  o.j = 1 + row - o.p * (n - 2);
+  o.i = NE + t - row * ni;
+  return o.p < 6;
+}
+
 template <class T, int ORD, int MODE>
-__global__ void __launch_bounds__(PT_TPB)
+__global__ void __launch_bounds__(PT_TPB, 5)
     point_stage_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many,
                        const __grid_constant__ Topology tp) {
   constexpr int NE = Ord<ORD>::NE;
@@ -286,26 +369,9 @@ __global__ void __launch_bounds__(PT_TPB)
   constexpr bool needA = MODE == MODE_RK2 || MODE == MODE_RK3 || MODE == MODE_RK4;
   const InstDev<T>& I = many ? many[blockIdx.y] : one;
   const int n = I.n, P = I.P, tid = blockIdx.x * PT_TPB + threadIdx.x;
-  const PointRanges rg = point_ranges<ORD>(n);
-  int p, i, j;
-  if (tid < rg.nb) {
-    const int nb = 4 * n - 4, t = min(tid >> 1, 6 * nb - 1);   // surplus lanes stay for the shuffles
-    p = t / nb;
-    boundary_node(t - p * nb, n, i, j);
-  } else if (tid < rg.closed) {   // along the column: rows 1..n-2
-    const int t = tid - rg.nb, r = t / (n - 2);
-    if (r >= 12 * (NE - 1)) return;
-    j = 1 + t - r * (n - 2);
-    const int s = r / (NE > 1 ? NE - 1 : 1), c = 1 + r - s * (NE - 1);
-    i = (s & 1) ? n - 1 - c : c;
-    p = s >> 1;
-  } else {
-    const int t = tid - rg.closed, ni = n - 2 * NE, row = t / ni;
-    p = row / (n - 2);
-    if (p >= 6) return;
-    j = 1 + row - p * (n - 2);
-    i = NE + t - row * ni;
-  }
+  PointAt at;
+  if (!point_at<ORD>(n, tid, at)) return;
+  const int p = at.p, i = at.i, j = at.j;
   const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
   T rb[3] = {}, ra[3] = {}, rl[3] = {};
 #pragma unroll
@@ -316,7 +382,7 @@ __global__ void __launch_bounds__(PT_TPB)
   const T f = I.metric[MF * fs + x];
   const T jut = I.der[DR_JUT * fs + x], jvt = I.der[DR_JVT * fs + x];
   T kh, ku, kv;
-  if (tid < rg.nb) {
+  if (at.boundary) {
     // A boundary node: one lane forms the raw terms of its own panel, the other
     // those of the panels that hold copies of it (formed here again rather
     // than exchanged); then their sync (2-way average on edges, 3-way at cube
@@ -355,36 +421,41 @@ __global__ void __launch_bounds__(PT_TPB)
     sgy += __shfl_xor_sync(0xffffffffu, sgy, 1);
     sz += __shfl_xor_sync(0xffffffffu, sz, 1);
     sd += __shfl_xor_sync(0xffffffffu, sd, 1);
-    if (!own || (tid >> 1) >= 6 * (4 * n - 4)) return;
+    if (!own || !at.live) return;
     const T w = lr && bt ? T(1.0 / 3.0) : T(0.5);
     const T fz = f + w * sz;
     kh = -(w * sd);
     ku = fz * jvt - w * sgx;
     kv = -(fz * jut) - w * sgy;
   } else {
-    const T* __restrict__ K = I.der + DR_K2 * fs + x;
-    const T* __restrict__ GU = I.der + DR_GU * fs + x;
-    const T* __restrict__ GV = I.der + DR_GV * fs + x;
-    const T* __restrict__ U = I.in + fs + x;
-    const T* __restrict__ V = I.in + 2 * fs + x;
-    T rJ = I.metric[MRJ * fs + x];
-    T gx, gy, zw, dw;   // zw, dw: the curl and the divergence before the factor rJ
+    T gx, gy, fz;
     if (i >= NE && i < n - NE && j >= NE && j < n - NE) {
+      const T* __restrict__ K = I.der + DR_K2 * fs + x;
+      const T* __restrict__ GU = I.der + DR_GU * fs + x;
+      const T* __restrict__ GV = I.der + DR_GV * fs + x;
+      const T* __restrict__ U = I.in + fs + x;
+      const T* __restrict__ V = I.in + 2 * fs + x;
+      const T rJ = I.metric[MRJ * fs + x] * T(d_coef<ORD>(1));
       gx = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o] - K[-o]; });
       gy = d_scaled<ORD, T>(I.gc, [&](int o) { return K[o * P] - K[-o * P]; });
-      zw = d_ratio<ORD, T>([&](int o) { return (V[o] - V[-o]) - (U[o * P] - U[-o * P]); });
-      dw = d_ratio<ORD, T>([&](int o) { return (GU[o] - GU[-o]) + (GV[o * P] - GV[-o * P]); });
-      rJ = rJ * T(d_coef<ORD>(1));
+      const T zw = d_ratio<ORD, T>([&](int o) { return (V[o] - V[-o]) - (U[o * P] - U[-o * P]); });
+      const T dw = d_ratio<ORD, T>([&](int o) { return (GU[o] - GU[-o]) + (GV[o * P] - GV[-o * P]); });
+      fz = f + zw * rJ;
+      kh = -(dw * rJ);
     } else {
+      const T* __restrict__ K = I.der + DR_K2 * fs + x;
+      const T* __restrict__ GU = I.der + DR_GU * fs + x;
+      const T* __restrict__ GV = I.der + DR_GV * fs + x;
+      const T* __restrict__ U = I.in + fs + x;
+      const T* __restrict__ V = I.in + 2 * fs + x;
+      const T rJ = I.metric[MRJ * fs + x];
       auto dx = [&](const T* q) { return d_line<ORD, T>(i, n, [&](int m) { return q[m - i]; }); };
       auto dy = [&](const T* q) { return d_line<ORD, T>(j, n, [&](int m) { return q[(m - j) * P]; }); };
       gx = dx(K) * I.ghs2;
       gy = dy(K) * I.ghs2;
-      zw = dx(V) - dy(U);
-      dw = dx(GU) + dy(GV);
+      fz = f + (dx(V) - dy(U)) * rJ;
+      kh = -((dx(GU) + dy(GV)) * rJ);
     }
-    const T fz = f + zw * rJ;
-    kh = -(dw * rJ);
     ku = fz * jvt - gx;
     kv = -(fz * jut) - gy;
   }

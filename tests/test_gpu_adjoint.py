@@ -58,6 +58,22 @@ def test_operator_dot_product(setup):
     assert abs(a - b) <= 1e-10 * max(abs(a), abs(b))
 
 
+# The FP64 adjoint kernels number boundary pairs, closure columns and inner
+# nodes apart: the smallest panel of each order, whole warps and one node more.
+# Random fields, so that the copies of an edge node differ.
+@pytest.mark.parametrize("order,n_cells", [(42, 16), (43, 17), (63, 24), (42, 39), (63, 50)])
+def test_operator_dot_product_small_panels(order, n_cells):
+    op = swm.OperatorSWM(swm.ModelConfig(N=n_cells, sbp_order=order))
+    rng = np.random.default_rng(n_cells)
+    y = _stvec(op, initial.balanced_zonal(n_cells, 3, 8)[:3])
+    dx, lk = _rand(rng, op), _rand(rng, op)
+    dk, lx = op.create_stvec(), op.create_stvec()
+    ad.apply_tl(op, y, _stvec(op, dx), dk)
+    ad.apply_ad(op, y, _stvec(op, lk), lx)
+    a, b = _dot(dk.download(), lk), _dot(dx, lx.download())
+    assert abs(a - b) <= 1e-10 * max(abs(a), abs(b))
+
+
 def test_tangent_linear_matches_central_differences(setup):
     op, x0 = setup
     rng = np.random.default_rng(12)
