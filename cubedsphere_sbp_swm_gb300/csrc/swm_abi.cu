@@ -254,6 +254,7 @@ long long round_up(long long a, long long b) { return (a + b - 1) / b * b; }
 // members share one launch).
 constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
 constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
+constexpr int kSpread = 152;           // units that give every SM of a GB300 one
 double row_closure_cost(const SbpC& s) { return s.ne >= 6 ? 2.0 : 1.0; }
 
 bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<WorkUnit>& out,
@@ -316,12 +317,16 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
       cut_equal(k, std::max(1, std::min(n, (int)std::lround(m))));
     }
   } else {
-    // At least 3 rows a unit.  On a panel too small to fill the GPU the row
-    // loop of a unit is the launch's latency: N=48 d42 FP32, width 128, took
-    // 51.4 us a step at 8 rows a unit, 41.3 at 3 and 39.2 at 2 (one instance
-    // at a time; three at once 18.4, 15.9 and 18.9: the halo rows of shorter
-    // units are then paid for).
-    const int max_units = std::max(1, n / 3);
+    // At least 8 rows a unit; 3, up to a unit per SM, where 8 rows would leave
+    // half of the SMs without one.  On a panel too small to fill the GPU the
+    // row loop of a unit is the launch's latency; on a larger one shorter units
+    // only add halo rows.  d42 FP32, width 128, us a step of one instance / of
+    // three at once: N=48 51.4/18.4 at 8 rows, 41.3/15.9 at 3; N=96 49.4/19.1 at
+    // 8, 43.3/17.7 at 4; N=120 54.4/21.3 at 8, 48.2/23.1 at 4; N=144 54.4/26.8 at
+    // 8, 49.5/28.2 at 4.  (The ensemble's units are bounded by its own budget.)
+    const int at8 = std::max(1, n / std::min(8, n));
+    const int spread = 2 * 6 * nstrip * at8 <= kSpread ? kSpread / (6 * nstrip) : 0;
+    const int max_units = tau_fixed > 0.0 ? n / 3 : std::max(at8, std::min(n / 3, spread));
     // units of strip k for a unit cost of at most tau: m units of a strip of
     // factor f cost f * (pre[n] + m * over) in total
     auto units_of = [&](int k, double tau) {
