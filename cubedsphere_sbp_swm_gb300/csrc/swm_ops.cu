@@ -173,49 +173,163 @@ __global__ void ke_update_kernel(FieldGeom g, double grav, const double* h, cons
   ke[x] = ke[x] + grav * h[x] + grav * (hs ? hs[x] : 0.0);
 }
 
-// SBP derivative with a runtime operator index (table in constant memory).
-template <class FA>
-__device__ __forceinline__ double d_line_rt(int id, int k, int n, FA fa) {
-  const SbpC& s = c_sbp[id];
-  double acc = 0.0;
-  if (k < s.ne) {
-    for (int m = 0; m < s.last[k]; ++m) acc += s.Ql[k * MAXNW + m] * fa(m);
-  } else if (k >= n - s.ne) {
-    const int r = n - 1 - k;
-    for (int m = s.last[r] - 1; m >= 0; --m) acc += (-s.Ql[r * MAXNW + m]) * fa(n - 1 - m);
-  } else {
-    for (int t = 0; t < s.nin; ++t) acc += s.Qin[t] * fa(k + s.inshift + t);
+// Differential operators with their cube-edge syncs in one launch, on the
+// node ranges of the FP64 stage kernel (swm_stage.cuh): straight-line interior,
+// closure columns in warps of their own, and a boundary node's own and
+// neighbour terms formed by two lanes.  FP64 bounds the interior and latency
+// the small panels; as a pass over table-driven stencils (the curl with the
+// reference's J (v / J), two divisions a tap) and two sync launches, the curl
+// at N=130 took 61 us a call with its synchronisation, the divergence 34 and the
+// gradient 30; each now 25.
+struct OpArgs {
+  FieldGeom g;
+  const double *a, *b, *m, *qw;   // a, b: input fields (grad: a)
+  double s;                        // grad: 1 / (hx a)
+  double *o1, *o2;
+};
+
+// The copies of a boundary node: raw(p, i, j, L) is called for the node itself
+// (even lane, L null) and for the neighbours' nodes at the same point (odd
+// lane, L the link that led there and slr whether it crosses a left / right
+// side); its results x, y add up over the copies of both lanes.
+template <class F>
+__device__ __forceinline__ void over_copies(const Topology& tp, int n, int tid, const PointAt& at, F raw,
+                                            double& x, double& y) {
+  const int e = n - 1, i = at.i, j = at.j;
+  const bool lr = (i == 0) | (i == e), bt = (j == 0) | (j == e), own = (tid & 1) == 0;
+  x = y = 0.0;
+  const int copies = !own && lr && bt ? 2 : 1;
+#pragma unroll 1
+  for (int s = 0; s < copies; ++s) {
+    const bool slr = lr && s == 0;
+    int q = at.p, iq = i, jq = j;
+    EdgeLink L{};
+    if (!own) {
+      L = tp.link[at.p][slr ? (i == 0 ? SIDE_L : SIDE_R) : (j == 0 ? SIDE_B : SIDE_T)];
+      const int k = slr ? j : i, kk = L.rev ? e - k : k;
+      q = L.q;
+      iq = L.side_q == SIDE_L ? 0 : L.side_q == SIDE_R ? e : kk;
+      jq = L.side_q == SIDE_B ? 0 : L.side_q == SIDE_T ? e : kk;
+    }
+    double a, b;
+    raw(q, iq, jq, own ? nullptr : &L, slr, a, b);
+    x += a;
+    y += b;
   }
-  return acc;
+  x += __shfl_xor_sync(0xffffffffu, x, 1);
+  y += __shfl_xor_sync(0xffffffffu, y, 1);
+}
+__device__ __forceinline__ double copy_weight(int n, const PointAt& at) {
+  const bool lr = (at.i == 0) | (at.i == n - 1), bt = (at.j == 0) | (at.j == n - 1);
+  return lr && bt ? 1.0 / 3.0 : 0.5;
 }
 
-__global__ void grad_kernel(FieldGeom g, int id, double ghs, const double* f, double* gx,
-                            double* gy) {
-  const long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= 6LL * g.n * g.n) return;
-  const NodeIx k = node_of(g, gi);
-  const double* F = f + (long long)k.p * g.ps;
-  const double dx = d_line_rt(id, k.i, g.n, [&](int m) { return F[(long long)k.j * g.P + m]; });
-  const double dy = d_line_rt(id, k.j, g.n, [&](int m) { return F[(long long)m * g.P + k.i]; });
-  gx[k.idx] = dx * ghs;
-  gy[k.idx] = dy * ghs;
+// grad_ah_sbp_t%calc_grad (grad_ah_sbp_mod.f90:26-90) with its covariant sync
+// (ecs_Ah_vec_sync_mod.f90:62-125)
+template <int ORD>
+__global__ void __launch_bounds__(PT_TPB)
+    grad_kernel(const __grid_constant__ OpArgs a, const __grid_constant__ Topology tp) {
+  constexpr int NE = Ord<ORD>::NE;
+  const FieldGeom& g = a.g;
+  const int n = g.n, P = g.P, tid = blockIdx.x * PT_TPB + threadIdx.x;
+  PointAt at;
+  if (!point_at<ORD>(n, tid, at)) return;
+  const int i = at.i, j = at.j;
+  const long long x = (long long)at.p * g.ps + (long long)j * P + i;
+  auto raw = [&](int p, int ii, int jj, double& gx, double& gy) {
+    const double* f = a.a + (long long)p * g.ps + (long long)jj * P + ii;
+    gx = a.s * taps_sum<ORD>(taps_of<ORD>(ii, n), f, ii, 1);
+    gy = a.s * taps_sum<ORD>(taps_of<ORD>(jj, n), f, jj, P);
+  };
+  double gx, gy;
+  if (at.boundary) {
+    over_copies(tp, n, tid, at, [&](int p, int ii, int jj, const EdgeLink* L, bool slr, double& ax, double& ay) {
+      raw(p, ii, jj, ax, ay);
+      if (!L) return;
+      const double rx = L->dim_i ? L->istep * ax : L->jstep * ay;
+      const double ry = L->dim_i ? L->jstep * ay : L->istep * ax;
+      ax = slr ? rx + a.qw[(i == 0 ? 2 : 3) * n + j] * ry : rx;
+      ay = slr ? ry : ry + a.qw[(j == 0 ? 0 : 1) * n + i] * rx;
+    }, gx, gy);
+    if ((tid & 1) || !at.live) return;
+    const double w = copy_weight(n, at);
+    gx *= w;
+    gy *= w;
+  } else if (i >= NE && i < n - NE && j >= NE && j < n - NE) {
+    const double* f = a.a + x;
+    const double c = a.s * d_coef<ORD>(1);
+    gx = c * d_ratio<ORD, double>([&](int o) { return f[o] - f[-o]; });
+    gy = c * d_ratio<ORD, double>([&](int o) { return f[o * P] - f[-o * P]; });
+  } else {
+    raw(at.p, i, j, gx, gy);
+  }
+  a.o1[x] = gx;
+  a.o2[x] = gy;
 }
 
-__global__ void div_kernel(FieldGeom g, int id, double hx_a, const double* mt, const double* u,
-                           const double* v, int curl_form, double* out) {
-  const long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= 6LL * g.n * g.n) return;
-  const NodeIx k = node_of(g, gi);
-  const long long pb = (long long)k.p * g.ps;
-  const double* J = mt + MJ * g.fs + pb;
-  const double* U = u + pb;
-  const double* V = v + pb;
-  // Gu = J*u, Gv = J*v; for the curl, (u', v') = (v/J, -u/J) first
-  auto gu = [&](long long o) { return curl_form ? J[o] * (V[o] / J[o]) : J[o] * U[o]; };
-  auto gv = [&](long long o) { return curl_form ? J[o] * (-U[o] / J[o]) : J[o] * V[o]; };
-  const double dx = d_line_rt(id, k.i, g.n, [&](int m) { return gu((long long)k.j * g.P + m); });
-  const double dy = d_line_rt(id, k.j, g.n, [&](int m) { return gv((long long)m * g.P + k.i); });
-  out[k.idx] = (dx + dy) / (mt[MJ * g.fs + k.idx] * hx_a);
+// Pre-sync curl (Dx b - Dy a) / (J hx a) of the covariant (a, b), or
+// divergence (Dx(J a) + Dy(J b)) / (J hx a) of the contravariant ones, at any
+// node.
+template <int ORD, bool CURL>
+__device__ __forceinline__ double div_raw(const OpArgs& A, int p, int i, int j) {
+  const FieldGeom& g = A.g;
+  const int n = g.n, P = g.P;
+  const long long x = (long long)p * g.ps + (long long)j * P + i;
+  const Taps<ORD> tx = taps_of<ORD>(i, n), ty = taps_of<ORD>(j, n);
+  double s;
+  if (CURL) {
+    s = taps_sum<ORD>(tx, A.b + x, i, 1) - taps_sum<ORD>(ty, A.a + x, j, P);
+  } else {
+    const double* J = A.m + MJ * g.fs + x;
+    s = 0.0;
+#pragma unroll
+    for (int k = 0; k < Taps<ORD>::NT; ++k) {
+      const int ox = tx.s + k - i, oy = (ty.s + k - j) * P;
+      s += tx.c[k] * (J[ox] * A.a[x + ox]);
+      s += ty.c[k] * (J[oy] * A.b[x + oy]);
+    }
+  }
+  return s * A.m[MRJ * g.fs + x];
+}
+// The synced value at a node; live false for lanes that store nothing.
+template <int ORD, bool CURL>
+__device__ __forceinline__ double div_synced(const OpArgs& A, const Topology& tp, int tid, const PointAt& at,
+                                             bool& live) {
+  constexpr int NE = Ord<ORD>::NE;
+  const FieldGeom& g = A.g;
+  const int n = g.n, P = g.P, i = at.i, j = at.j;
+  live = true;
+  if (at.boundary) {
+    double d, unused;
+    over_copies(tp, n, tid, at, [&](int p, int ii, int jj, const EdgeLink*, bool, double& v, double& w) {
+      v = div_raw<ORD, CURL>(A, p, ii, jj);
+      w = 0.0;
+    }, d, unused);
+    live = !(tid & 1) && at.live;
+    return d * copy_weight(n, at);
+  }
+  if (!(i >= NE && i < n - NE && j >= NE && j < n - NE)) return div_raw<ORD, CURL>(A, at.p, i, j);
+  const long long x = (long long)at.p * g.ps + (long long)j * P + i;
+  const double *U = A.a + x, *V = A.b + x, *J = A.m + MJ * g.fs + x;
+  const double rJ = A.m[MRJ * g.fs + x] * d_coef<ORD>(1);
+  if (CURL)
+    return rJ * d_ratio<ORD, double>([&](int o) { return (V[o] - V[-o]) - (U[o * P] - U[-o * P]); });
+  return rJ * d_ratio<ORD, double>([&](int o) {
+           return (J[o] * U[o] - J[-o] * U[-o]) + (J[o * P] * V[o * P] - J[-o * P] * V[-o * P]);
+         });
+}
+
+// curl_div_based_t%calc_curl (curl_div_based_mod.f90:26-66) and
+// div_ah_sbp_t%calc_div (div_ah_sbp_mod.f90:24-98), synced
+template <int ORD, bool CURL>
+__global__ void __launch_bounds__(PT_TPB)
+    div_kernel(const __grid_constant__ OpArgs a, const __grid_constant__ Topology tp) {
+  const int tid = blockIdx.x * PT_TPB + threadIdx.x;
+  PointAt at;
+  if (!point_at<ORD>(a.g.n, tid, at)) return;
+  bool live;
+  const double d = div_synced<ORD, CURL>(a, tp, tid, at, live);
+  if (live) a.o1[(long long)at.p * a.g.ps + (long long)at.j * a.g.P + at.i] = d;
 }
 
 __global__ void coriolis_kernel(FieldGeom g, const double* m, const double* hu, const double* hv,
@@ -296,68 +410,103 @@ __global__ void sync_vector_kernel(FieldGeom g, Topology tp, const double* qw, c
 // Deterministic reductions: fixed grid, per-block tree, then one block sums
 // the partials in a fixed order.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double red_op(int kind, double x, double y) {
-  return kind == 2 ? fmin(x, y) : kind == 3 ? fmax(x, y) : x + y;
-}
-
 __global__ void reduce_partial_kernel(FieldGeom g, int kind, const double* a, const double* b,
                                       const double* J, const double* Aw, double hx2,
                                       double* partial) {
   __shared__ double sh[TPB];
   const long long total = 6LL * g.n * g.n;
-  const double init = kind == 2 ? INFINITY : kind == 3 ? -INFINITY : 0.0;
-  double acc = init;
+  double acc = 0.0;
   for (long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x; gi < total;
        gi += (long long)gridDim.x * blockDim.x) {
     const NodeIx k = node_of(g, gi);
     double val = a[k.idx];
     if (kind == 0 && b) val = val * b[k.idx];
-    if (kind == 1 || kind == 4) {
-      if (kind == 4) val = val * b[k.idx];
-      val = val * J[k.idx] * hx2 * Aw[k.i] * Aw[k.j];
-    }
-    acc = red_op(kind, acc, val);
+    if (kind == 1) val = val * J[k.idx] * hx2 * Aw[k.i] * Aw[k.j];
+    acc += val;
   }
   sh[threadIdx.x] = acc;
   __syncthreads();
   for (int s = TPB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] = red_op(kind, sh[threadIdx.x], sh[threadIdx.x + s]);
+    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
     __syncthreads();
   }
   if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
-__global__ void reduce_final_kernel(int kind, const double* partial, int np, double* result) {
+__global__ void reduce_final_kernel(const double* partial, int np, double* result) {
   __shared__ double sh[TPB];
-  const double init = kind == 2 ? INFINITY : kind == 3 ? -INFINITY : 0.0;
-  double acc = init;
-  for (int k = threadIdx.x; k < np; k += blockDim.x) acc = red_op(kind, acc, partial[k]);
+  double acc = 0.0;
+  for (int k = threadIdx.x; k < np; k += blockDim.x) acc += partial[k];
   sh[threadIdx.x] = acc;
   __syncthreads();
   for (int s = TPB / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] = red_op(kind, sh[threadIdx.x], sh[threadIdx.x + s]);
+    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
     __syncthreads();
   }
   if (threadIdx.x == 0) *result = sh[0];
 }
 
-__global__ void diag_kernel(FieldGeom g, const double* m, double grav, const double* h,
-                            const double* u, const double* v, const double* hs, const double* z,
-                            double* ke_u, double* ke_v, double* pe, double* ens) {
-  const long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= 6LL * g.n * g.n) return;
-  const long long x = node_of(g, gi).idx;
-  const double q1 = m[MQI1 * g.fs + x], q2 = m[MQI2 * g.fs + x], q3 = m[MQI3 * g.fs + x];
-  const double ut = q1 * u[x] + q2 * v[x];
-  const double vt = q2 * u[x] + q3 * v[x];
-  const double hu = 1.0 * h[x] * ut, hv = 1.0 * h[x] * vt;
-  ke_u[x] = 0.5 * hu * u[x];
-  ke_v[x] = 0.5 * hv * v[x];
-  const double ph = 1.0 * h[x] + 1.0 * (hs ? hs[x] : 0.0);
-  pe[x] = 0.5 * grav * ph * ph;
-  double c = z[x] + 1.0 * m[MF * g.fs + x];
-  c = 0.5 * c * c;
-  ens[x] = 1.0 * c / h[x];
+// The seven global values of get_diagnostics (operator_swm_mod.f90:115-155) in
+// one pass: minimum and maximum of h, and the SBP integrals of h, of the kinetic
+// and potential energy and of the enstrophy, with the synced curl formed where
+// it is used.  Per-block trees, then one block over the partials in a fixed
+// order: two launches instead of 19 (curl, syncs, integrands and a pair of
+// launches per value), 158 -> 66 us a call at N=130.
+constexpr int DIAG_N = 6;   // hmin, hmax, mass, KE, PE, enstrophy
+
+__device__ __forceinline__ double diag_op(int k, double x, double y) {
+  return k == 0 ? fmin(x, y) : k == 1 ? fmax(x, y) : x + y;
+}
+
+template <int ORD>
+__global__ void __launch_bounds__(PT_TPB)
+    diag_kernel(const __grid_constant__ OpArgs a, const __grid_constant__ Topology tp, const double* h,
+                const double* hs, const double* Aw, double grav, double hx2, int threads, double* partial) {
+  const FieldGeom& g = a.g;
+  const int n = g.n;
+  const long long fs = g.fs;
+  double r[DIAG_N] = {INFINITY, -INFINITY, 0.0, 0.0, 0.0, 0.0};
+  // whole blocks of nodes a turn, so that the lanes of a pair stay together
+  for (int t0 = blockIdx.x * PT_TPB; t0 < threads; t0 += gridDim.x * PT_TPB) {
+    PointAt at;
+    const int tid = t0 + threadIdx.x;
+    if (!point_at<ORD>(n, tid, at)) continue;
+    bool live;
+    const double z = div_synced<ORD, true>(a, tp, tid, at, live);
+    if (!live) continue;
+    const long long x = (long long)at.p * g.ps + (long long)at.j * g.P + at.i;
+    const double u = a.a[x], v = a.b[x], hh = h[x], q2 = a.m[MQI2 * fs + x];
+    const double ut = a.m[MQI1 * fs + x] * u + q2 * v, vt = q2 * u + a.m[MQI3 * fs + x] * v;
+    const double w = a.m[MJ * fs + x] * hx2 * Aw[at.i] * Aw[at.j];
+    const double ph = hs ? hh + hs[x] : hh, c = z + a.m[MF * fs + x];
+    r[0] = fmin(r[0], hh);
+    r[1] = fmax(r[1], hh);
+    r[2] += hh * w;
+    r[3] += (0.5 * hh * (ut * u + vt * v)) * w;
+    r[4] += (0.5 * grav * ph * ph) * w;
+    r[5] += (0.5 * c * c / hh) * w;
+  }
+  __shared__ double sh[DIAG_N][PT_TPB / 32];
+#pragma unroll
+  for (int k = 0; k < DIAG_N; ++k) {
+    for (int o = 16; o > 0; o >>= 1) r[k] = diag_op(k, r[k], __shfl_xor_sync(0xffffffffu, r[k], o));
+    if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = r[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < DIAG_N) {
+    double s = sh[threadIdx.x][0];
+    for (int t = 1; t < PT_TPB / 32; ++t) s = diag_op(threadIdx.x, s, sh[threadIdx.x][t]);
+    partial[threadIdx.x * gridDim.x + blockIdx.x] = s;
+  }
+}
+
+// one warp per value
+__global__ void diag_final_kernel(const double* partial, int np, double* result) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double s = k == 0 ? INFINITY : k == 1 ? -INFINITY : 0.0;
+  for (int t = lane; t < np; t += 32) s = diag_op(k, s, partial[k * np + t]);
+  for (int o = 16; o > 0; o >>= 1) s = diag_op(k, s, __shfl_xor_sync(0xffffffffu, s, o));
+  if (lane == 0) result[k] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -525,17 +674,30 @@ cudaError_t launch_ke_update(const FieldGeom& g, double grav, const double* h, c
   return cudaGetLastError();
 }
 
-cudaError_t launch_grad_presync(const FieldGeom& g, int order, double ghs, const double* f,
-                                double* gx, double* gy, cudaStream_t st) {
-  grad_kernel<<<nblk(6LL * g.n * g.n), TPB, 0, st>>>(g, sbp_index(order), ghs, f, gx, gy);
+#define SWM_BY_ORDER(order, call)                  \
+  switch (order) {                                 \
+    case 21: { constexpr int ORD = 21; call; } break; \
+    case 42: { constexpr int ORD = 42; call; } break; \
+    case 43: { constexpr int ORD = 43; call; } break; \
+    case 63: { constexpr int ORD = 63; call; } break; \
+    default: return cudaErrorInvalidValue;         \
+  }
+
+cudaError_t launch_grad(const FieldGeom& g, int order, const Topology& tp, const double* qw, double ghs,
+                        const double* f, double* gx, double* gy, cudaStream_t st) {
+  const OpArgs a{g, f, nullptr, nullptr, qw, ghs, gx, gy};
+  SWM_BY_ORDER(order, (grad_kernel<ORD><<<point_ranges<ORD>(g.n).total / PT_TPB, PT_TPB, 0, st>>>(a, tp)));
   return cudaGetLastError();
 }
 
-cudaError_t launch_div_presync(const FieldGeom& g, int order, double hx_a, const double* m64,
-                               const double* u, const double* v, int curl_form, double* out,
-                               cudaStream_t st) {
-  div_kernel<<<nblk(6LL * g.n * g.n), TPB, 0, st>>>(g, sbp_index(order), hx_a, m64, u, v,
-                                                     curl_form, out);
+cudaError_t launch_div(const FieldGeom& g, int order, const Topology& tp, const double* m64, const double* u,
+                       const double* v, bool curl, double* out, cudaStream_t st) {
+  const OpArgs a{g, u, v, m64, nullptr, 0.0, out, nullptr};
+  if (curl) {
+    SWM_BY_ORDER(order, (div_kernel<ORD, true><<<point_ranges<ORD>(g.n).total / PT_TPB, PT_TPB, 0, st>>>(a, tp)));
+  } else {
+    SWM_BY_ORDER(order, (div_kernel<ORD, false><<<point_ranges<ORD>(g.n).total / PT_TPB, PT_TPB, 0, st>>>(a, tp)));
+  }
   return cudaGetLastError();
 }
 
@@ -596,16 +758,22 @@ cudaError_t launch_reduce(const FieldGeom& g, int kind, const double* a, const d
                           const double* J, const double* Aw, double hx2, double* partial,
                           int nblocks, double* result, cudaStream_t st) {
   reduce_partial_kernel<<<nblocks, TPB, 0, st>>>(g, kind, a, b, J, Aw, hx2, partial);
-  reduce_final_kernel<<<1, TPB, 0, st>>>(kind, partial, nblocks, result);
+  reduce_final_kernel<<<1, TPB, 0, st>>>(partial, nblocks, result);
   return cudaGetLastError();
 }
 
-cudaError_t launch_diag_integrands(const FieldGeom& g, const double* m64, double grav,
-                                   const double* h, const double* u, const double* v,
-                                   const double* hs, const double* zeta, double* ke_u,
-                                   double* ke_v, double* pe, double* ens, cudaStream_t st) {
-  diag_kernel<<<nblk(6LL * g.n * g.n), TPB, 0, st>>>(g, m64, grav, h, u, v, hs, zeta, ke_u, ke_v,
-                                                      pe, ens);
+cudaError_t launch_diagnostics(const FieldGeom& g, int order, const Topology& tp, const double* m64,
+                               double grav, const double* h, const double* u, const double* v,
+                               const double* hs, const double* Aw, double hx2, double* partial,
+                               double* result, cudaStream_t st) {
+  const OpArgs a{g, u, v, m64, nullptr, 0.0, nullptr, nullptr};
+  int blocks = 0;
+  SWM_BY_ORDER(order, {
+    const int threads = point_ranges<ORD>(g.n).total;
+    blocks = threads / PT_TPB < DIAG_BLOCKS ? threads / PT_TPB : DIAG_BLOCKS;
+    (diag_kernel<ORD><<<blocks, PT_TPB, 0, st>>>(a, tp, h, hs, Aw, grav, hx2, threads, partial));
+  });
+  diag_final_kernel<<<1, 32 * DIAG_N, 0, st>>>(partial, blocks, result);
   return cudaGetLastError();
 }
 

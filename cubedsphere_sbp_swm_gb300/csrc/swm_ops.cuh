@@ -33,14 +33,13 @@ cudaError_t launch_ke(const FieldGeom& g, const double* u, const double* v, cons
 // ke += grav*h + grav*hs (hs nullable)
 cudaError_t launch_ke_update(const FieldGeom& g, double grav, const double* h, const double* hs,
                              double* ke, cudaStream_t st);
-// pre-sync SBP gradient: gx = Dx f / (hx a), gy = Dy f / (hx a)
-cudaError_t launch_grad_presync(const FieldGeom& g, int order, double ghs, const double* f,
-                                double* gx, double* gy, cudaStream_t st);
-// pre-sync SBP divergence (Dx(J u) + Dy(J v)) / (J hx a); curl_form: the
-// input is covariant and the operator uses (v/J, -u/J).
-cudaError_t launch_div_presync(const FieldGeom& g, int order, double hx_a, const double* m64,
-                               const double* u, const double* v, int curl_form, double* out,
-                               cudaStream_t st);
+// SBP gradient gx = Dx f / (hx a), gy = Dy f / (hx a) with its covariant sync
+cudaError_t launch_grad(const FieldGeom& g, int order, const Topology& tp, const double* qw, double ghs,
+                        const double* f, double* gx, double* gy, cudaStream_t st);
+// SBP divergence (Dx(J u) + Dy(J v)) / (J hx a) of contravariant (u, v), or
+// curl (Dx v - Dy u) / (J hx a) of covariant ones, with the scalar sync
+cudaError_t launch_div(const FieldGeom& g, int order, const Topology& tp, const double* m64, const double* u,
+                       const double* v, bool curl, double* out, cudaStream_t st);
 cudaError_t launch_coriolis(const FieldGeom& g, const double* m64, const double* hu,
                             const double* hv, const double* h, const double* curl,
                             double* cor_u, double* cor_v, cudaStream_t st);
@@ -115,20 +114,19 @@ cudaError_t launch_ad_main(const FieldGeom& g, int order, const SbpT& t, const T
 int adjoint_table_ct(int order);
 
 // Deterministic FP64 reductions over the valid nodes of a field.
-// kind: 0 sum(a*b), 1 SBP mass sum(a*J*hx^2*Ax*Ay), 2 min(a), 3 max(a),
-//       4 SBP mass of a*b.
+// kind: 0 sum(a*b), 1 SBP mass sum(a*J*hx^2*Ax*Ay).
 cudaError_t launch_reduce(const FieldGeom& g, int kind, const double* a, const double* b,
                           const double* J, const double* Aw, double hx2, double* partial,
                           int nblocks, double* result, cudaStream_t st);
 constexpr int REDUCE_BLOCKS = 264;
 
-// Per-node integrands of the SWM diagnostics (operator_swm_mod.f90:211-260):
-// ke_u = 0.5*(h*ut)*u, ke_v = 0.5*(h*vt)*v, pe = 0.5*g*(h+hs)^2,
-// ens = 0.5*(zeta+f)^2/h.
-cudaError_t launch_diag_integrands(const FieldGeom& g, const double* m64, double grav,
-                                   const double* h, const double* u, const double* v,
-                                   const double* hs, const double* zeta, double* ke_u,
-                                   double* ke_v, double* pe, double* ens, cudaStream_t st);
+// The SWM diagnostics (operator_swm_mod.f90:211-260): hmin, hmax, mass, KE, PE and enstrophy into result[6]; partial holds
+// 6 * DIAG_BLOCKS values
+constexpr int DIAG_BLOCKS = 1216;   // 8 blocks of 128 threads on each of 152 SMs
+cudaError_t launch_diagnostics(const FieldGeom& g, int order, const Topology& tp, const double* m64,
+                               double grav, const double* h, const double* u, const double* v,
+                               const double* hs, const double* Aw, double hx2, double* partial,
+                               double* result, cudaStream_t st);
 
 // State combinations for the FP32 compensated representation: out = s1*(a_hi
 // + a_lo) + s2*(b_hi + b_lo) (b nullable) in double-float arithmetic on FP32
@@ -235,12 +233,18 @@ struct LatLonDev {
 // covariant or contravariant components); -1 on bad arguments
 int latlon_setup(int N, int nlon, int nlat, int width, int contravariant, const FieldGeom& g,
                  LatLonHost& h);
-// nf = 1: out = regrid of fa; nf = 2: the vector (fa, fb) regridded and
-// rotated, out = (u plane, v plane).  la/lb: FP32 low parts (nullable);
-// out (FP64) and out32 (FP32) nullable.
+// nf = 1: out = regrid of a scalar; 2: a vector regridded and rotated, out = (u
+// plane, v plane); 3: a scalar, then a vector.  out (FP64) and out32 (FP32)
+// nullable.
+// Input fields of a lat-lon launch: up to three, with the low parts of an FP32
+// pair (null in FP64).
 template <class T>
-cudaError_t launch_latlon(const FieldGeom& g, const LatLonDev& L, int nf, const T* fa, const T* fb,
-                          const float* la, const float* lb, double* out, float* out32,
-                          cudaStream_t st);
+struct LatLonFields {
+  const T* hi[3];
+  const float* lo[3];
+};
+template <class T>
+cudaError_t launch_latlon(const FieldGeom& g, const LatLonDev& L, const LatLonFields<T>& f, int nf,
+                          double* out, float* out32, cudaStream_t st);
 
 }  // namespace swm

@@ -62,42 +62,49 @@ void basis_proto(double a, double b, bool contravariant_components, double e1[3]
   }
 }
 
-template <class T>
-__global__ void latlon_kernel(FieldGeom g, LatLonDev L, int nf, const T* fa, const T* fb,
-                              const float* la, const float* lb, double* out, float* out32) {
+// nf planes: a scalar (1), a vector (2), or a scalar and a vector (3).  FP64
+// and the gathers bound it: the stencil is summed row by row (20 FP64
+// instructions a value for a cubic stencil, not 32), and a state's three
+// planes share a point's weights in one launch.
+template <class T, int W>
+__global__ void latlon_kernel(FieldGeom g, LatLonDev L, LatLonFields<T> f, int nf, double* out, float* out32) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int np = L.nlon * L.nlat;
+  const long long np = (long long)L.nlon * L.nlat;
   if (q >= np) return;
-  const int w = L.w;
   const long long base = L.base[q];
-  double wx[4], wy[4];
+  double wx[W], wy[W];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    wx[a] = a < w ? L.wx[a * np + q] : 0.0;
-    wy[a] = a < w ? L.wy[a * np + q] : 0.0;
+  for (int a = 0; a < W; ++a) {
+    wx[a] = L.wx[a * np + q];
+    wy[a] = L.wy[a * np + q];
   }
-  double v[2] = {0.0, 0.0};
+  double v[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
+  for (int c = 0; c < 3; ++c) {
     if (c >= nf) break;
-    const T* F = (c ? fb : fa) + base;
-    const float* Lo = c ? lb : la;
-    if (Lo) Lo += base;
-    double acc = 0.0;
-    for (int j1 = 0; j1 < w; ++j1)
-      for (int i1 = 0; i1 < w; ++i1) {
-        const long long o = (long long)j1 * g.P + i1;
-        const double p = Lo ? (double)F[o] + (double)Lo[o] : (double)F[o];
-        acc = acc + wx[i1] * wy[j1] * p;
+    const T* F = f.hi[c] + base;
+    const float* Lo = f.lo[c] ? f.lo[c] + base : nullptr;
+#pragma unroll
+    for (int j1 = 0; j1 < W; ++j1) {
+      double row = 0.0;
+#pragma unroll
+      for (int i1 = 0; i1 < W; ++i1) {
+        const int o = j1 * g.P + i1;
+        row += wx[i1] * (Lo ? (double)F[o] + (double)Lo[o] : (double)F[o]);
       }
-    v[c] = acc;
+      v[c] += wy[j1] * row;
+    }
   }
-  if (nf == 2) {   // rotate to lat-lon components
-    const double zu = v[0], zv = v[1];
-    v[0] = L.rot[0 * np + q] * zu + L.rot[2 * np + q] * zv;   // u2u*zu + v2u*zv
-    v[1] = L.rot[1 * np + q] * zu + L.rot[3 * np + q] * zv;   // u2v*zu + v2v*zv
+  if (nf >= 2) {   // rotate to lat-lon components
+    double& a = nf == 2 ? v[0] : v[1];
+    double& b = nf == 2 ? v[1] : v[2];
+    const double zu = a, zv = b;
+    a = L.rot[0 * np + q] * zu + L.rot[2 * np + q] * zv;   // u2u*zu + v2u*zv
+    b = L.rot[1 * np + q] * zu + L.rot[3 * np + q] * zv;   // u2v*zu + v2v*zv
   }
-  for (int c = 0; c < nf; ++c) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (c >= nf) break;
     if (out) out[c * np + q] = v[c];
     if (out32) out32[c * np + q] = (float)v[c];
   }
@@ -180,19 +187,17 @@ int latlon_setup(int N, int nlon, int nlat, int width, int contravariant, const 
 }
 
 template <class T>
-cudaError_t launch_latlon(const FieldGeom& g, const LatLonDev& L, int nf, const T* fa, const T* fb,
-                          const float* la, const float* lb, double* out, float* out32,
-                          cudaStream_t st) {
-  if (nf != 1 && nf != 2) return cudaErrorInvalidValue;
-  const int np = L.nlon * L.nlat;
-  latlon_kernel<T><<<(np + 255) / 256, 256, 0, st>>>(g, L, nf, fa, fb, la, lb, out, out32);
+cudaError_t launch_latlon(const FieldGeom& g, const LatLonDev& L, const LatLonFields<T>& f, int nf,
+                          double* out, float* out32, cudaStream_t st) {
+  if (nf < 1 || nf > 3) return cudaErrorInvalidValue;
+  const int nb = (int)(((long long)L.nlon * L.nlat + 127) / 128);
+  if (L.w == 2) latlon_kernel<T, 2><<<nb, 128, 0, st>>>(g, L, f, nf, out, out32);
+  else latlon_kernel<T, 4><<<nb, 128, 0, st>>>(g, L, f, nf, out, out32);
   return cudaGetLastError();
 }
-template cudaError_t launch_latlon<double>(const FieldGeom&, const LatLonDev&, int, const double*,
-                                           const double*, const float*, const float*, double*,
-                                           float*, cudaStream_t);
-template cudaError_t launch_latlon<float>(const FieldGeom&, const LatLonDev&, int, const float*,
-                                          const float*, const float*, const float*, double*,
-                                          float*, cudaStream_t);
+template cudaError_t launch_latlon<double>(const FieldGeom&, const LatLonDev&, const LatLonFields<double>&,
+                                           int, double*, float*, cudaStream_t);
+template cudaError_t launch_latlon<float>(const FieldGeom&, const LatLonDev&, const LatLonFields<float>&,
+                                          int, double*, float*, cudaStream_t);
 
 }  // namespace swm

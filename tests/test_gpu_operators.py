@@ -106,6 +106,34 @@ def test_grad_div_curl_match_oracle(pair):
     assert _maxrel(c.download(), od.curl(u, v)) < 1e-12
 
 
+# The operators sync their boundary nodes themselves, two lanes a node: the
+# smallest panel, an odd one and one past whole warps, with random fields whose
+# copies of an edge node differ.  Bars of test_grad_div_curl_match_oracle and
+# test_quadrature_mass_matches_oracle.
+@pytest.mark.parametrize("order,N", [(42, 16), (43, 17), (63, 16), (63, 39), (42, 64)])
+def test_operators_and_diagnostics_small_panels(order, N):
+    from cubedsphere_sbp_swm_gb300 import initial
+    od = oracle.OracleDomain(N, order)
+    op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=order))
+    rng = np.random.default_rng(N)
+    h, u, v, _ = initial.balanced_zonal(N, 3, 6)
+    h, u, v = (a + s * rng.standard_normal(a.shape) for a, s in zip((h, u, v), (50.0, 2.0, 2.0)))
+    gx, gy, d, c = (op.create_field() for _ in range(4))
+    op.calc_grad(gx, gy, _field(op, h))
+    for a, b in zip((gx, gy), od.grad(h)):
+        assert _maxrel(a.download(), b) < 1e-13
+    op.calc_div(d, _field(op, u), _field(op, v))
+    assert _maxrel(d.download(), od.div(u, v)) < 1e-12
+    op.calc_curl(c, _field(op, u), _field(op, v))
+    assert _maxrel(c.download(), od.curl(u, v)) < 1e-12
+    s = op.create_stvec()
+    s.upload(h, u, v)
+    got, want = list(op.get_diagnostics(s).values()), list(od.diagnostics(h, u, v))
+    assert got[0] == h.min() and got[1] == h.max()
+    for a, b in zip(got[2:], want[2:]):
+        assert abs(a - b) < 1e-13 * abs(b)
+
+
 def test_syncs_match_oracle(pair):
     od, op, rng, _ = pair
     a = rng.standard_normal((6, op.n, op.n))
