@@ -802,24 +802,22 @@ def diffusion_leg(w, h, u, v, local, steps, warmup):
     return out
 
 
-# The C-grid SBP family (&shallow_water_model_c) at N=384, SBP 4/2, FP64:
-# six passes per RK4 stage (centre_a, faces_a, curl, w2uv with the curl's
-# corner sync, centre_b, faces_b).  Algorithmic HBM words per point and stage of
-# those passes (inputs and outputs of each pass, metric included):
-#   centre_a 6 + faces_a 17 + curl 4 + w2uv 3 + centre_b 13 + faces_b 3,
-#   plus the stage epilogues of the three state components (2, 4, 2 and 3
-#   words in stages 1..4): 4 x 46 + 3 x 11 = 217 words per point and step.
-CGRID_WORDS_PER_POINT_STEP = 217
+# The C-grid SBP family (&shallow_water_model_c) at N=384, SBP 4/2, FP64: four
+# passes per RK4 stage (rhs1..rhs4).  Algorithmic HBM words per point and stage
+# of those passes (inputs and outputs of each pass, metric included): 7 + 17 +
+# 12 + 3, plus the stage epilogues of the three state components (2, 4, 2 and
+# 3 words in stages 1..4): 4 x 39 + 3 x 11 = 189 words per point and step.
+CGRID_WORDS_PER_POINT_STEP = 189
 CGRID_LAUNCHES_PER_STEP = 16          # 4 x 4 passes (the curl's corner sync rides in the reads of the second)
 # The namelist's C-grid model step adds one explicit Euler step of the
 # hyperdiffusion (hordiff_c_biharm_curl_div, hordiff_scalar_C; 2/1
 # operators).  Words per point of its passes, inputs + outputs + metric:
-# co2contra / contra2co 15 (centre_a 5 + faces_a 10), div 6, grad 3, curl 4,
-# grad_perp 5; curl part 2 x (4 + 5 + 15), div part 2 x (15 + 6 + 3), h part
-# 2 x (3 + 15 + 6), the combine pass 11 (5 results, state read and written):
-# 48 + 48 + 48 + 11 = 155 words per point.
-CGRID_DIFF_WORDS_PER_POINT_STEP = 155
-CGRID_DIFF_LAUNCHES_PER_STEP = 29     # 24 passes, 2 corner syncs of 2 kernels, combine
+# co2contra / contra2co 9, div 6, grad 3, curl 4, grad_perp 5; curl part
+# 2 x (4 + 5 + 9), div part 2 x (9 + 6 + 3), h part 2 x (3 + 9 + 6), the
+# combine pass 11 (5 results, state read and written): 36 + 36 + 36 + 11 =
+# 119 words per point.
+CGRID_DIFF_WORDS_PER_POINT_STEP = 119
+CGRID_DIFF_LAUNCHES_PER_STEP = 7      # six launches of a pass of each chain, combine
 
 
 def cgrid_leg(local, steps, warmup, cpu=True):

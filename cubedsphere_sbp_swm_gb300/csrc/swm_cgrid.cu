@@ -205,19 +205,35 @@ __device__ __forceinline__ int at(const FieldGeom& g, int p, int i, int j) {
   return p * (int)g.ps + j * g.P + i;
 }
 
+// Closure row k (from either end, nin inputs) of an operator: the loops run to
+// the widest row (ORD 42: 6 inputs, 21: 2) with the taps past the row skipped, so
+// that the loads of a row are in flight together (with the row's own length as
+// the bound the FP32 RK4 step took 130 us at N=48, so 119); the terms come in
+// the order of the reference's sums.
+template <int W, class T, class Fn>
+__device__ __forceinline__ T stag_closure(const StagOpT<T>& s, Fn F, int nout, int k) {
+  constexpr int NW = W == 4 ? 6 : 2;
+  T acc = T(0.0);
+  if (k < s.ne) {
+#pragma unroll
+    for (int m = 0; m < NW; ++m)
+      if (m < s.last[k]) acc += s.Ql[k * s.nw + m] * F(m);
+  } else {
+    const int nin = nout - s.dnx, r = nout - 1 - k;
+#pragma unroll
+    for (int m = NW - 1; m >= 0; --m)
+      if (m < s.last[r]) acc += (s.rsign * s.Ql[r * s.nw + m]) * F(nin - 1 - m);
+  }
+  return acc;
+}
+
 // sbp_apply for output k of nout outputs over a line read through F(m)
 template <int W, class T, class Fn>
 __device__ __forceinline__ T stag_at_f(const StagOpT<T>& s, Fn F, int nout, int k) {
+  if (k < s.ne || k >= nout - s.ne) return stag_closure<W, T>(s, F, nout, k);
   T acc = T(0.0);
-  if (k >= s.ne && k < nout - s.ne) {
 #pragma unroll
-    for (int t = 0; t < W; ++t) acc += s.Qin[t] * F(k + s.inshift + t);
-  } else if (k < s.ne) {
-    for (int m = 0; m < s.last[k]; ++m) acc += s.Ql[k * s.nw + m] * F(m);
-  } else {
-    const int nin = nout - s.dnx, r = nout - 1 - k;
-    for (int m = s.last[r] - 1; m >= 0; --m) acc += (s.rsign * s.Ql[r * s.nw + m]) * F(nin - 1 - m);
-  }
+  for (int t = 0; t < W; ++t) acc += s.Qin[t] * F(k + s.inshift + t);
   return acc;
 }
 
@@ -225,18 +241,7 @@ __device__ __forceinline__ T stag_at_f(const StagOpT<T>& s, Fn F, int nout, int 
 template <int W, class T>
 __device__ __forceinline__ T stag_at(const StagOpT<T>& s, const T* __restrict__ f, int st, int nout,
                                           int k) {
-  T acc = T(0.0);
-  if (k >= s.ne && k < nout - s.ne) {
-    const T* b = f + (k + s.inshift) * st;
-#pragma unroll
-    for (int t = 0; t < W; ++t) acc += s.Qin[t] * b[t * st];
-  } else if (k < s.ne) {
-    for (int m = 0; m < s.last[k]; ++m) acc += s.Ql[k * s.nw + m] * f[m * st];
-  } else {
-    const int nin = nout - s.dnx, r = nout - 1 - k;
-    for (int m = s.last[r] - 1; m >= 0; --m) acc += (s.rsign * s.Ql[r * s.nw + m]) * f[(nin - 1 - m) * st];
-  }
-  return acc;
+  return stag_at_f<W, T>(s, [&](int m) { return f[m * st]; }, nout, k);
 }
 
 // value of a neighbour's point in the cross halo: mesh 0 o, 1 u, 2 v, 3 q; side 0
@@ -869,7 +874,9 @@ __device__ __forceinline__ T grad_line(const A& a, int N, int i, Fn F) {
     const T dx1 = a.dx1;
     if (i <= 3) {
       T s = T(0.0);
-      for (int m = 0; m < D.last[i]; ++m) s += D.Ql[i * D.nw + m] * F(m);
+#pragma unroll
+      for (int m = 0; m < 5; ++m)
+        if (m < D.last[i]) s += D.Ql[i * D.nw + m] * F(m);
       T gv = s * dx1;
       if (i == 0) {
         const T dh =
@@ -886,7 +893,9 @@ __device__ __forceinline__ T grad_line(const A& a, int N, int i, Fn F) {
     }
     const int r = N - i;
     T s = T(0.0);
-    for (int m = 0; m < D.last[r]; ++m) s += D.Ql[r * D.nw + m] * F(N - 1 - m);
+#pragma unroll
+    for (int m = 0; m < 5; ++m)
+      if (m < D.last[r]) s += D.Ql[r * D.nw + m] * F(N - 1 - m);
     T gv = -s * dx1;
     if (i == N) {
       const T dh =
@@ -1014,6 +1023,7 @@ __global__ void cpack_kernel(FieldGeom g, int nx, int ny, const double* __restri
 }
 
 #include "swm_cgrid_rhs.cuh"
+#include "swm_cgrid_diff.cuh"
 
 __global__ void mass_final_kernel(const double* part, int n, double* out) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
@@ -1033,16 +1043,12 @@ struct CGrid {
   COpsT<float> ops32{};
   COps ops21{};             // the 2/1 operators of the hyperdiffusion (any order)
   COpsT<float> ops21_32{};
-  ScaledOps<double> sops{};        // the fused FP64 passes' operators
+  ScaledOps<double> sops{}, sops21{};  // the fused FP64 passes' operators
   double* met = nullptr;   // M_COUNT fields
   float* met32 = nullptr;  // their FP32 copies (contexts of the FP32 form)
   double* wk = nullptr;    // W_COUNT fields
   double* rk = nullptr;    // Y, Kb, acc: 3 fields each
-  // hyperdiffusion (allocated on first use): kDiffFields work fields, the two
-  // side streams of its branches and the fork / join events
-  double* dw = nullptr;
-  cudaStream_t bs[2] = {nullptr, nullptr};
-  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  double* dw = nullptr;    // hyperdiffusion: kDiffFields work fields (allocated on first use)
   int* halo = nullptr;
   double* ecs_w = nullptr;  // ECS_O weights [2][N+4][4]
   int* ecs_ind = nullptr;   // ECS_O stencil bases [2][N+4]
@@ -1154,6 +1160,15 @@ RhsArgs<T> rhs_args(const CGrid* c) {
   return a;
 }
 
+// Launch grid of rhs_map and its slabs of column warps.
+dim3 rhs_grid(int N, int& strips) {
+  dim3 grid((N - 2 * kRhsEdge + kRhsX) / kRhsX, (N + kRhsY) / kRhsY, 6);
+  const int blocks = 6 * ((N + kRhsX) / kRhsX), slab = grid.x * grid.y;
+  strips = (blocks + slab - 1) / slab;
+  grid.z += strips;
+  return grid;
+}
+
 // One right-hand side of the state (h, u, v) at `in` with the epilogue of
 // mode (rhs1..rhs4).
 template <class T>
@@ -1161,10 +1176,7 @@ cudaError_t rhs(const CGrid* c, RhsArgs<T> a, int mode, const T* in, cudaStream_
   const long long fs = c->g.fs;
   const int N = c->N;
   a.h = in; a.u = in + fs; a.v = in + 2 * fs;
-  dim3 grid((N - 2 * kRhsEdge + kRhsX) / kRhsX, (N + kRhsY) / kRhsY, 6);
-  const int blocks = 6 * ((N + kRhsX) / kRhsX), slab = grid.x * grid.y;
-  a.strips = (blocks + slab - 1) / slab;
-  grid.z += a.strips;
+  const dim3 grid = rhs_grid(N, a.strips);
   return c->order == 42 ? rhs_passes<42, T>(a, mode, grid, st) : rhs_passes<21, T>(a, mode, grid, st);
 }
 
@@ -1279,10 +1291,9 @@ cudaError_t transform(const CGrid* c, CArgsT<T> a, const T* x, const T* y, T* xo
 }
 
 // Work fields of the hyperdiffusion: the results L(L(h)), the curl part
-// (u, v) and the divergence part (u, v), then per branch (curl, divergence,
-// h) the centre scratch of the transforms (2), two face pairs (4) and one
-// centre or corner field.
-constexpr int kDiffResults = 5, kDiffBranch = 7, kDiffFields = kDiffResults + 3 * kDiffBranch;
+// (u, v) and the divergence part (u, v), then per chain (curl, divergence, h)
+// two face pairs (4) and one centre or corner field.
+constexpr int kDiffResults = 5, kDiffChain = 5, kDiffFields = kDiffResults + 3 * kDiffChain;
 
 // The C-grid hyperdiffusion of operator_swm_diff_t (operator_swm_diff_mod.f90
 // :25-46) with the 2/1 operators the factory uses at any order
@@ -1290,89 +1301,54 @@ constexpr int kDiffResults = 5, kDiffBranch = 7, kDiffFields = kDiffResults + 3 
 //   curl part  contra2co grad_perp curl contra2co grad_perp curl (u, v)
 //   div part   grad div co2contra grad div co2contra (u, v)
 //   h          L(L(h)), L = div co2contra grad
-// The three chains are independent: they run as three branches (the
-// context stream and two side streams, forked and joined with events, so a
-// captured step becomes a three-branch graph), each on its own work fields.
-// Then the combine pass on the context stream (mode 0 tendency into out, 1 /
-// 2 Euler step on out = the state, 2 with the FP32 low part lo).
+// in six launches of one pass of each chain (swm_cgrid_diff.cuh), then the
+// combine pass (mode 0 tendency into out, 1 / 2 Euler step on out = the state,
+// 2 with the FP32 low part lo).
 template <class T>
-cudaError_t diffusion(const CGrid* c, const Topology& tp, T* edge, int parts, double c4uv, double c4h, const T* in,
-                      T* out, float* lo, double dt, int mode, cudaStream_t st) {
+cudaError_t diffusion(const CGrid* c, int parts, double c4uv, double c4h, const T* in, T* out, float* lo, double dt,
+                      int mode, cudaStream_t st) {
   if (!c->dw) return cudaErrorInvalidValue;  // cgrid_diffusion_prepare first
   const long long fs = c->g.fs;
   auto F = [&](int k) { return reinterpret_cast<T*>(c->dw + (long long)k * fs); };
   T *TH = F(0), *TU = F(1), *TV = F(2), *U3 = F(3), *V3 = F(4);
   const T *h = in, *u = in + fs, *v = in + 2 * fs;
-  struct Branch {
-    CArgsT<T> a;  // with this branch's transform scratch
+  DiffArgs<T> a{};
+  a.r = rhs_args<T>(c);
+  if constexpr (sizeof(T) == 8) a.r.ops = c->sops21;
+  else a.r.ops = c->ops21_32;
+  auto M = [&](int k) { return metric_t<T>(c, k); };
+  a.jq = M(M_JQI2P); a.q1 = M(M_QI1U); a.q3 = M(M_QI3V);
+  a.jqc = M(M_JQ2P); a.q1c = M(M_Q1U); a.q3c = M(M_Q3V);
+  a.rju = M(M_RJU); a.rjv = M(M_RJV); a.rjq = M(M_RJQHA); a.rjp = M(M_RJPHA);
+  a.rjuh = M(M_RJUHA); a.rjvh = M(M_RJVHA);
+  struct Chain {
     T *X1, *Y1, *X2, *Y2, *S;
-    cudaStream_t st;
   };
-  const cudaStream_t side[2] = {c->bs[0], c->bs[1]};
-  auto branch = [&](int b) {
-    const int o = kDiffResults + kDiffBranch * b;
-    Branch r{base_args<T>(c, 21), F(o + 2), F(o + 3), F(o + 4), F(o + 5), F(o + 6), b ? side[b - 1] : st};
-    r.a.Ap = F(o);
-    r.a.Bp = F(o + 1);
-    return r;
+  auto chain = [&](int k) {
+    const int o = kDiffResults + kDiffChain * k;
+    return Chain{F(o), F(o + 1), F(o + 2), F(o + 3), F(o + 4)};
   };
-  auto div = [&](const Branch& B, const T* x, const T* y, T* o) {
-    CArgsT<T> b = B.a;
-    b.hu_in = x; b.hv_in = y; b.o1 = o;
-    b.flags = F_DIV;
-    return run_centre_b(c, b, B.st);
-  };
-  auto grad = [&](const Branch& B, const T* f, T* gx, T* gy) {
-    CArgsT<T> b = B.a;
-    b.ke_in = f; b.o1 = gx; b.o2 = gy;
-    b.flags = F_GRAD;
-    return run_faces_b(c, b, B.st);
-  };
-  auto curl = [&](const Branch& B, const T* x, const T* y, T* q) {
-    CArgsT<T> b = B.a;
-    b.u = x; b.v = y; b.curl = q;
-    CKE(run_curl(c, b, B.st));
-    return launch_sync_scalar_t<T>(c->g, tp, q, edge, B.st);
-  };
-  auto gperp = [&](const Branch& B, const T* q, T* gu, T* gv) {
-    CArgsT<T> b = B.a;
-    b.curl_in = q; b.o1 = gu; b.o2 = gv;
-    return run_gperp(c, b, B.st);
-  };
-  auto xf = [&](const Branch& B, const T* x, const T* y, T* xo, T* yo, bool to_co) {
-    return transform(c, B.a, x, y, xo, yo, to_co, B.st);
-  };
-  const Branch bc = branch(0), bd = branch(1), bh = branch(2);
-  CKE(cudaEventRecord(c->ev[0], st));
-  CKE(cudaStreamWaitEvent(bd.st, c->ev[0], 0));
-  CKE(cudaStreamWaitEvent(bh.st, c->ev[0], 0));
-  if (parts & 2) {
-    CKE(curl(bc, u, v, bc.S));
-    CKE(gperp(bc, bc.S, bc.X1, bc.Y1));
-    CKE(xf(bc, bc.X1, bc.Y1, bc.X2, bc.Y2, true));
-    CKE(curl(bc, bc.X2, bc.Y2, bc.S));
-    CKE(gperp(bc, bc.S, bc.X1, bc.Y1));
-    CKE(xf(bc, bc.X1, bc.Y1, TU, TV, true));
+  const Chain C = chain(0), D = chain(1), H = chain(2);
+  const DiffRole<T> none{DK_NONE, nullptr, nullptr, nullptr, nullptr};
+  const DiffRole<T> curl[6] = {{DK_CURL, u, v, C.S, nullptr},           {DK_GPERP, C.S, nullptr, C.X1, C.Y1},
+                               {DK_XF_CO, C.X1, C.Y1, C.X2, C.Y2},      {DK_CURL, C.X2, C.Y2, C.S, nullptr},
+                               {DK_GPERP, C.S, nullptr, C.X1, C.Y1},    {DK_XF_CO, C.X1, C.Y1, TU, TV}};
+  const DiffRole<T> div[6] = {{DK_XF, u, v, D.X1, D.Y1},       {DK_DIV, D.X1, D.Y1, D.S, nullptr},
+                              {DK_GRAD, D.S, nullptr, D.X2, D.Y2}, {DK_XF, D.X2, D.Y2, D.X1, D.Y1},
+                              {DK_DIV, D.X1, D.Y1, D.S, nullptr},  {DK_GRAD, D.S, nullptr, U3, V3}};
+  const DiffRole<T> lap[6] = {{DK_GRAD, h, nullptr, H.X1, H.Y1},   {DK_XF, H.X1, H.Y1, H.X2, H.Y2},
+                              {DK_DIV, H.X2, H.Y2, H.S, nullptr},  {DK_GRAD, H.S, nullptr, H.X1, H.Y1},
+                              {DK_XF, H.X1, H.Y1, H.X2, H.Y2},     {DK_DIV, H.X2, H.Y2, TH, nullptr}};
+  dim3 grid = rhs_grid(c->N, a.r.strips);
+  a.zs = grid.z;
+  grid.z *= 3;
+  for (int k = 0; k < 6; ++k) {
+    a.role[0] = parts & 2 ? curl[k] : none;
+    a.role[1] = parts & 1 ? div[k] : none;
+    a.role[2] = lap[k];
+    diff_pass_kernel<T><<<grid, dim3(kRhsX, kRhsY), 0, st>>>(a);
+    CKE(cudaGetLastError());
   }
-  if (parts & 1) {
-    CKE(xf(bd, u, v, bd.X1, bd.Y1, false));
-    CKE(div(bd, bd.X1, bd.Y1, bd.S));
-    CKE(grad(bd, bd.S, bd.X2, bd.Y2));
-    CKE(xf(bd, bd.X2, bd.Y2, bd.X1, bd.Y1, false));
-    CKE(div(bd, bd.X1, bd.Y1, bd.S));
-    CKE(grad(bd, bd.S, U3, V3));
-  }
-  const T* f = h;
-  for (int rep = 0; rep < 2; ++rep) {
-    CKE(grad(bh, f, bh.X1, bh.Y1));
-    CKE(xf(bh, bh.X1, bh.Y1, bh.X2, bh.Y2, false));
-    CKE(div(bh, bh.X2, bh.Y2, rep ? TH : bh.S));
-    f = bh.S;
-  }
-  CKE(cudaEventRecord(c->ev[1], bd.st));
-  CKE(cudaEventRecord(c->ev[2], bh.st));
-  CKE(cudaStreamWaitEvent(st, c->ev[1], 0));
-  CKE(cudaStreamWaitEvent(st, c->ev[2], 0));
   diff_combine_kernel<T><<<grid_for(c->N + 1, c->N + 1), kBlock, 0, st>>>(
       c->g, c->N, parts, T(c4uv), T(c4h), TH, TU, TV, U3, V3, mode, dt, out, lo);
   return cudaGetLastError();
@@ -1517,6 +1493,7 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
   c->ops32 = ops_cast<float>(c->ops);
   c->sops = scaled_ops<double>(c->ops, order);
   fill_ops(21, c->ops21);
+  c->sops21 = scaled_ops<double>(c->ops21, 21);
   c->ops21_32 = ops_cast<float>(c->ops21);
   const double an = std::sqrt(axis[0] * axis[0] + axis[1] * axis[1] + axis[2] * axis[2]);
   const double ax[3] = {axis[0] / an, axis[1] / an, axis[2] / an};
@@ -1659,10 +1636,6 @@ void cgrid_destroy(CGrid* c) {
                   (void*)c->xy_w, (void*)c->xy_ind, (void*)c->xy_ext, (void*)c->xy_mt, (void*)c->wts,
                   (void*)c->part})
     if (p) cudaFree(p);
-  for (cudaStream_t s : c->bs)
-    if (s) cudaStreamDestroy(s);
-  for (cudaEvent_t e : c->ev)
-    if (e) cudaEventDestroy(e);
   delete c;
 }
 
@@ -1824,16 +1797,10 @@ cudaError_t cgrid_diffusion_prepare(CGrid* c) {
   cudaError_t e = cudaMalloc(&c->dw, sizeof(double) * kDiffFields * c->g.fs);
   if (e == cudaSuccess) e = cudaMemset(c->dw, 0, sizeof(double) * kDiffFields * c->g.fs);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the context stream does not wait on the legacy one
-  for (cudaStream_t& s : c->bs)
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  for (cudaEvent_t& ev : c->ev)
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     // leave nothing half made: the next call retries from scratch
     if (c->dw) cudaFree(c->dw);
     c->dw = nullptr;
-    for (cudaStream_t& s : c->bs) { if (s) cudaStreamDestroy(s); s = nullptr; }
-    for (cudaEvent_t& ev : c->ev) { if (ev) cudaEventDestroy(ev); ev = nullptr; }
   }
   return e;
 }
@@ -1841,25 +1808,25 @@ cudaError_t cgrid_diffusion_prepare(CGrid* c) {
 cudaError_t cgrid_diffusion(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
                             const double* in, double* out, cudaStream_t st) {
   if (in == out || parts < 1 || parts > 3) return cudaErrorInvalidValue;
-  return diffusion<double>(c, tp, edge, parts, c4uv, c4h, in, out, nullptr, 0.0, 0, st);
+  return diffusion<double>(c, parts, c4uv, c4h, in, out, nullptr, 0.0, 0, st);
 }
 
 cudaError_t cgrid_diffusion_step(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
                                  double* y0, double dt, cudaStream_t st) {
   if (parts < 1 || parts > 3) return cudaErrorInvalidValue;
-  return diffusion<double>(c, tp, edge, parts, c4uv, c4h, y0, y0, nullptr, dt, 1, st);
+  return diffusion<double>(c, parts, c4uv, c4h, y0, y0, nullptr, dt, 1, st);
 }
 
 cudaError_t cgrid_diffusion32(CGrid* c, const Topology& tp, float* edge, int parts, double c4uv, double c4h,
                               const float* in, float* out, cudaStream_t st) {
   if (!c->met32 || in == out || parts < 1 || parts > 3) return cudaErrorInvalidValue;
-  return diffusion<float>(c, tp, edge, parts, c4uv, c4h, in, out, nullptr, 0.0, 0, st);
+  return diffusion<float>(c, parts, c4uv, c4h, in, out, nullptr, 0.0, 0, st);
 }
 
 cudaError_t cgrid_diffusion_step32(CGrid* c, const Topology& tp, float* edge, int parts, double c4uv, double c4h,
                                    float* hi, float* lo, double dt, cudaStream_t st) {
   if (!c->met32 || parts < 1 || parts > 3) return cudaErrorInvalidValue;
-  return diffusion<float>(c, tp, edge, parts, c4uv, c4h, hi, hi, lo, dt, 2, st);
+  return diffusion<float>(c, parts, c4uv, c4h, hi, hi, lo, dt, 2, st);
 }
 
 cudaError_t cgrid_grad_a2_ecs(CGrid* c, const double* f, double* gx, double* gy, cudaStream_t st) {

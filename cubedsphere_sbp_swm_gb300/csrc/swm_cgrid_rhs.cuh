@@ -96,7 +96,7 @@ constexpr int kRhsX = 32, kRhsY = 8, kRhsEdge = 4;
 template <class T>
 constexpr int kRhsBlocks = sizeof(T) == 4 ? 8 : 6;
 
-// Point of this thread: i for the interface outputs along x (0..N) and ip for
+// Point of this thread in slab z: i for the interface outputs along x (0..N) and ip for
 // the centre outputs (0..N-1, or -1 where a thread has none).  The first grid.z
 // slabs hold the column warps: lanes along j, one of the four columns of
 // either side per warp; the others hold the columns between.
@@ -105,11 +105,11 @@ struct RhsPoint {
   bool strip;
 };
 template <class T>
-__device__ __forceinline__ bool rhs_map(const RhsArgs<T>& a, RhsPoint& r) {
+__device__ __forceinline__ bool rhs_map(const RhsArgs<T>& a, int z, RhsPoint& r) {
   const int N = a.N;
-  if ((int)blockIdx.z < a.strips) {
+  if (z < a.strips) {
     const int nb = (N + kRhsX) / kRhsX;   // blocks of 32 rows along 0..N
-    const int b = ((int)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const int b = (z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     r.p = b / nb;
     if (r.p >= 6) return false;
     r.j = (b - r.p * nb) * kRhsX + threadIdx.x;
@@ -119,7 +119,7 @@ __device__ __forceinline__ bool rhs_map(const RhsArgs<T>& a, RhsPoint& r) {
     r.strip = true;
     return r.j <= N;
   }
-  r.p = blockIdx.z - a.strips;
+  r.p = z - a.strips;
   r.i = kRhsEdge + blockIdx.x * kRhsX + threadIdx.x;
   r.j = blockIdx.y * kRhsY + threadIdx.y;
   r.ip = r.i < N - kRhsEdge ? r.i : -1;
@@ -198,14 +198,7 @@ __device__ __forceinline__ T any_row(const StagOpT<T>& s, int nout, int k, int o
     else
       return (F(off) + F(off + 1)) + T(Sc<ORD>::rW) * (F(off - 1) + F(off + 2));
   }
-  T acc = T(0);
-  if (k < s.ne) {
-    for (int m = 0; m < s.last[k]; ++m) acc += s.Ql[k * s.nw + m] * F(m);
-  } else {
-    const int nin = nout - s.dnx, r = nout - 1 - k;
-    for (int m = s.last[r] - 1; m >= 0; --m) acc += (s.rsign * s.Ql[r * s.nw + m]) * F(nin - 1 - m);
-  }
-  return acc;
+  return stag_closure<ORD == 42 ? 4 : 2, T>(s, F, nout, k);
 }
 template <int ORD, class T, class Fn>
 __device__ __forceinline__ T w_c2i(const RhsArgs<T>& a, int k, Fn F) {
@@ -242,7 +235,8 @@ __device__ __forceinline__ T d_c2i_sat(const RhsArgs<T>& a, int k, Fn F, Hn H) {
   T s = d_c2i<ORD, T>(a, k, F);
   if (k == 0 || k == N) {
     T dj = T(0.0);
-    for (int m = 0; m < a.ops.np; ++m)
+#pragma unroll
+    for (int m = 0; m < (ORD == 42 ? 3 : 2); ++m)
       dj = dj + a.ops.proj[m] * (k == 0 ? F(m) - H(0, m + 1) : H(1, m + 1) - F(N - 1 - m));
     if constexpr (sizeof(T) == 8) s += a.ops.csat * dj;
     else s = s + T(0.5) * dj / a.ops.a_i0;
@@ -275,12 +269,19 @@ __device__ __forceinline__ T grad_any(const RhsArgs<T>& a, int k, Fn F) {
     T s = d_c2i<ORD, T>(a, k, F);
     if (k == 0 || k == N) {
       T dj = T(0);
-      for (int m = 0; m < a.ops.np; ++m)
+#pragma unroll
+      for (int m = 0; m < (ORD == 42 ? 3 : 2); ++m)
         dj += a.ops.proj[m] * (k == 0 ? F(m) - F(-1 - m) : F(N + m) - F(N - 1 - m));
       s += a.ops.gsat * dj;
     }
     return s;
   }
+}
+// The 2/1 gradient at the two panel-edge interfaces (k = 0, N), scaled.
+template <class T, class Fn>
+__device__ __forceinline__ T grad_edge(const RhsArgs<T>& a, int k, Fn F) {
+  if constexpr (sizeof(T) == 4) return grad_line<21, T>(a, a.N, k, F);
+  else return grad_any<21, T>(a, k, F) * a.dx1;   // the 2/1 difference has the scale 1
 }
 // The 2/1 divergence along one line in FP32 from the raw fluxes F (with the
 // neighbour's at -1 and N+1) and J at the interfaces (div_c2_mod.f90:97-177).
@@ -353,7 +354,7 @@ __device__ __forceinline__ bool rhs_yin(int N, int j) { return j >= kRhsEdge && 
 template <int ORD, class T>
 __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs1_kernel(const __grid_constant__ RhsArgs<T> a) {
   RhsPoint r;
-  if (!rhs_map(a, r)) return;
+  if (!rhs_map(a, blockIdx.z, r)) return;
   const int N = a.N, P = a.g.P, p = r.p, j = r.j;
   const bool yin = rhs_yin(N, j);
   {  // corner (i, j): the curl, curl_c_sbp_mod.f90:44-127
@@ -388,11 +389,11 @@ __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs1_kernel(cons
   }
 }
 
-// The curl with its corner-mesh sync taken as it is read (curl_synced).
+// A corner field with its Ah-type sync (halo_Ah_scalar_sync_mod.f90:38-93, in the
+// order of the sync kernel) taken as it is read.
 template <class T>
-__device__ __forceinline__ T rhs_curl_synced(const RhsArgs<T>& a, int p, int i, int j) {
+__device__ __forceinline__ T rhs_corner_synced(const RhsArgs<T>& a, const T* c, int p, int i, int j) {
   const int N = a.N;
-  const T* c = a.curl;
   const T own = c[at(a.g, p, i, j)];
   const bool lr = i == 0 || i == N, bt = j == 0 || j == N;
   if (!lr && !bt) return own;
@@ -422,7 +423,7 @@ __device__ __forceinline__ void flux_out(T qi, T w, T t, T sj, T J, T h, T* G, T
 template <int ORD, class T>
 __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs2_kernel(const __grid_constant__ RhsArgs<T> a) {
   RhsPoint r;
-  if (!rhs_map(a, r)) return;
+  if (!rhs_map(a, blockIdx.z, r)) return;
   const int N = a.N, P = a.g.P, p = r.p, i = r.i, j = r.j;
   const bool yin = rhs_yin(N, j);
   const int e = at(a.g, p, i, j);
@@ -433,7 +434,7 @@ __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs2_kernel(cons
     const T hu = r.strip ? w_c2i<ORD, T>(a, i, [&](int m) { return hrow[m]; }) : w_in<ORD, T>(a.h + e - 1, 1);
     flux_out<ORD, T>(ro(a.Qi1u + e), ro(a.u + e), t, ro(a.sju + e), ro(a.Ju + e), hu, a.Gu + e, a.KEu + e, a.hu + e);
     a.fu[e] = !r.strip && yin ? w_in<ORD, T>(a.curl + e, P)
-                              : w_i2c<ORD, T>(a, j, [&](int m) { return rhs_curl_synced(a, p, i, m); });
+                              : w_i2c<ORD, T>(a, j, [&](int m) { return rhs_corner_synced(a, a.curl, p, i, m); });
   }
   if (i < N) {  // y-face
     const T* Bcol = a.Bp + at(a.g, p, i, 0);
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs2_kernel(cons
 template <int ORD, int MODE, class T>
 __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs3_kernel(const __grid_constant__ RhsArgs<T> a) {
   RhsPoint r;
-  if (!rhs_map(a, r) || r.ip < 0 || r.j >= a.N) return;
+  if (!rhs_map(a, blockIdx.z, r) || r.ip < 0 || r.j >= a.N) return;
   const int N = a.N, P = a.g.P, p = r.p, i = r.ip, j = r.j;
   const int e = at(a.g, p, i, j);
   const RkIn<T> rk = rk_in<MODE, T>(a, e);
@@ -524,7 +525,7 @@ __device__ __forceinline__ T uv_tend(const RhsArgs<T>& a, T g, T c) {
 template <int ORD, int MODE, class T>
 __global__ void __launch_bounds__(kRhsX * kRhsY, kRhsBlocks<T>) rhs4_kernel(const __grid_constant__ RhsArgs<T> a) {
   RhsPoint r;
-  if (!rhs_map(a, r)) return;
+  if (!rhs_map(a, blockIdx.z, r)) return;
   const int N = a.N, P = a.g.P, p = r.p, i = r.i, j = r.j, fs = (int)a.g.fs;
   const int e = at(a.g, p, i, j);
   const bool yin = rhs_yin(N, j), onu = j < N, onv = i < N;

@@ -82,6 +82,22 @@ def test_diffusion_tendency_matches_oracle(order, uv_name):
         assert _rel(a, b) < 1e-12, _rel(a, b)
 
 
+# The three chains share their launches: each part alone and all together at
+# the smallest panel and around a whole tile of inner columns.
+@pytest.mark.parametrize("uv_name", UV_NAMES)
+@pytest.mark.parametrize("N", [16, 17, 38, 39])
+def test_diffusion_tendency_small_panels(N, uv_name):
+    op, od = c_op(N, 42), oracle.OracleCDomain(N, 42)
+    dop = swm.OperatorSWMDiff(op, uv_name, 0.03, "hordiff_scalar_C", 0.02)
+    h, u, v = _rough_state(N, 4)
+    vin = op.create_stvec()
+    vin.upload(h, u, v)
+    vout = vin.create_similar()
+    dop.apply(vout, vin)
+    for a, b in zip(vout.download(), od.hordiff(h, u, v, uv_name, 0.03, 0.02)):
+        assert _rel(a, b) < 1e-12, _rel(a, b)
+
+
 @pytest.mark.parametrize("order,prec,tol", [(42, "fp64", 1e-12), (21, "fp64", 1e-12), (42, "fp32", 1e-5)])
 def test_model_step_with_diffusion_matches_oracle(order, prec, tol):
     """The namelist's C-grid configuration (namelist_swm:80-102: the 4/2
