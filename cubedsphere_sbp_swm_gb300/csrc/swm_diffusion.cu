@@ -83,6 +83,9 @@ struct NarrowShape {
   // stencil taps a node keeps: a closure row's cols or the interior's w
   // (2/1: 2 and 3)
   static constexpr int taps = cols > w ? cols : w;
+  // entry of the interior stencil matrix
+  template <int C, int Q>
+  static constexpr float in32 = float(kNarrowAll[ni].in[C][Q]);
 };
 
 // Node kernels run on 2-D tiles of TX columns x TY rows of the (6n)-row
@@ -245,6 +248,39 @@ __device__ __forceinline__ void lap_region(int a0, int len, int n, int& lo, int&
   }
 }
 
+// Start of tile t of count along a line of n nodes, tiles of len nodes with
+// closure rows of `rows` nodes at each end.  The last tile ends on the panel
+// edge.  Where the tile before it would reach the far closure rows too (every
+// n = k len + 1 .. k len + rows, so every N that is a multiple of len), it is
+// moved back next to the last one if that leaves it between the closures: a
+// tile with closure nodes costs about 2.5 tiles without (1890 against 770
+// instructions a warp, 4/2), and at N=384 there are 720 of them instead of
+// 1062 in 3822.  Nodes in two tiles get the same value twice.  With the inner
+// tiles' flat loops the model step with hyperdiffusion went 0.213 -> 0.201 ms
+// at N=384 (4/2), 1.150 -> 1.095 ms at N=1024 (6/3).
+__device__ __forceinline__ int lap_tile_start(int t, int count, int len, int n, int rows) {
+  const int a = min(t * len, n - min(len, n));
+  const int b = n - 2 * len;
+  return t == count - 2 && a + len > n - rows && b >= rows ? b : a;
+}
+
+// Coefficient of tap C of the interior D2 row from the variable coefficients
+// b(0), b(1), ...; the zeros of the order's table are left out at compile time
+// (4/2: 6 of 25).
+template <int NARROW, int C, int Q, class F>
+__device__ __forceinline__ float narrow_tap(F b) {
+  constexpr float c = NarrowShape<NARROW>::template in32<C, Q>;
+  float acc = 0.f;
+  if constexpr (Q > 0) acc = narrow_tap<NARROW, C, Q - 1>(b);
+  if constexpr (c != 0.f) acc = __fmaf_rn(c, b(Q), acc);
+  return acc;
+}
+template <int NARROW, int C, class F>
+__device__ __forceinline__ void narrow_taps(float* a, F b) {
+  if constexpr (C > 0) narrow_taps<NARROW, C - 1>(a, b);
+  a[C] = narrow_tap<NARROW, C, NarrowShape<NARROW>::w - 1>(b);
+}
+
 // SYNC_IN: Ein is the edge buffer of the kernel that wrote f, whose
 // panel-side nodes still need their cube-edge scalar sync: the block applies
 // it to the staged values of those nodes (value slot c of Ein for field c),
@@ -277,7 +313,8 @@ __global__ void __launch_bounds__(LTPB, 4) lap_tile_kernel(FieldGeom g, int nty,
   const int n = g.n, P = g.P;
   const int p = blockIdx.y / nty, ty = blockIdx.y - p * nty;
   const int tw = min(LTX, n), th = min(LTY, n);
-  const int i0 = min((int)blockIdx.x * LTX, n - tw), j0 = min(ty * LTY, n - th);
+  const int i0 = lap_tile_start(blockIdx.x, gridDim.x, LTX, n, S::rows);
+  const int j0 = lap_tile_start(ty, nty, LTY, n, S::rows);
   int xlo, xhi, ylo, yhi;
   lap_region<NARROW>(i0, tw, n, xlo, xhi);
   lap_region<NARROW>(j0, th, n, ylo, yhi);
@@ -293,26 +330,53 @@ __global__ void __launch_bounds__(LTPB, 4) lap_tile_kernel(FieldGeom g, int nty,
   // Region rows go to thread rows, region columns to lanes.
   const T* MJp = mt + MJ * g.fs + pb;
   const T* MQp = mt + MQI2 * g.fs + pb;
-  for (int y = ly; y < ry; y += LTY) {
-    const long long rowa = (long long)(ylo + y) * P;
-    for (int x = lx; x < rx; x += LTX) {
+  const bool inner = xin && yin;
+  constexpr int IX = LTX + 2 * LT::R, IY = LTY + 2 * LT::R;   // region of an inner tile
+  if (inner) {
+    // the region's size is known: its nodes in one run over the threads, where
+    // the loops below take a second turn for the few columns past a warp
+    const T* fp = f + pb + (long long)ylo * P + xlo;
+    const T* jp = MJp + (long long)ylo * P + xlo;
+    const T* qp = MQp + (long long)ylo * P + xlo;
+    const T* bp = bco + pb + (long long)ylo * P + xlo;
+    for (int e = ly * LTX + lx; e < IX * IY; e += LTPB) {
+      const int y = e / IX, x = e - y * IX, a = y * P + x;
 #pragma unroll
-      for (int c = 0; c < NF; ++c) cp_async4(&Fs[c][y][x], f + c * g.fs + pb + rowa + xlo + x);
+      for (int c = 0; c < NF; ++c) cp_async4(&Fs[c][y][x], fp + c * g.fs + a);
+      const int xi = x - LT::R, yi = y - LT::R;
+      if ((unsigned)xi < LTX) {
+        cp_async4(&JXs[y][xi], jp + a);
+        cp_async4(&QXs[y][xi], qp + a);
+        cp_async4(&BYs[y][xi], bp + g.fs + a);
+      }
+      if ((unsigned)yi < LTY) {
+        cp_async4(&JYs[yi][x], jp + a);
+        cp_async4(&QYs[yi][x], qp + a);
+        cp_async4(&BXs[yi][x], bp + a);
+      }
     }
-    if (lx < tw) {
-      const long long a = rowa + i0 + lx;
-      cp_async4(&JXs[y][lx], MJp + a);
-      cp_async4(&QXs[y][lx], MQp + a);
-      cp_async4(&BYs[y][lx], bco + g.fs + pb + a);
+  } else {
+    for (int y = ly; y < ry; y += LTY) {
+      const long long rowa = (long long)(ylo + y) * P;
+      for (int x = lx; x < rx; x += LTX) {
+  #pragma unroll
+        for (int c = 0; c < NF; ++c) cp_async4(&Fs[c][y][x], f + c * g.fs + pb + rowa + xlo + x);
+      }
+      if (lx < tw) {
+        const long long a = rowa + i0 + lx;
+        cp_async4(&JXs[y][lx], MJp + a);
+        cp_async4(&QXs[y][lx], MQp + a);
+        cp_async4(&BYs[y][lx], bco + g.fs + pb + a);
+      }
     }
-  }
-  if (ly < th) {
-    const long long rowa = (long long)(j0 + ly) * P;
-    for (int x = lx; x < rx; x += LTX) {
-      const long long a = rowa + xlo + x;
-      cp_async4(&JYs[ly][x], MJp + a);
-      cp_async4(&QYs[ly][x], MQp + a);
-      cp_async4(&BXs[ly][x], bco + pb + a);
+    if (ly < th) {
+      const long long rowa = (long long)(j0 + ly) * P;
+      for (int x = lx; x < rx; x += LTX) {
+        const long long a = rowa + xlo + x;
+        cp_async4(&JYs[ly][x], MJp + a);
+        cp_async4(&QYs[ly][x], MQp + a);
+        cp_async4(&BXs[ly][x], bco + pb + a);
+      }
     }
   }
   cp_async_wait_all();
@@ -359,7 +423,17 @@ __global__ void __launch_bounds__(LTPB, 4) lap_tile_kernel(FieldGeom g, int nty,
       }
     }
   }
-  if (ly < th) {
+  if (inner) {
+    for (int e = ly * LTX + lx; e < LTY * IX; e += LTPB) {
+      const int y = e / IX, x = e - y * IX;
+      const T jq = JYs[y][x], qq = QYs[y][x];
+#pragma unroll
+      for (int c = 0; c < NF; ++c) {
+        const T dy = d_interior<NARROW, T>([&](int o) { return Fs[c][y + LT::R + o][x]; });
+        DYs[c][y][x] = dy * jq * qq;
+      }
+    }
+  } else if (ly < th) {
     const int j = j0 + ly;
     for (int x = lx; x < rx; x += LTX) {
       const T jq = JYs[ly][x], qq = QYs[ly][x];
@@ -377,22 +451,13 @@ __global__ void __launch_bounds__(LTPB, 4) lap_tile_kernel(FieldGeom g, int nty,
 
   const int i = i0 + lx, j = j0 + ly;
   const int yr = j - ylo, xr = i - xlo;
-  if (xin && yin) {
+  if (inner) {
     // A tile with no closure node and no panel side (most tiles): the same
     // terms in the same order as below, with every stencil offset known at
     // compile time and no per-node tests.
     T ax[S::w], ay[S::w];
-#pragma unroll
-    for (int c = 0; c < S::w; ++c) {
-      T accx = T(0), accy = T(0);
-#pragma unroll
-      for (int q = 0; q < S::w; ++q) {
-        accx += c_in32.v[S::ni][c][q] * BXs[ly][xr - S::hw + q];
-        accy += c_in32.v[S::ni][c][q] * BYs[yr - S::hw + q][lx];
-      }
-      ax[c] = accx;
-      ay[c] = accy;
-    }
+    narrow_taps<NARROW, S::w - 1>(ax, [&](int q) { return BXs[ly][xr - S::hw + q]; });
+    narrow_taps<NARROW, S::w - 1>(ay, [&](int q) { return BYs[yr - S::hw + q][lx]; });
     const T inv = T(1) / (hs2 * JXs[yr][lx]);
 #pragma unroll
     for (int c = 0; c < NF; ++c) {

@@ -150,6 +150,25 @@ def test_fp32_diffusion_small_panels(N, narrow):
         assert rel_l2(a, b, J) <= 1e-4
 
 
+@pytest.mark.parametrize("N,narrow", [(64, 42), (95, 42), (96, 42), (101, 42), (96, 63), (104, 63), (96, 21), (97, 21)])
+def test_fp32_diffusion_tile_ends(N, narrow):
+    """The FP32 Laplacian where the last tile but one of a line is moved (panel
+    lines of k*32 + 1 nodes and up to the closure rows more), where it just is
+    not, and where the move would run into the near closure: the tendency
+    stays within 1e-4 of FP64, the small panels' bound."""
+    res = {}
+    for prec in ("fp64", "fp32"):
+        op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=42, precision=prec))
+        dop = swm.OperatorSWMDiff(op, UV[narrow], 0.03, H[narrow], 0.01)
+        x, t = op.create_stvec(), op.create_stvec()
+        x.upload(*_state(N))
+        dop.apply(t, x)
+        res[prec] = t.download()
+    J = oracle.OracleDomain(N, 42).geometry()["J"]
+    for a, b in zip(res["fp32"], res["fp64"]):
+        assert rel_l2(a, b, J) <= 1e-4
+
+
 def test_fp32_diffusion_tendency_tracks_fp64():
     N = 48
     res = {}
