@@ -720,14 +720,6 @@ cudaError_t launch_axpby(long long count, double s1, const double* a, double s2,
 }
 
 template <class T>
-cudaError_t launch_sync_scalar_t(const FieldGeom& g, const Topology& tp, T* f, T* edge,
-                                 cudaStream_t st) {
-  const int nb = 6 * (4 * g.n - 4);
-  gather_edge_kernel<T><<<nblk(nb), TPB, 0, st>>>(g, f, EV_ZETA, nullptr, 0, edge);
-  sync_scalar_kernel<T><<<nblk(nb), TPB, 0, st>>>(g, tp, edge, f);
-  return cudaGetLastError();
-}
-template <class T>
 cudaError_t launch_sync_vector_t(const FieldGeom& g, const Topology& tp, const double* qw, T* gx,
                                  T* gy, T* edge, cudaStream_t st) {
   const int nb = 6 * (4 * g.n - 4);
@@ -735,10 +727,6 @@ cudaError_t launch_sync_vector_t(const FieldGeom& g, const Topology& tp, const d
   sync_vector_kernel<T><<<nblk(nb), TPB, 0, st>>>(g, tp, qw, edge, gx, gy);
   return cudaGetLastError();
 }
-template cudaError_t launch_sync_scalar_t<float>(const FieldGeom&, const Topology&, float*, float*,
-                                                 cudaStream_t);
-template cudaError_t launch_sync_scalar_t<double>(const FieldGeom&, const Topology&, double*,
-                                                  double*, cudaStream_t);
 template cudaError_t launch_sync_vector_t<float>(const FieldGeom&, const Topology&, const double*,
                                                  float*, float*, float*, cudaStream_t);
 template cudaError_t launch_sync_vector_t<double>(const FieldGeom&, const Topology&, const double*,
@@ -746,7 +734,10 @@ template cudaError_t launch_sync_vector_t<double>(const FieldGeom&, const Topolo
 
 cudaError_t launch_sync_scalar(const FieldGeom& g, const Topology& tp, double* f, double* edge,
                                cudaStream_t st) {
-  return launch_sync_scalar_t<double>(g, tp, f, edge, st);
+  const int nb = 6 * (4 * g.n - 4);
+  gather_edge_kernel<double><<<nblk(nb), TPB, 0, st>>>(g, f, EV_ZETA, nullptr, 0, edge);
+  sync_scalar_kernel<double><<<nblk(nb), TPB, 0, st>>>(g, tp, edge, f);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_sync_vector(const FieldGeom& g, const Topology& tp, const double* qw,

@@ -54,10 +54,7 @@ cudaError_t launch_sync_scalar(const FieldGeom& g, const Topology& tp, double* f
                                cudaStream_t st);
 cudaError_t launch_sync_vector(const FieldGeom& g, const Topology& tp, const double* qw,
                                double* gx, double* gy, double* edge, cudaStream_t st);
-// the same syncs on fields of either precision (edge buffer of that precision)
-template <class T>
-cudaError_t launch_sync_scalar_t(const FieldGeom& g, const Topology& tp, T* f, T* edge,
-                                 cudaStream_t st);
+// the vector sync on fields of either precision (edge buffer of that precision)
 template <class T>
 cudaError_t launch_sync_vector_t(const FieldGeom& g, const Topology& tp, const double* qw, T* gx,
                                  T* gy, T* edge, cudaStream_t st);
