@@ -405,14 +405,16 @@ InstDev<T> base_inst(swm_ctx* c) {
   I.qw = c->qw;
   I.hs = (const T*)c->hsT;
   I.edge = (T*)c->edge;
-  if constexpr (sizeof(T) == 8) I.der = der_fields(c, 0);
   I.ghs = (T)c->ghs;
   I.grav = (T)c->cfg.grav;
-  // constants of the FP64 stage, so that no thread forms them
-  const SbpC& tab = kTables[sbp_index(c->order)];
-  I.grav2 = (T)(2.0 * c->cfg.grav);
-  I.ghs2 = (T)(0.5 * c->ghs);
-  for (int o = 1; o <= tab.H; ++o) I.gc[o - 1] = (T)(0.5 * c->ghs * tab.Qin[o - tab.inshift]);
+  if constexpr (sizeof(T) == 8) {
+    I.der = der_fields(c, 0);
+    // constants of the FP64 stage, so that no thread forms them
+    const SbpC& tab = kTables[sbp_index(c->order)];
+    I.grav2 = 2.0 * c->cfg.grav;
+    I.ghs2 = 0.5 * c->ghs;
+    for (int o = 1; o <= tab.H; ++o) I.gc[o - 1] = 0.5 * c->ghs * tab.Qin[o - tab.inshift];
+  }
   return I;
 }
 

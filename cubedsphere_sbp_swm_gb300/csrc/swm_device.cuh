@@ -192,8 +192,18 @@ struct WorkUnit {
 };
 
 // Per-instance pointers and constants of one fused stage launch.
+// (the FP64 stage's part, which FP32 kernels do not carry as a parameter)
 template <class T>
-struct InstDev {
+struct InstDev64 {};
+template <>
+struct InstDev64<double> {
+  const double* der;   // stencil inputs of `in` (DR_N fields)
+  double* der_out;     // stencil inputs of the next stage state (nullable)
+  double grav2, ghs2;  // 2 grav, ghs / 2
+  double gc[3];        // ghs / 2 times the interior coefficients
+};
+template <class T>
+struct InstDev : InstDev64<T> {
   int n, P;
   int boxw;                   // TMA box width (columns) of this instance's strips
   long long ps, fs;           // panel stride n*P, field stride 6*n*P
@@ -207,15 +217,11 @@ struct InstDev {
   T* base_lo;                 // FP32 RK4 final stage: S_lo; S_hi is written via base_out
   T* base_out;                // final stage: new state (FP64 v0 / FP32 S_hi)
   T* edge;                    // edge buffer (6*4*4*n)
-  const T* der;               // FP64: stencil inputs of `in` (DR_N fields)
-  T* der_out;                 // FP64: stencil inputs of the next stage state (nullable)
   const StageMaps* maps;      // TMA maps of this instance (batched launches; else null)
   T c_in;                     // stage coefficient for the next stage state
   T c_acc;                    // stage coefficient for the running sum
   T ghs;                      // 1 / (hx * a)
   T grav;
-  T grav2, ghs2;              // FP64 stage: 2 grav, ghs / 2
-  T gc[3];                    // FP64 stage: ghs / 2 times the interior coefficients
 };
 
 enum StageMode { MODE_APPLY = 0, MODE_RK1 = 1, MODE_RK2 = 2, MODE_RK3 = 3, MODE_RK4 = 4 };
