@@ -85,11 +85,10 @@ cudaError_t cgrid_contra2co(CGrid* c, const double* ut, const double* vt, double
 // -(c^4) of the two coefficients.  cgrid_diffusion*: the tendency of the
 // state in into out (distinct); cgrid_diffusion_step*: one explicit Euler
 // step in place (FP32: on the (hi, lo) pair, with an exact two-sum).  The three
-// parts run as three branches (the stream st and two side streams of the
-// context, forked and joined with events).  cgrid_diffusion_prepare
-// allocates their work fields, streams and events; call it once, outside
-// any stream capture, before the others (they return cudaErrorInvalidValue
-// until then).
+// parts advance together, a launch for pass k of all of them
+// (swm_cgrid_diff.cuh), on st.  cgrid_diffusion_prepare allocates their work
+// fields; call it once, outside any stream capture, before the others (they
+// return cudaErrorInvalidValue until then).
 cudaError_t cgrid_diffusion_prepare(CGrid* c);
 cudaError_t cgrid_diffusion(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
                             const double* in, double* out, cudaStream_t st);
