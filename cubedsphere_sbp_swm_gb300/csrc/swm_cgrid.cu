@@ -1586,7 +1586,7 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
               }
               hm[(size_t)j * g.P + i] = x;
             }
-          ok(cudaMemcpy(dst + p * g.ps, hm.data(), sizeof(double) * g.ps, cudaMemcpyHostToDevice));
+          ok(upload_on(st, dst + p * g.ps, hm.data(), sizeof(double) * g.ps));   // the copies below read it on st
         }
         for (int p = 1; p < 6 && k != M_FP; ++p)
           ok(cudaMemcpyAsync(dst + p * g.ps, dst, sizeof(double) * g.ps, cudaMemcpyDeviceToDevice, st));

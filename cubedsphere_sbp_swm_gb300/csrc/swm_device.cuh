@@ -29,6 +29,16 @@ struct StageMaps {
   CUtensorMap hs;    // orography           box {boxw, rps, 1}
 };
 
+// Copy of set-up data from pageable host memory, complete on return and ordered
+// with what runs on st.  Contexts and ensembles have non-blocking streams, which
+// do not wait for the legacy default stream; a plain cudaMemcpy runs there
+// and may return (always, up to 64 KB) before its data have landed, so a kernel
+// or copy on st could read what the allocation held before.
+inline cudaError_t upload_on(cudaStream_t st, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 // Launch shape of the fused stage kernel of one precision and SBP order.
 struct StageShape {
   int ctas_per_sm;   // resident CTAs per SM

@@ -1,4 +1,6 @@
 """Shared helpers of the GPU parity tests."""
+import contextlib
+
 import numpy as np
 
 
@@ -11,3 +13,18 @@ def rel_l2(a, b, J):
 
 def fmt7(x):
     return "%.6E" % x
+
+
+@contextlib.contextmanager
+def busy_default_stream():
+    """Some 100 ms of work queued on the legacy default stream (another
+    library's, say), so that nothing else put there runs before it."""
+    import torch
+    a = torch.ones(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(300):
+        a.mul_(1.0)
+    try:
+        yield
+    finally:
+        torch.cuda.synchronize()

@@ -25,7 +25,7 @@ import oracle
 from cubedsphere_sbp_swm_gb300 import initial
 from analytic_fields import cross_polar as _cross_polar, solid_rotation as _solid_rotation
 from analytic_fields import vsh_curl_free_10 as _vsh_curl_free_10
-from gpu_helpers import fmt7
+from gpu_helpers import busy_default_stream, fmt7
 
 pytestmark = pytest.mark.gpu
 
@@ -280,6 +280,30 @@ def test_fused_passes_match_unfused_operators(order, N):
     op.apply_unfused(b, x)
     for f, g in zip(a.download(), b.download()):
         assert _rel(f, g) < 1e-10, _rel(f, g)
+
+
+# A panel of a metric field is below 64 KB here, which a copy on the default
+# stream does not wait for; the context made before leaves other values in the
+# memory the new one gets.
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", [20, 64])
+def test_context_made_while_the_default_stream_is_busy(N, prec):
+    def tendency():
+        op = c_op(N, 42, precision=prec)
+        x = op.create_stvec()
+        x.upload(*_state(N))
+        y = x.create_similar()
+        op.apply(y, x)
+        out = y.download()
+        op.close()
+        return out
+
+    want = tendency()
+    c_op(N, 21, precision=prec, radius=1.0, omega=1.0).close()
+    with busy_default_stream():
+        got = tendency()
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("order,N,steps", [(42, 40, 1), (42, 40, 24), (21, 40, 24), (42, 96, 2)])
