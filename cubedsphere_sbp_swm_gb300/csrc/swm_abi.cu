@@ -682,7 +682,7 @@ int stage_layout(swm_ctx* ctx, int cols, int seg_rows = 0, int grid = 0, int box
   CK(cudaStreamSynchronize(ctx->st), "sync");
   WorkUnit* d = nullptr;
   CK(cudaMalloc(&d, sizeof(WorkUnit) * units.size()), "alloc");
-  cudaError_t e = cudaMemcpy(d, units.data(), sizeof(WorkUnit) * units.size(), cudaMemcpyHostToDevice);
+  cudaError_t e = upload_on(ctx->st, d, units.data(), sizeof(WorkUnit) * units.size());
   if (e != cudaSuccess) { cudaFree(d); return cuda_fail(ctx, e, "copy units"); }
   if (ctx->units) cudaFree(ctx->units);
   ctx->units = d;
@@ -1058,7 +1058,7 @@ int swm_ctx_create_named(const swm_config* cfg, const char* div_op_name, const c
     std::vector<double> A(ctx->n, 1.0);
     for (int i = 0; i < std::min(q.nA, ctx->n); ++i) A[i] = q.A[i];
     for (int i = std::max(ctx->n - q.nA, 0); i < ctx->n; ++i) A[i] = q.A[ctx->n - 1 - i];
-    CKC(cudaMemcpy(ctx->Aw, A.data(), sizeof(double) * ctx->n, cudaMemcpyHostToDevice), "copy");
+    CKC(upload_on(ctx->st, ctx->Aw, A.data(), sizeof(double) * ctx->n), "copy");
   }
   CKC(cudaStreamSynchronize(ctx->st), "sync");
 #undef CKC
@@ -2411,8 +2411,7 @@ int ens_units(swm_ensemble* ens, int seg_rows) {
     ECK(cudaMalloc(&ens->dunits, sizeof(WorkUnit) * all.size()), "alloc units");
     ens->cap_units = (int)all.size();
   }
-  ECK(cudaMemcpy(ens->dunits, all.data(), sizeof(WorkUnit) * all.size(), cudaMemcpyHostToDevice),
-      "copy units");
+  ECK(upload_on(ens->st, ens->dunits, all.data(), sizeof(WorkUnit) * all.size()), "copy units");
   ens->nunits = (int)all.size();
   ens->seg_rows = seg_rows;
   return SWM_OK;
@@ -2450,10 +2449,8 @@ int ens_tables(swm_ensemble* ens) {
       inst[i * M + m] = I;
     }
   }
-  ECK(cudaMemcpy(ens->dmaps, maps.data(), sizeof(StageMaps) * maps.size(), cudaMemcpyHostToDevice),
-      "copy maps");
-  ECK(cudaMemcpy(ens->dinst, inst.data(), sizeof(InstDev<T>) * inst.size(), cudaMemcpyHostToDevice),
-      "copy instances");
+  ECK(upload_on(ens->st, ens->dmaps, maps.data(), sizeof(StageMaps) * maps.size()), "copy maps");
+  ECK(upload_on(ens->st, ens->dinst, inst.data(), sizeof(InstDev<T>) * inst.size()), "copy instances");
   return SWM_OK;
 }
 
@@ -3309,10 +3306,10 @@ int swm_latlon_create(swm_ctx* ctx, int nlon, int nlat, const char* interp_type,
   if (e == cudaSuccess) e = cudaMalloc(&r->out, sizeof(double) * 3 * np);
   if (e == cudaSuccess) e = cudaMalloc(&r->out32, sizeof(float) * 2 * np);
   if (e == cudaSuccess) e = cudaMallocHost(&r->hout32, sizeof(float) * 2 * np);
-  if (e == cudaSuccess) e = cudaMemcpy(r->base, h.base.data(), sizeof(long long) * np, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(r->wx, h.wx.data(), sizeof(double) * 4 * np, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(r->wy, h.wy.data(), sizeof(double) * 4 * np, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(r->rot, h.rot.data(), sizeof(double) * 4 * np, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload_on(ctx->st, r->base, h.base.data(), sizeof(long long) * np);
+  if (e == cudaSuccess) e = upload_on(ctx->st, r->wx, h.wx.data(), sizeof(double) * 4 * np);
+  if (e == cudaSuccess) e = upload_on(ctx->st, r->wy, h.wy.data(), sizeof(double) * 4 * np);
+  if (e == cudaSuccess) e = upload_on(ctx->st, r->rot, h.rot.data(), sizeof(double) * 4 * np);
   if (e != cudaSuccess) {
     release_latlon(r);
     delete r;

@@ -1901,7 +1901,7 @@ cudaError_t xy_prepare(CGrid* c, bool metric, cudaStream_t st) {
         }
     CKE(cudaStreamSynchronize(st));
     CKE(cudaMalloc(&c->xy_mt, sizeof(double) * t.size()));
-    CKE(cudaMemcpy(c->xy_mt, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
+    CKE(upload_on(st, c->xy_mt, t.data(), sizeof(double) * t.size()));
   }
   return cudaSuccess;
 }
