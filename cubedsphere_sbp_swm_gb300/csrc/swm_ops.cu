@@ -285,8 +285,8 @@ __device__ __forceinline__ double div_raw(const OpArgs& A, int p, int i, int j) 
 #pragma unroll
     for (int k = 0; k < Taps<ORD>::NT; ++k) {
       const int ox = tx.s + k - i, oy = (ty.s + k - j) * P;
-      s += tx.c[k] * (J[ox] * A.a[x + ox]);
-      s += ty.c[k] * (J[oy] * A.b[x + oy]);
+      s += tx.c[k] * (J[ox] * (tx.has(k) ? A.a[x + ox] : 0.0));
+      s += ty.c[k] * (J[oy] * (ty.has(k) ? A.b[x + oy] : 0.0));
     }
   }
   return s * A.m[MRJ * g.fs + x];
@@ -459,7 +459,7 @@ __device__ __forceinline__ double diag_op(int k, double x, double y) {
 }
 
 template <int ORD>
-__global__ void __launch_bounds__(PT_TPB)
+__global__ void __launch_bounds__(PT_TPB, DIAG_BLOCKS / 152)   // its grid is one wave
     diag_kernel(const __grid_constant__ OpArgs a, const __grid_constant__ Topology tp, const double* h,
                 const double* hs, const double* Aw, double grav, double hx2, int threads, double* partial) {
   const FieldGeom& g = a.g;

@@ -244,16 +244,24 @@ __device__ __forceinline__ T d_scaled(const T (&c)[3], F dif) {
   return s;
 }
 
-// The SBP derivative at line index k as one row of taps: sum_m c[m] f(s + m),
-// closure or interior alike, zero past the row.  No branch separates the loads
-// of one derivative from the next, so a panel-boundary node waits for memory
-// once a direction and not once a derivative (with d_line in its place the RK4
-// step took 0.085 ms at N=48 and 0.141 at N=192, against 0.052 and 0.112).
+// The SBP derivative at line index k as one row of taps: sum_m c[m] f(s + m) over
+// the taps m in the bit set `on`, closure or interior alike.  All taps are loaded
+// and a value of one that the row does not have is replaced by zero (a select, not
+// a product with a zero coefficient), so that an infinity or NaN outside the
+// row's stencil stays out of the sum.  With predicated loads in its place the
+// stage kernel spilled 80 to 180 bytes (N=384 d42 0.356 ms a step, 0.345 so),
+// with predicated sums it waited longer (N=64 0.059 against 0.055).
+// No branch separates the loads of one derivative from the next, so a
+// panel-boundary node waits for memory once a direction and not once a
+// derivative (with d_line in its place the RK4 step took 0.085 ms at N=48 and
+// 0.141 at N=192, against 0.052 and 0.112).
 template <int ORD>
 struct Taps {
   static constexpr int NT = Ord<ORD>::NW > 2 * Ord<ORD>::H + 1 ? Ord<ORD>::NW : 2 * Ord<ORD>::H + 1;
   int s;
+  unsigned on;
   double c[NT];
+  __device__ __forceinline__ bool has(int m) const { return on >> m & 1u; }
 };
 template <int ORD>
 __device__ __forceinline__ Taps<ORD> taps_of(int k, int n) {
@@ -262,6 +270,8 @@ __device__ __forceinline__ Taps<ORD> taps_of(int k, int n) {
   const bool left = k < NE, right = k >= n - NE;
   const int r = left ? k : right ? n - 1 - k : 0, last = c_sbp[ID].last[r];
   t.s = left ? 0 : right ? n - NT : k - H;
+  const unsigned row = (1u << last) - 1u;
+  t.on = left ? row : right ? row << (NT - last) : ((1u << (2 * H + 1)) - 1u) & ~(1u << H);
 #pragma unroll
   for (int m = 0; m < NT; ++m) {
     const int mm = right ? NT - 1 - m : m;
@@ -278,7 +288,7 @@ __device__ __forceinline__ double taps_sum(const Taps<ORD>& t, const double* __r
 #pragma unroll
   for (int m = 0; m < Taps<ORD>::NT; ++m) v[m] = __ldg(q + m * st);
 #pragma unroll
-  for (int m = 0; m < Taps<ORD>::NT; ++m) s += t.c[m] * v[m];
+  for (int m = 0; m < Taps<ORD>::NT; ++m) s += t.c[m] * (t.has(m) ? v[m] : 0.0);
   return s;
 }
 

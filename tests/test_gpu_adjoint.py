@@ -74,6 +74,22 @@ def test_operator_dot_product_small_panels(order, n_cells):
     assert abs(a - b) <= 1e-10 * max(abs(a), abs(b))
 
 
+@pytest.mark.parametrize("order,reach", [(42, 2), (43, 2), (63, 3)])
+def test_infinite_base_value_stays_within_its_stencils(order, reach):
+    """On a panel side the stencils along the side are interior ones and reach
+    so many nodes: an infinite base wind leaves the nodes past them finite."""
+    n, j0 = 24, 12
+    op = swm.OperatorSWM(swm.ModelConfig(N=n, sbp_order=order))
+    base = [a.copy() for a in initial.balanced_zonal(n, 3, 8)[:3]]
+    base[1][0, j0, 0] = base[2][0, j0, 0] = np.inf
+    lx = op.create_stvec()
+    ad.apply_ad(op, _stvec(op, base), _stvec(op, _rand(np.random.default_rng(5), op)), lx)
+    for a in lx.download():
+        assert not np.isfinite(a[0, j0, 0])
+        past = np.r_[j0 - 2 * reach - 2:j0 - reach, j0 + reach + 1:j0 + 2 * reach + 3]
+        assert np.isfinite(a[0, past, 0]).all()
+
+
 def test_tangent_linear_matches_central_differences(setup):
     op, x0 = setup
     rng = np.random.default_rng(12)

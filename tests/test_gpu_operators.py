@@ -134,6 +134,46 @@ def test_operators_and_diagnostics_small_panels(order, N):
         assert abs(a - b) < 1e-13 * abs(b)
 
 
+# The nodes that an infinite value may touch: those whose stencil holds its node
+# (the oracle's response to a unit value there) and the node's own copies.  At a
+# node past the closure row of a panel-boundary node, and on a panel side, where
+# the stencil along the side is an interior one.
+@pytest.mark.parametrize("order,i0", [(42, 4), (63, 6), (42, 0), (43, 0), (63, 0)])
+def test_infinite_values_stay_within_their_stencils(order, i0):
+    N, j0 = 24, 12
+    od, op = oracle.OracleDomain(N, order), swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=order))
+    zero, unit, bad = np.zeros(op.shape), np.zeros(op.shape), np.ones(op.shape)
+    unit[0, j0, i0], bad[0, j0, i0] = 1.0, np.inf
+    out = [op.create_field() for _ in range(2)]
+    one = _field(op, np.ones(op.shape))
+    own = od.sync_scalar(unit) != 0
+
+    def check(fields, *responses):
+        may = own.copy()
+        for r in responses:
+            may |= r != 0
+        for f in fields:
+            f = f.download() if hasattr(f, "download") else f
+            assert not np.isfinite(f).all() and np.isfinite(f[~may]).all()
+
+    grad, du, dv = od.grad(unit), od.div(unit, zero), od.div(zero, unit)
+    op.calc_grad(*out, _field(op, bad))
+    check(out, *grad)
+    op.calc_div(out[0], _field(op, bad), one)
+    check(out[:1], du)
+    op.calc_div(out[0], one, _field(op, bad))
+    check(out[:1], dv)
+    op.calc_curl(out[0], _field(op, bad), one)
+    check(out[:1], od.curl(unit, zero))
+    op.calc_curl(out[0], one, _field(op, bad))
+    check(out[:1], od.curl(zero, unit))
+    x = op.create_stvec()
+    x.upload(bad, np.ones(op.shape), np.ones(op.shape))
+    y = x.create_similar()
+    op.apply(y, x)
+    check(y.download(), *grad, du, dv)
+
+
 def test_syncs_match_oracle(pair):
     od, op, rng, _ = pair
     a = rng.standard_normal((6, op.n, op.n))
