@@ -264,6 +264,8 @@ def ensemble_leg(local, steps, warmup, peak):
     for m, N in enumerate(Ns):
         ens.upload(m, *initial.balanced_zonal(N, 1000 + m, 16)[:3])
     tuned = ens.tune(steps=5)
+    if tuned["seg_rows"] == ens.ROWS_AUTO:
+        tuned["seg_rows"] = "modelled"
     dev = torch.device("cuda", local)
     stream = torch.cuda.ExternalStream(ens.stream, device=dev)
     ens.step(warmup)

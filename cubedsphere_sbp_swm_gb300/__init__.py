@@ -682,6 +682,8 @@ class Ensemble:
         self._check(self._L.swm_ensemble_member(self._h, int(m), ctypes.byref(c), ctypes.byref(s)))
         return c, s
 
+    ROWS_AUTO = 2147483647  # seg_rows of the default split, units of equal modelled cost
+
     def set_shape(self, seg_rows: int, grid: int):
         self._check(self._L.swm_ensemble_set_shape(self._h, int(seg_rows), int(grid)))
 

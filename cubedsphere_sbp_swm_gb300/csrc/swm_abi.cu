@@ -2295,7 +2295,6 @@ struct swm_ensemble {
   WorkUnit* dunits = nullptr;
   int nunits = 0, cap_units = 0;
   int seg_rows = 0;                  // rows per work unit (0: whole panel height, kAutoRows: modelled)
-  int unit_rows = 0;                 // rows of the tallest unit
   int grid = 0;                      // persistent CTAs (0: one CTA per unit)
   cudaGraphExec_t graph = nullptr;
   std::string err;
@@ -2340,7 +2339,7 @@ std::string mem_err(swm_ensemble* ens) {
 // units, the earlier default, left a small ensemble on a few CTAs: 9 members
 // (3 each of N=48, 96, 192, d42, FP32) 485 us a step, with 456 such units
 // 125 us; 96 members 1044 us whole-panel, 1010 with 1728 units.
-constexpr int kAutoRows = -1;
+constexpr int kAutoRows = SWM_ENSEMBLE_ROWS_AUTO;
 
 double ens_makespan(const std::vector<double>& cost, int slots) {
   std::priority_queue<double, std::vector<double>, std::greater<double>> q;
@@ -2364,7 +2363,7 @@ int ens_units(swm_ensemble* ens, int seg_rows) {
   // the units of one member size
   auto units_of = [&](int n, int rows, double tau, std::vector<WorkUnit>& u) {
     u.clear();
-    const int nseg = rows > 0 ? std::max(1, (n + rows - 1) / rows) : rows == 0 ? 1 : 0;
+    const int nseg = rows == kAutoRows ? 0 : rows > 0 ? 1 + (n - 1) / rows : 1;
     return make_units(tab, n, ens->cols, 1, u, why, nseg, tau);
   };
   std::vector<WorkUnit> u;
@@ -2402,8 +2401,6 @@ int ens_units(swm_ensemble* ens, int seg_rows) {
   std::stable_sort(all.begin(), all.end(), [&](const WorkUnit& a, const WorkUnit& b) {
     return unit_cost(tab, ens->mem[a.inst]->n, a) > unit_cost(tab, ens->mem[b.inst]->n, b);
   });
-  ens->unit_rows = 0;
-  for (const WorkUnit& w : all) ens->unit_rows = std::max(ens->unit_rows, (int)(w.j1 - w.j0));
   if ((int)all.size() > ens->cap_units) {
     if (ens->dunits) cudaFree(ens->dunits);
     ens->dunits = nullptr;
@@ -2673,8 +2670,7 @@ int swm_ensemble_get_width(const swm_ensemble* ens, int* cols) {
 
 int swm_ensemble_get_shape(const swm_ensemble* ens, int* seg_rows, int* grid, int* nunits) {
   if (!ens) return efail(nullptr, SWM_E_INVALID, "null ensemble");
-  // the modelled split reports its tallest unit
-  if (seg_rows) *seg_rows = ens->seg_rows == kAutoRows ? ens->unit_rows : ens->seg_rows;
+  if (seg_rows) *seg_rows = ens->seg_rows;
   if (grid) *grid = ens->grid;
   if (nunits) *nunits = ens->nunits;
   return SWM_OK;
@@ -2722,7 +2718,7 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
     const int persistent = std::max(1, ens->occ) * ens->num_sms;
     const int grids[] = {persistent, 0};
     for (int si = 0; si < (int)(sizeof(segs) / sizeof(segs[0])) && rc == SWM_OK; ++si) {
-      if (segs[si] > 0 && segs[si] >= ens->max_n) continue;
+      if (segs[si] != kAutoRows && segs[si] >= ens->max_n) continue;
       for (int gi = 0; gi < 2 && rc == SWM_OK; ++gi) {
         if (!f32 && grids[gi] != 0) continue;  // FP64 kernel: one CTA per unit
         if (segs[si] == kAutoRows && grids[gi] != 0) continue;
@@ -2750,7 +2746,7 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
   if (rc == SWM_OK) rc = ens_rebuild(ens, best_seg, best_grid);
   if (rc == SWM_OK) {
     EMEM(sync_check(ens->mem[0], ens->st));
-    if (seg_rows_out) *seg_rows_out = best_seg == kAutoRows ? ens->unit_rows : best_seg;
+    if (seg_rows_out) *seg_rows_out = best_seg;
     if (grid_out) *grid_out = best_grid;
     if (ms_per_step_out) *ms_per_step_out = best;
   }

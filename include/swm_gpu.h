@@ -421,10 +421,12 @@ int  swm_ensemble_diagnostics(swm_ensemble* ens, int m, double out[7]);
 int  swm_ensemble_step(swm_ensemble* ens, int nsteps);
 int  swm_ensemble_synchronize(swm_ensemble* ens);
 void* swm_ensemble_stream(swm_ensemble* ens);
-/* Tile shape: a new ensemble splits its members into units of equal modelled
- * cost, one CTA each (get_shape then reports the rows of the tallest unit).
- * set_shape fixes the rows per work unit (0: whole panel height) and the persistent
- * CTAs of the stage kernel (0: one CTA per work unit). */
+/* Tile shape: rows per work unit (0: whole panel height) and persistent CTAs
+ * of the stage kernel (0: one CTA per work unit).  A new ensemble has
+ * SWM_ENSEMBLE_ROWS_AUTO rows and no persistent CTAs: units of equal modelled
+ * cost over all members.  What get_shape and tune return can be given back to
+ * set_shape. */
+#define SWM_ENSEMBLE_ROWS_AUTO 2147483647
 int  swm_ensemble_set_shape(swm_ensemble* ens, int seg_rows, int grid);
 /* Consumer width of the members' FP32 stage kernel (64, 96, 128, 160 or 192;
  * bit-identical results); swm_ensemble_tune also searches it. */

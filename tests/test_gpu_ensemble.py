@@ -101,6 +101,34 @@ def test_autotuner_keeps_states_and_picks_a_valid_shape(prec, states, single):
             assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_shapes_can_be_given_back(prec, states, single):
+    """The default split, a fixed one and the tuned one: setting what get_shape or
+    tune returned makes the same units again."""
+    ens = _ensemble(prec, states)
+    default = ens.get_shape()
+    ens.set_shape(24, 0)
+    fixed = ens.get_shape()
+    ens.set_shape(default["seg_rows"], default["grid"])
+    assert ens.get_shape() == default
+    ens.set_shape(fixed["seg_rows"], fixed["grid"])
+    assert ens.get_shape() == fixed
+    res = ens.tune(steps=2)
+    tuned = ens.get_shape()
+    ens.set_shape(16, 0)
+    ens.set_shape(res["seg_rows"], res["grid"])
+    assert ens.get_shape() == tuned
+    ens.set_shape(default["seg_rows"], 152)   # persistent CTAs on the default units
+    ens.step(3)
+    ens.synchronize()
+    for m in range(len(MEMBERS)):
+        for a, b in zip(ens.download(m), single[prec][m]):
+            assert np.array_equal(a, b)
+    for rows, grid in ((-1, 0), (0, -1)):
+        with pytest.raises(swm.SwmError):
+            ens.set_shape(rows, grid)
+
+
 def test_member_diagnostics_and_access(states):
     ens = _ensemble("fp32", states)
     d = ens.get_diagnostics(2)
