@@ -2717,12 +2717,17 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
     if (ens_set_width(ens, cols) != SWM_OK) continue;   // width cannot cover a member
     const int persistent = std::max(1, ens->occ) * ens->num_sms;
     const int grids[] = {persistent, 0};
-    for (int si = 0; si < (int)(sizeof(segs) / sizeof(segs[0])) && rc == SWM_OK; ++si) {
-      if (segs[si] != kAutoRows && segs[si] >= ens->max_n) continue;
-      for (int gi = 0; gi < 2 && rc == SWM_OK; ++gi) {
-        if (!f32 && grids[gi] != 0) continue;  // FP64 kernel: one CTA per unit
-        if (segs[si] == kAutoRows && grids[gi] != 0) continue;
-        if ((rc = ens_rebuild(ens, segs[si], grids[gi]))) break;
+    // FP64 has no work units, so every shape is the same launches: the set one
+    // is timed and stays
+    const int nseg = f32 ? (int)(sizeof(segs) / sizeof(segs[0])) : 1, ngrid = f32 ? 2 : 1;
+    const int set_seg = ens->seg_rows, set_grid = ens->grid;
+    for (int si = 0; si < nseg && rc == SWM_OK; ++si) {
+      const int seg = f32 ? segs[si] : set_seg;
+      if (f32 && seg != kAutoRows && seg >= ens->max_n) continue;
+      for (int gi = 0; gi < ngrid && rc == SWM_OK; ++gi) {
+        const int cta = f32 ? grids[gi] : set_grid;
+        if (f32 && seg == kAutoRows && cta != 0) continue;
+        if ((rc = ens_rebuild(ens, seg, cta))) break;
         cudaGraphLaunch(ens->graph, ens->st);                          // warm-up
         cudaEventRecord(a, ens->st);
         for (int k = 0; k < steps; ++k) cudaGraphLaunch(ens->graph, ens->st);
@@ -2732,7 +2737,7 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
         cudaEventElapsedTime(&ms, a, b);
         restore();
         if (ms / steps < best) {
-          best = ms / steps; best_seg = segs[si]; best_grid = grids[gi]; best_cols = cols;
+          best = ms / steps; best_seg = seg; best_grid = cta; best_cols = cols;
         }
       }
     }

@@ -129,6 +129,17 @@ def test_shapes_can_be_given_back(prec, states, single):
             ens.set_shape(rows, grid)
 
 
+def test_fp64_tuner_keeps_the_set_shape(states):
+    """The FP64 stage has no work units: there is one launch to time."""
+    ens = _ensemble("fp64", states)
+    for rows, grid in ((24, 0), (0, 152), (ens.ROWS_AUTO, 0), (16, 0)):
+        ens.set_shape(rows, grid)
+        want = ens.get_shape()
+        res = ens.tune(steps=1)
+        assert (res["seg_rows"], res["grid"]) == (rows, grid) and res["ms_per_step"] > 0
+        assert ens.get_shape() == want
+
+
 def test_member_diagnostics_and_access(states):
     ens = _ensemble("fp32", states)
     d = ens.get_diagnostics(2)
