@@ -247,61 +247,75 @@ int cuda_fail(swm_ctx* c, cudaError_t e, const char* where) {
 
 long long round_up(long long a, long long b) { return (a + b - 1) / b * b; }
 
-// Work units of the fused stage kernel: column strips x row segments, as
-// many as fit on the GPU at once (target_ctas) so no CTA waits for a wave,
-// or exactly nseg_fixed row segments per strip when that is > 0, or units of
-// a modelled cost of at most tau_fixed when that is > 0 (the ensemble, whose
-// members share one launch).
+// Work units of the FP32 stage kernel: column strips x row segments, of about
+// the same modelled cost in row-equivalents.  The model is measured per unit on
+// GB300: a strip on a panel edge costs 1 + kStripEdge per row (its closure columns
+// make one warp diverge, and the per-row barrier makes the CTA wait for
+// it); a closure row at a panel end costs 1 + row_closure_cost; every unit adds
+// kUnitHalo * rmax rows for its halo.
 constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
 constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
 constexpr int kSpread = 152;           // units that give every SM of a GB300 one
 double row_closure_cost(const SbpC& s) { return s.ne >= 6 ? 2.0 : 1.0; }
 
-bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<WorkUnit>& out,
-                std::string& why, int nseg_fixed = 0, double tau_fixed = 0.0) {
-  auto need_lo = [&](int k) {
-    if (k < s.ne) return 0;
-    if (k >= n - s.ne) return n - s.last[n - 1 - k];
-    return k - s.H;
-  };
-  auto need_hi = [&](int k) {
-    if (k < s.ne) return s.last[k] - 1;
-    if (k >= n - s.ne) return n - 1;
-    return k + s.H;
-  };
-  int nstrip = (n + (threads - 2 * s.rmax) - 1) / (threads - 2 * s.rmax);
-  std::vector<int> cs;
-  for (;; ++nstrip) {
-    cs.assign(nstrip + 1, 0);
-    for (int k = 0; k <= nstrip; ++k) cs[k] = (int)((long long)n * k / nstrip);
-    bool ok = true;
-    for (int k = 0; k < nstrip && ok; ++k) {
-      int lo = n, hi = 0;
-      for (int c = cs[k]; c < cs[k + 1]; ++c) { lo = std::min(lo, need_lo(c)); hi = std::max(hi, need_hi(c)); }
-      ok = (hi + 1 - lo) <= threads && (cs[k + 1] - cs[k]) >= 1;
-    }
-    if (ok) break;
-    if (nstrip > n) { why = "work split failed"; return false; }
+// The column strips of a panel of n nodes a side and the cost model of its rows.
+// Units of one panel serve all six, and unit counts need no units, so an
+// ensemble's search for its split costs little (a member of N=384: set-up
+// 7.7 -> 1.3 ms against building every trial's units).
+struct Split {
+  const SbpC& s;
+  int n, nstrip = 0;
+  std::vector<int> cs;        // column cuts
+  std::vector<double> pre;    // cost of the rows below
+
+  Split(const SbpC& tab, int nodes) : s(tab), n(nodes), pre(nodes + 1, 0.0) {}
+
+  // first and last node that the stencil at node k reads
+  int need_lo(int k) const { return k < s.ne ? 0 : k >= n - s.ne ? n - s.last[n - 1 - k] : k - s.H; }
+  int need_hi(int k) const { return k < s.ne ? s.last[k] - 1 : k >= n - s.ne ? n - 1 : k + s.H; }
+  void span(int a, int b, int& lo, int& hi) const {   // of nodes a..b-1; hi one past
+    lo = n;
+    hi = 0;
+    for (int c = a; c < b; ++c) { lo = std::min(lo, need_lo(c)); hi = std::max(hi, need_hi(c) + 1); }
   }
-  // Row cuts of every strip, so that units carry about the same modelled
-  // cost in row-equivalents.  The model is measured per unit on GB300: a
-  // strip on a panel edge costs 1 + kStripEdge per row (its closure columns
-  // make one warp diverge, and the per-row barrier makes the CTA wait for
-  // it); a closure row at a panel end costs 1 + kRowClosure; every unit adds
-  // 0.8 * rmax rows for its halo.  nseg_fixed > 0: inner strips get that many
-  // units and edge strips (1 + kStripEdge) times as many when the panel also
-  // has inner strips; otherwise the unit
-  // counts fill one wave of target_ctas.  Each strip is cut at equal shares
-  // of its row cost.
-  std::vector<std::vector<int>> cuts(nstrip);
-  const double kRowClosure = row_closure_cost(s), over = kUnitHalo * s.rmax;
-  std::vector<double> pre(n + 1, 0.0);
-  for (int j = 0; j < n; ++j)
-    pre[j + 1] = pre[j] + ((j < s.ne || j >= n - s.ne) ? 1.0 + kRowClosure : 1.0);
-  auto edge_strip = [&](int k) { return cs[k] == 0 || cs[k + 1] == n; };
-  auto cut_equal = [&](int k, int m) {
-    auto& c = cuts[k];
-    c.assign(1, 0);
+  bool init(int threads, std::string& why) {
+    nstrip = (n + (threads - 2 * s.rmax) - 1) / (threads - 2 * s.rmax);
+    for (;; ++nstrip) {
+      cs.assign(nstrip + 1, 0);
+      for (int k = 0; k <= nstrip; ++k) cs[k] = (int)((long long)n * k / nstrip);
+      bool ok = true;
+      for (int k = 0; k < nstrip && ok; ++k) {
+        int lo, hi;
+        span(cs[k], cs[k + 1], lo, hi);
+        ok = hi - lo <= threads && cs[k + 1] - cs[k] >= 1;
+      }
+      if (ok) break;
+      if (nstrip > n) { why = "work split failed"; return false; }
+    }
+    for (int j = 0; j < n; ++j)
+      pre[j + 1] = pre[j] + ((j < s.ne || j >= n - s.ne) ? 1.0 + row_closure_cost(s) : 1.0);
+    return true;
+  }
+  bool edge_strip(int k) const { return cs[k] == 0 || cs[k + 1] == n; }
+  double over() const { return kUnitHalo * s.rmax; }
+  // units of strip k for a unit cost of at most tau: m units of a strip of
+  // factor f cost f * (pre[n] + m * over) in total
+  int units_of(int k, double tau, int max_units) const {
+    const double f = edge_strip(k) ? 1.0 + kStripEdge : 1.0;
+    const double per = tau - f * over();
+    if (per <= 0.0) return max_units;
+    return std::max(1, std::min(max_units, (int)std::ceil(f * pre[n] / per - 1e-9)));
+  }
+  int total(double tau, int max_units) const {
+    int t = 0;
+    for (int k = 0; k < nstrip; ++k) t += units_of(k, tau, max_units);
+    return 6 * t;
+  }
+  // rows of a unit of an ensemble: three or more
+  int ens_max() const { return n / 3; }
+  // row cuts of a strip into m units of equal row cost
+  std::vector<int> cut_equal(int m) const {
+    std::vector<int> c(1, 0);
     int j = 0;
     for (int r = 1; r < m; ++r) {
       const double want = pre[n] * r / m;
@@ -309,62 +323,81 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
       if (j > c.back()) c.push_back(j);
     }
     c.push_back(n);
-  };
-  if (nseg_fixed > 0) {
-    // (with no inner strip every strip is an edge strip and none waits)
-    for (int k = 0; k < nstrip; ++k) {
-      const double m = nseg_fixed * (nstrip > 2 && edge_strip(k) ? 1.0 + kStripEdge : 1.0);
-      cut_equal(k, std::max(1, std::min(n, (int)std::lround(m))));
-    }
-  } else {
-    // At least 8 rows a unit; 3, up to a unit per SM, where 8 rows would leave
-    // half of the SMs without one.  On a panel too small to fill the GPU the
-    // row loop of a unit is the launch's latency; on a larger one shorter units
-    // only add halo rows.  d42 FP32, width 128, us a step of one instance / of
-    // three at once: N=48 51.4/18.4 at 8 rows, 41.3/15.9 at 3; N=96 49.4/19.1 at
-    // 8, 43.3/17.7 at 4; N=120 54.4/21.3 at 8, 48.2/23.1 at 4; N=144 54.4/26.8 at
-    // 8, 49.5/28.2 at 4.  (The ensemble's units are bounded by its own budget.)
-    const int at8 = std::max(1, n / std::min(8, n));
-    const int spread = 2 * 6 * nstrip * at8 <= kSpread ? kSpread / (6 * nstrip) : 0;
-    const int max_units = tau_fixed > 0.0 ? n / 3 : std::max(at8, std::min(n / 3, spread));
-    // units of strip k for a unit cost of at most tau: m units of a strip of
-    // factor f cost f * (pre[n] + m * over) in total
-    auto units_of = [&](int k, double tau) {
-      const double f = edge_strip(k) ? 1.0 + kStripEdge : 1.0;
-      const double per = tau - f * over;
-      if (per <= 0.0) return max_units;
-      return std::max(1, std::min(max_units, (int)std::ceil(f * pre[n] / per - 1e-9)));
-    };
-    auto total = [&](double tau) {
-      int t = 0;
-      for (int k = 0; k < nstrip; ++k) t += units_of(k, tau);
-      return 6 * t;
-    };
-    // the smallest unit cost whose units fit the wave
-    double lo = 0.0, hi = tau_fixed > 0.0 ? tau_fixed : (1.0 + kStripEdge) * (pre[n] + over);
-    const int budget = std::max(target_ctas, 6 * nstrip);
-    for (int it = 0; it < 60 && !(tau_fixed > 0.0); ++it) {
-      const double mid = 0.5 * (lo + hi);
-      if (total(mid) <= budget) hi = mid; else lo = mid;
-    }
-    for (int k = 0; k < nstrip; ++k) cut_equal(k, units_of(k, hi));
+    return c;
   }
-  for (int p = 0; p < 6; ++p)
-    for (int k = 0; k < nstrip; ++k)
-      for (size_t r = 0; r + 1 < cuts[k].size(); ++r) {
+  // the units of all panels, m[k] per strip k
+  void build(const std::vector<int>& m, std::vector<WorkUnit>& out) const {
+    const size_t first = out.size();
+    for (int k = 0; k < nstrip; ++k) {
+      const std::vector<int> cuts = cut_equal(m[k]);
+      int cl0, cl1;
+      span(cs[k], cs[k + 1], cl0, cl1);
+      for (size_t r = 0; r + 1 < cuts.size(); ++r) {
+        if (cuts[r + 1] <= cuts[r]) continue;
+        int rl0, rl1;
+        span(cuts[r], cuts[r + 1], rl0, rl1);
         WorkUnit w;
-        w.inst = 0; w.panel = (int16_t)p;
+        w.inst = 0; w.panel = 0;
         w.i0 = (int16_t)cs[k]; w.i1 = (int16_t)cs[k + 1];
-        w.j0 = (int16_t)cuts[k][r]; w.j1 = (int16_t)cuts[k][r + 1];
-        if (w.j1 <= w.j0) continue;
-        int lo = n, hi = 0;
-        for (int c = w.i0; c < w.i1; ++c) { lo = std::min(lo, need_lo(c)); hi = std::max(hi, need_hi(c)); }
-        w.cl0 = (int16_t)lo; w.cl1 = (int16_t)(hi + 1);
-        lo = n; hi = 0;
-        for (int c = w.j0; c < w.j1; ++c) { lo = std::min(lo, need_lo(c)); hi = std::max(hi, need_hi(c)); }
-        w.rl0 = (int16_t)lo; w.rl1 = (int16_t)(hi + 1);
+        w.j0 = (int16_t)cuts[r]; w.j1 = (int16_t)cuts[r + 1];
+        w.cl0 = (int16_t)cl0; w.cl1 = (int16_t)cl1;
+        w.rl0 = (int16_t)rl0; w.rl1 = (int16_t)rl1;
         out.push_back(w);
       }
+    }
+    const size_t count = out.size() - first;
+    out.reserve(first + 6 * count);
+    for (int p = 1; p < 6; ++p)
+      for (size_t q = 0; q < count; ++q) {
+        out.push_back(out[first + q]);
+        out.back().panel = (int16_t)p;
+      }
+  }
+  // units of a modelled cost of at most tau
+  void build_tau(double tau, int max_units, std::vector<WorkUnit>& out) const {
+    std::vector<int> m(nstrip);
+    for (int k = 0; k < nstrip; ++k) m[k] = units_of(k, tau, max_units);
+    build(m, out);
+  }
+  // nseg units a strip, edge strips 1 + kStripEdge times as many when the panel
+  // also has inner strips (with none, every strip is an edge strip and none waits)
+  void build_fixed(int nseg, std::vector<WorkUnit>& out) const {
+    std::vector<int> m(nstrip);
+    for (int k = 0; k < nstrip; ++k)
+      m[k] = std::max(1, std::min(n, (int)std::lround(nseg * (nstrip > 2 && edge_strip(k) ? 1.0 + kStripEdge : 1.0))));
+    build(m, out);
+  }
+};
+
+// Units of one instance: nseg_fixed row segments a strip when that is > 0, else
+// as many as fill one wave of target_ctas, each strip cut at equal shares of its
+// row cost.
+bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<WorkUnit>& out,
+                std::string& why, int nseg_fixed = 0) {
+  Split P(s, n);
+  if (!P.init(threads, why)) return false;
+  if (nseg_fixed > 0) {
+    P.build_fixed(nseg_fixed, out);
+    return true;
+  }
+  // At least 8 rows a unit; 3, up to a unit per SM, where 8 rows would leave
+  // half of the SMs without one.  On a panel too small to fill the GPU the
+  // row loop of a unit is the launch's latency; on a larger one shorter units
+  // only add halo rows.  d42 FP32, width 128, us a step of one instance / of
+  // three at once: N=48 51.4/18.4 at 8 rows, 41.3/15.9 at 3; N=96 49.4/19.1 at
+  // 8, 43.3/17.7 at 4; N=120 54.4/21.3 at 8, 48.2/23.1 at 4; N=144 54.4/26.8 at
+  // 8, 49.5/28.2 at 4.
+  const int at8 = std::max(1, n / std::min(8, n));
+  const int spread = 2 * 6 * P.nstrip * at8 <= kSpread ? kSpread / (6 * P.nstrip) : 0;
+  const int max_units = std::max(at8, std::min(n / 3, spread));
+  // the smallest unit cost whose units fit the wave
+  double lo = 0.0, hi = (1.0 + kStripEdge) * (P.pre[n] + P.over());
+  const int budget = std::max(target_ctas, 6 * P.nstrip);
+  for (int it = 0; it < 60; ++it) {
+    const double mid = 0.5 * (lo + hi);
+    if (P.total(mid, max_units) <= budget) hi = mid; else lo = mid;
+  }
+  P.build_tau(hi, max_units, out);
   return true;
 }
 
@@ -2356,48 +2389,52 @@ double ens_makespan(const std::vector<double>& cost, int slots) {
 
 int ens_units(swm_ensemble* ens, int seg_rows) {
   std::string why;
-  std::map<int, int> sizes;   // members of each edge length
-  for (const swm_ctx* c : ens->mem) ++sizes[c->n];
   const SbpC& tab = kTables[sbp_index(ens->order)];
-  const int slots = std::max(1, ens->occ) * ens->num_sms;
-  // the units of one member size
-  auto units_of = [&](int n, int rows, double tau, std::vector<WorkUnit>& u) {
-    u.clear();
-    const int nseg = rows == kAutoRows ? 0 : rows > 0 ? 1 + (n - 1) / rows : 1;
-    return make_units(tab, n, ens->cols, 1, u, why, nseg, tau);
+  struct Size {
+    Split split;
+    int members = 0;
+    std::vector<WorkUnit> units;   // of one member
   };
-  std::vector<WorkUnit> u;
-  double tau = 0.0;
+  std::map<int, Size> sizes;   // by edge length
+  for (const swm_ctx* c : ens->mem) {
+    auto it = sizes.find(c->n);
+    if (it == sizes.end()) {
+      it = sizes.emplace(c->n, Size{Split(tab, c->n)}).first;
+      if (!it->second.split.init(ens->cols, why)) return efail(ens, SWM_E_INVALID, why);
+    }
+    ++it->second.members;
+  }
   if (seg_rows == kAutoRows) {
-    double best = 0.0, top = 0.0;
+    const int slots = std::max(1, ens->occ) * ens->num_sms;
+    double best = 0.0, tau = 0.0, top = 0.0;
     for (const auto& sz : sizes) top = std::max(top, (1.0 + kStripEdge) * (3.0 * sz.first + kUnitHalo * tab.rmax));
     for (int waves = 1; waves <= 4; ++waves) {
       double lo = 0.0, hi = top;
       for (int it = 0; it < 16; ++it) {
         const double mid = 0.5 * (lo + hi);
         long long total = 0;
-        for (const auto& sz : sizes) {
-          if (!units_of(sz.first, kAutoRows, mid, u)) return efail(ens, SWM_E_INVALID, why);
-          total += (long long)sz.second * u.size();
-        }
+        for (const auto& sz : sizes)
+          total += (long long)sz.second.members * sz.second.split.total(mid, sz.second.split.ens_max());
         if (total <= (long long)waves * slots) hi = mid; else lo = mid;
       }
+      if (hi == tau) continue;   // the members' fewest units are more than another wave
       std::vector<double> cost;
-      for (const auto& sz : sizes) {
-        if (!units_of(sz.first, kAutoRows, hi, u)) return efail(ens, SWM_E_INVALID, why);
-        for (int m = 0; m < sz.second; ++m)
-          for (const WorkUnit& w : u) cost.push_back(unit_cost(tab, sz.first, w));
+      for (auto& sz : sizes) {
+        std::vector<WorkUnit> u;
+        sz.second.split.build_tau(hi, sz.second.split.ens_max(), u);
+        for (const WorkUnit& w : u) cost.insert(cost.end(), sz.second.members, unit_cost(tab, sz.first, w));
       }
       std::sort(cost.begin(), cost.end(), std::greater<double>());
       const double t = ens_makespan(cost, slots);
       if (tau == 0.0 || t < best) { tau = hi; best = t; }
     }
+    for (auto& sz : sizes) sz.second.split.build_tau(tau, sz.second.split.ens_max(), sz.second.units);
+  } else {
+    for (auto& sz : sizes) sz.second.split.build_fixed(seg_rows > 0 ? 1 + (sz.first - 1) / seg_rows : 1, sz.second.units);
   }
   std::vector<WorkUnit> all;
-  for (int m = 0; m < ens->nmem; ++m) {
-    if (!units_of(ens->mem[m]->n, seg_rows, tau, u)) return efail(ens, SWM_E_INVALID, why);
-    for (WorkUnit& w : u) { w.inst = (int16_t)m; all.push_back(w); }
-  }
+  for (int m = 0; m < ens->nmem; ++m)
+    for (WorkUnit w : sizes.at(ens->mem[m]->n).units) { w.inst = (int16_t)m; all.push_back(w); }
   std::stable_sort(all.begin(), all.end(), [&](const WorkUnit& a, const WorkUnit& b) {
     return unit_cost(tab, ens->mem[a.inst]->n, a) > unit_cost(tab, ens->mem[b.inst]->n, b);
   });
