@@ -255,6 +255,7 @@ long long round_up(long long a, long long b) { return (a + b - 1) / b * b; }
 // kUnitHalo * rmax rows for its halo.
 constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
 constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
+constexpr double kCrowdHalo = 3.3;     // the same where an ensemble's whole-panel units fill the GPU
 constexpr int kSpread = 152;           // units that give every SM of a GB300 one
 double row_closure_cost(const SbpC& s) { return s.ne >= 6 ? 2.0 : 1.0; }
 
@@ -267,6 +268,7 @@ struct Split {
   int n, nstrip = 0;
   std::vector<int> cs;        // column cuts
   std::vector<double> pre;    // cost of the rows below
+  double halo = kUnitHalo;    // cost of a unit's halo, in rows per RMAX
 
   Split(const SbpC& tab, int nodes) : s(tab), n(nodes), pre(nodes + 1, 0.0) {}
 
@@ -297,7 +299,7 @@ struct Split {
     return true;
   }
   bool edge_strip(int k) const { return cs[k] == 0 || cs[k + 1] == n; }
-  double over() const { return kUnitHalo * s.rmax; }
+  double over() const { return halo * s.rmax; }
   // units of strip k for a unit cost of at most tau: m units of a strip of
   // factor f cost f * (pre[n] + m * over) in total
   int units_of(int k, double tau, int max_units) const {
@@ -402,11 +404,11 @@ bool make_units(const SbpC& s, int n, int threads, int target_ctas, std::vector<
 }
 
 // Modelled cost of a unit, in row-equivalents (the model of make_units).
-double unit_cost(const SbpC& s, int n, const WorkUnit& w) {
+double unit_cost(const SbpC& s, int n, const WorkUnit& w, double halo = kUnitHalo) {
   const double f = (w.i0 == 0 || w.i1 == n) ? 1.0 + kStripEdge : 1.0;
   const int closed = std::max(0, std::min((int)w.j1, s.ne) - (int)w.j0) +
                      std::max(0, (int)w.j1 - std::max((int)w.j0, n - s.ne));
-  return f * ((w.j1 - w.j0) + closed * row_closure_cost(s) + kUnitHalo * s.rmax);
+  return f * ((w.j1 - w.j0) + closed * row_closure_cost(s) + halo * s.rmax);
 }
 
 bool name_order(const std::string& nm, const char* prefix, const char* suffix, int& order) {
@@ -569,7 +571,7 @@ int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode, bool derive = true) {
       CK(cudaEventCreate(&a), "event"); CK(cudaEventCreate(&b), "event");
       CK(cudaEventRecord(a, ctx->st), "event record");
     }
-    CK(launch_edge32(I, nullptr, 1, ctx->n, ctx->topo, mode, ctx->st), "edge kernel");
+    CK(launch_edge32(I, nullptr, 1, ctx->n, ctx->topo, mode, false, ctx->st), "edge kernel");
     if (ctx->timing) {
       CK(cudaEventRecord(b, ctx->st), "event record");
       ctx->ev_edge.emplace_back(a, b);
@@ -2329,6 +2331,7 @@ struct swm_ensemble {
   int nunits = 0, cap_units = 0;
   int seg_rows = 0;                  // rows per work unit (0: whole panel height, kAutoRows: modelled)
   int grid = 0;                      // persistent CTAs (0: one CTA per unit)
+  bool crowded = false;              // whole-panel units take half of the CTA slots or more
   cudaGraphExec_t graph = nullptr;
   std::string err;
 };
@@ -2372,6 +2375,14 @@ std::string mem_err(swm_ensemble* ens) {
 // units, the earlier default, left a small ensemble on a few CTAs: 9 members
 // (3 each of N=48, 96, 192, d42, FP32) 485 us a step, with 456 such units
 // 125 us; 96 members 1044 us whole-panel, 1010 with 1728 units.
+// A crowded ensemble, whose whole-panel units take half of the CTA slots or
+// more, has CTAs beside each other on every SM, and a shorter unit costs it more:
+// its halo rows are issue slots that another unit would have used.  From the
+// times of 17 such ensembles the halo of a unit is 3.3 rows per RMAX there.  With
+// 0.8: 60 members of N=32 157 us a step, 133 with 3.3 (whole-panel units 133); 100
+// of N=16 155 and 138 (152); 100 of N=20 d63 223 and 190 (215).  Ensembles below
+// half, where 3.3 gave 6% less for 10 members of N=128 d63 and 11% less for one of
+// N=512 with 20 of N=32, keep 0.8.
 constexpr int kAutoRows = SWM_ENSEMBLE_ROWS_AUTO;
 
 double ens_makespan(const std::vector<double>& cost, int slots) {
@@ -2404,10 +2415,17 @@ int ens_units(swm_ensemble* ens, int seg_rows) {
     }
     ++it->second.members;
   }
+  const int slots = std::max(1, ens->occ) * ens->num_sms;
+  long long fewest = 0;   // whole-panel units
+  for (const auto& sz : sizes) fewest += 6LL * sz.second.members * sz.second.split.nstrip;
+  ens->crowded = 2 * fewest >= slots;
   if (seg_rows == kAutoRows) {
-    const int slots = std::max(1, ens->occ) * ens->num_sms;
+    const double halo = ens->crowded ? kCrowdHalo : kUnitHalo;
     double best = 0.0, tau = 0.0, top = 0.0;
-    for (const auto& sz : sizes) top = std::max(top, (1.0 + kStripEdge) * (3.0 * sz.first + kUnitHalo * tab.rmax));
+    for (auto& sz : sizes) {
+      sz.second.split.halo = halo;
+      top = std::max(top, (1.0 + kStripEdge) * (3.0 * sz.first + halo * tab.rmax));
+    }
     for (int waves = 1; waves <= 4; ++waves) {
       double lo = 0.0, hi = top;
       for (int it = 0; it < 16; ++it) {
@@ -2422,7 +2440,7 @@ int ens_units(swm_ensemble* ens, int seg_rows) {
       for (auto& sz : sizes) {
         std::vector<WorkUnit> u;
         sz.second.split.build_tau(hi, sz.second.split.ens_max(), u);
-        for (const WorkUnit& w : u) cost.insert(cost.end(), sz.second.members, unit_cost(tab, sz.first, w));
+        for (const WorkUnit& w : u) cost.insert(cost.end(), sz.second.members, unit_cost(tab, sz.first, w, halo));
       }
       std::sort(cost.begin(), cost.end(), std::greater<double>());
       const double t = ens_makespan(cost, slots);
@@ -2508,7 +2526,8 @@ int ens_capture(swm_ensemble* ens) {
       e = launch_stage<T>(ens->order, ens->cols, ens->fixbw, nullptr, InstDev<T>{}, I + i * ens->nmem,
                           ens->dunits, ens->nunits, MODE_RK1 + i, ens->boxw, ens->grid, derr, ens->st);
       if (e == cudaSuccess)
-        e = launch_edge32(InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i, ens->st);
+        e = launch_edge32(InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i, ens->crowded,
+                          ens->st);
     }
   }
   cudaError_t ec = cudaStreamEndCapture(ens->st, &g);
@@ -2545,9 +2564,22 @@ int ens_set_width(swm_ensemble* ens, int cols) {
   return SWM_OK;
 }
 
+// The default units of a crowded ensemble of one member size run on persistent
+// CTAs: their costs are alike, so taking turns evens them out, and a CTA sets its
+// pipeline up once (300 members of N=16 d42 311 -> 287 us a step, 100 139 -> 131).
+// Units of several sizes end earlier handed out longest first (nine of N=48, 96,
+// 192 ten times over 325 us, 330 persistent).
+int ens_default_grid(const swm_ensemble* ens) {
+  const int slots = std::max(1, ens->occ) * ens->num_sms;
+  bool one_size = true;
+  for (const swm_ctx* c : ens->mem) one_size = one_size && c->n == ens->max_n;
+  return ens->prec == SWM_FP32_FUSED && ens->crowded && one_size && ens->nunits > slots ? slots : 0;
+}
+constexpr int kAutoGrid = -1;
+
 int ens_rebuild(swm_ensemble* ens, int seg_rows, int grid) {
   if (int rc = ens_units(ens, seg_rows)) return rc;
-  ens->grid = grid;
+  ens->grid = grid == kAutoGrid ? ens_default_grid(ens) : grid;
   const bool f32 = ens->prec == SWM_FP32_FUSED;
   if (int rc = f32 ? ens_tables<float>(ens) : ens_tables<double>(ens)) return rc;
   return f32 ? ens_capture<float>(ens) : ens_capture<double>(ens);
@@ -2620,9 +2652,9 @@ int swm_ensemble_create(const swm_config* base, int nmembers, const int* member_
     return bail(e == cudaErrorMemoryAllocation ? SWM_E_NOMEM : SWM_E_CUDA,
                 std::string("ensemble alloc: ") + cudaGetErrorString(e));
   ens_box(ens);
-  // default tile shape: units of equal modelled cost, one CTA each;
-  // swm_ensemble_tune measures the others
-  if (int rc = ens_rebuild(ens, kAutoRows, 0)) return bail(rc, ens->err);
+  // default tile shape: units of equal modelled cost; swm_ensemble_tune
+  // measures the others
+  if (int rc = ens_rebuild(ens, kAutoRows, kAutoGrid)) return bail(rc, ens->err);
   *out = ens;
   return SWM_OK;
 }

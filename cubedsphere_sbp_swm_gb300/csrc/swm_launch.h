@@ -49,8 +49,9 @@ cudaError_t launch_derive64(const InstDev<double>& one, const InstDev<double>* m
                             int max_n, cudaStream_t st);
 cudaError_t launch_stage64(int order, const InstDev<double>& one, const InstDev<double>* many,
                            int ninst, int max_n, const Topology& tp, int mode, cudaStream_t st);
-// FP32 cube-edge kernel over ninst instances whose largest edge has max_n nodes.
+// FP32 cube-edge kernel over ninst instances whose largest edge has max_n nodes
+// (crowded: an ensemble whose stage kernel fills the GPU).
 cudaError_t launch_edge32(const InstDev<float>& one, const InstDev<float>* many, int ninst, int max_n,
-                          const Topology& tp, int mode, cudaStream_t st);
+                          const Topology& tp, int mode, bool crowded, cudaStream_t st);
 
 }  // namespace swm

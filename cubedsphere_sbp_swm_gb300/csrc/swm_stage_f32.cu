@@ -66,14 +66,18 @@ cudaError_t prepare_stage<float>(int order, StageShape* shape) {
 }
 
 cudaError_t launch_edge32(const InstDev<float>& one, const InstDev<float>* many, int ninst,
-                          int max_n, const Topology& tp, int mode, cudaStream_t st) {
+                          int max_n, const Topology& tp, int mode, bool crowded, cudaStream_t st) {
   // One warp a block: a block of 128 threads waits for a free slot on an SM
   // whose registers the stage kernel of another instance holds, and the nodes
   // spread over more SMs.  One instance, RK4 step d42: N=200 57.8 -> 54.6 us,
-  // N=384 86.5 -> 84.5; two instances, N=384 d63: 88.7 -> 83.1.
-  const int nodes = 6 * (4 * max_n - 4);
-  dim3 grid((nodes + 31) / 32, ninst);
-  edge_kernel<float><<<grid, 32, 0, st>>>(one, many, tp, mode);
+  // N=384 86.5 -> 84.5; two instances, N=384 d63: 88.7 -> 83.1.  A crowded
+  // ensemble has blocks for every SM at two warps each, and one-warp blocks would
+  // hold half of an SM's warp slots: 100 members of N=16 145.6 -> 141.6 us a step,
+  // 60 of N=24 110.8 -> 108.8; nine of N=48, 96 and 192, not crowded, 128 at one
+  // warp, 131 at two.
+  const int nodes = 6 * (4 * max_n - 4), threads = crowded ? 64 : 32;
+  dim3 grid((nodes + threads - 1) / threads, ninst);
+  edge_kernel<float><<<grid, threads, 0, st>>>(one, many, tp, mode);
   return cudaGetLastError();
 }
 

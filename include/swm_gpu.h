@@ -423,8 +423,7 @@ int  swm_ensemble_synchronize(swm_ensemble* ens);
 void* swm_ensemble_stream(swm_ensemble* ens);
 /* Tile shape: rows per work unit (0: whole panel height) and persistent CTAs
  * of the stage kernel (0: one CTA per work unit).  A new ensemble has
- * SWM_ENSEMBLE_ROWS_AUTO rows and no persistent CTAs: units of equal modelled
- * cost over all members.  What get_shape and tune return can be given back to
+ * SWM_ENSEMBLE_ROWS_AUTO rows: units of equal modelled cost over all members.  What get_shape and tune return can be given back to
  * set_shape. */
 #define SWM_ENSEMBLE_ROWS_AUTO 2147483647
 int  swm_ensemble_set_shape(swm_ensemble* ens, int seg_rows, int grid);

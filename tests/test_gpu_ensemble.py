@@ -199,3 +199,27 @@ def test_default_split_matches_single_instance(prec, sizes):
     for m, N in enumerate(sizes):
         for a, b in zip(ens.download(m), want[N]):
             assert np.array_equal(a, b), f"member {m} (N={N}) differs"
+
+
+# the default split of the wider closures (units of three rows can lie inside
+# them), of a crowded ensemble of one size, which has persistent CTAs where its
+# units are more than fit, and of a crowded mix
+@pytest.mark.parametrize("prec,order", [("fp32", 43), ("fp32", 63), ("fp64", 63)])
+@pytest.mark.parametrize("sizes", [(16, 97, 33), (16,) * 130, (20, 40) * 60])
+def test_default_split_of_other_orders_and_crowds(prec, order, sizes):
+    start = {N: initial.balanced_zonal(N, 7 + N, 4)[:3] for N in set(sizes)}
+    want = {}
+    for N, st in start.items():
+        op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=order, precision=prec))
+        s = op.create_stvec()
+        s.upload(*st)
+        swm.RK4().step(s, op, _dt(N), 2)
+        want[N] = s.download()
+    ens = swm.Ensemble(swm.ModelConfig(N=sizes[0], sbp_order=order, precision=prec), sizes, [_dt(N) for N in sizes])
+    for m, N in enumerate(sizes):
+        ens.upload(m, *start[N])
+    ens.step(2)
+    ens.synchronize()
+    for m, N in enumerate(sizes):
+        for a, b in zip(ens.download(m), want[N]):
+            assert np.array_equal(a, b), f"member {m} (N={N}) differs"
