@@ -555,8 +555,9 @@ int run_stage(swm_ctx* ctx, const InstDev<T>& I, int mode, bool derive = true) {
     CK(cudaEventRecord(a, ctx->st), "event record");
   }
   if constexpr (sizeof(T) == 8) {
-    if (derive) CK(launch_derive64(I, nullptr, 1, ctx->n, ctx->st), "stencil inputs");
-    CK(launch_stage64(ctx->order, I, nullptr, 1, ctx->n, ctx->topo, mode, ctx->st), "stage kernel");
+    const PointBatch<T> b{nullptr, 1, ctx->n, nullptr, 0};
+    if (derive) CK(launch_derive64(I, b, ctx->st), "stencil inputs");
+    CK(launch_stage64(ctx->order, I, b, ctx->topo, mode, ctx->st), "stage kernel");
   } else {
     CK(launch_stage<T>(ctx->order, ctx->shape.cols, ctx->shape.fixbw != 0, &maps, I, nullptr, ctx->units,
                        ctx->nunits, mode, ctx->shape.boxw, ctx->stage_grid, ctx->derr, ctx->st),
@@ -2327,8 +2328,9 @@ struct swm_ensemble {
   bool fixbw = false;   // every member uses its width's widest (compile-time) box
   StageMaps* dmaps = nullptr;        // [4 stages][nmem]
   void* dinst = nullptr;             // InstDev<T> [4 stages][nmem]
-  WorkUnit* dunits = nullptr;
-  int nunits = 0, cap_units = 0;
+  WorkUnit* dunits = nullptr;        // FP32
+  int2* dblocks = nullptr;           // FP64: (member, block) of each thread block, or null (grid rows)
+  int nunits = 0, cap_units = 0;     // work units (FP64: thread blocks)
   int seg_rows = 0;                  // rows per work unit (0: whole panel height, kAutoRows: modelled)
   int grid = 0;                      // persistent CTAs (0: one CTA per unit)
   bool crowded = false;              // whole-panel units take half of the CTA slots or more
@@ -2398,7 +2400,36 @@ double ens_makespan(const std::vector<double>& cost, int slots) {
   return end;
 }
 
+// The FP64 stage has no work units.  Grid rows as long as the largest member
+// needs leave most blocks empty where sizes differ much, and an empty block still
+// costs its launch: one member of N=384 with 60 of N=16 (d42) took 1623 us a step
+// so, 475 with a table of the blocks; 32 each of N=48, 96 and 192 3864 and 3650.
+// Members that fill half of the rows' blocks or more keep the rows and save the
+// look-up (64 of N=48 518 us, 524 with a table; two of N=24 49.4 and 51.4).
+int ens_blocks(swm_ensemble* ens) {
+  long long total = 0, largest = 0;
+  for (const swm_ctx* c : ens->mem) {
+    const int b = stage64_blocks(ens->order, c->n);
+    total += b;
+    largest = std::max<long long>(largest, b);
+  }
+  if (total > 0x7fffffffLL) return efail(ens, SWM_E_INVALID, "ensemble too large");
+  ens->nunits = (int)total;
+  if (ens->dblocks || 2 * total >= largest * ens->nmem) return SWM_OK;
+  std::vector<int2> all;
+  all.reserve(total);
+  for (int m = 0; m < ens->nmem; ++m)
+    for (int b = 0, nb = stage64_blocks(ens->order, ens->mem[m]->n); b < nb; ++b) all.push_back(make_int2(m, b));
+  ECK(cudaMalloc(&ens->dblocks, sizeof(int2) * all.size()), "alloc blocks");
+  ECK(upload_on(ens->st, ens->dblocks, all.data(), sizeof(int2) * all.size()), "copy blocks");
+  return SWM_OK;
+}
+
 int ens_units(swm_ensemble* ens, int seg_rows) {
+  if (ens->prec != SWM_FP32_FUSED) {
+    ens->seg_rows = seg_rows;
+    return ens_blocks(ens);
+  }
   std::string why;
   const SbpC& tab = kTables[sbp_index(ens->order)];
   struct Size {
@@ -2518,10 +2549,9 @@ int ens_capture(swm_ensemble* ens) {
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
     if constexpr (sizeof(T) == 8) {
-      if (i == 0) e = launch_derive64(InstDev<T>{}, I, ens->nmem, ens->max_n, ens->st);
-      if (e == cudaSuccess)
-        e = launch_stage64(ens->order, InstDev<T>{}, I + i * ens->nmem, ens->nmem, ens->max_n, tp, MODE_RK1 + i,
-                           ens->st);
+      const PointBatch<T> b{I + i * ens->nmem, ens->nmem, ens->max_n, ens->dblocks, ens->nunits};
+      if (i == 0) e = launch_derive64(InstDev<T>{}, b, ens->st);
+      if (e == cudaSuccess) e = launch_stage64(ens->order, InstDev<T>{}, b, tp, MODE_RK1 + i, ens->st);
     } else {
       e = launch_stage<T>(ens->order, ens->cols, ens->fixbw, nullptr, InstDev<T>{}, I + i * ens->nmem,
                           ens->dunits, ens->nunits, MODE_RK1 + i, ens->boxw, ens->grid, derr, ens->st);
@@ -2601,6 +2631,7 @@ void free_ensemble(swm_ensemble* ens) {
   if (ens->dmaps) cudaFree(ens->dmaps);
   if (ens->dinst) cudaFree(ens->dinst);
   if (ens->dunits) cudaFree(ens->dunits);
+  if (ens->dblocks) cudaFree(ens->dblocks);
   for (size_t m = 0; m < ens->mem.size(); ++m) {
     if (m < ens->state.size() && ens->state[m]) swm_state_free(ens->state[m]);
     swm_ctx_destroy(ens->mem[m]);

@@ -201,6 +201,19 @@ struct WorkUnit {
   int16_t cl0, cl1, rl0, rl1;  // columns / rows the unit reads
 };
 
+template <class T>
+struct InstDev;
+// The instances of an FP64 stage launch: one (many null), or `many` of them with
+// the largest edge of max_n nodes, as grid rows or through a table of (instance,
+// block of the instance).
+template <class T>
+struct PointBatch {
+  const InstDev<T>* many;
+  int ninst, max_n;
+  const int2* blocks;
+  int nblocks;
+};
+
 // Per-instance pointers and constants of one fused stage launch.
 // (the FP64 stage's part, which FP32 kernels do not carry as a parameter)
 template <class T>

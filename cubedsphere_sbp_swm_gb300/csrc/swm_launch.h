@@ -44,11 +44,12 @@ template <int CONS>
 cudaError_t stage_f32_prepare(int order);
 // FP64 stage: the stencil inputs of I.in into I.der, and the stage kernel that
 // reads them (and, where I.der_out is set, leaves those of the next stage
-// state), over ninst instances whose largest edge has max_n nodes.
-cudaError_t launch_derive64(const InstDev<double>& one, const InstDev<double>* many, int ninst,
-                            int max_n, cudaStream_t st);
-cudaError_t launch_stage64(int order, const InstDev<double>& one, const InstDev<double>* many,
-                           int ninst, int max_n, const Topology& tp, int mode, cudaStream_t st);
+// state), over the instances of a batch.  stage64_blocks: the thread blocks of an
+// instance of n nodes a panel edge.
+cudaError_t launch_derive64(const InstDev<double>& one, const PointBatch<double>& b, cudaStream_t st);
+cudaError_t launch_stage64(int order, const InstDev<double>& one, const PointBatch<double>& b, const Topology& tp,
+                           int mode, cudaStream_t st);
+int stage64_blocks(int order, int n);
 // FP32 cube-edge kernel over ninst instances whose largest edge has max_n nodes
 // (crowded: an ensemble whose stage kernel fills the GPU).
 cudaError_t launch_edge32(const InstDev<float>& one, const InstDev<float>* many, int ninst, int max_n,

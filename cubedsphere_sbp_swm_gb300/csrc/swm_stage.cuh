@@ -210,11 +210,23 @@ __device__ __forceinline__ void derive_store(T* der, long long fs, long long idx
   der[DR_JVT * fs + idx] = jvt;
 }
 
+// Instance of this block and its first thread: a batch has a grid row per
+// instance, each as long as the largest needs, or, where that leaves most blocks
+// without a node, a table of (instance, block).
+template <class T>
+__device__ __forceinline__ const InstDev<T>& point_inst(const InstDev<T>& one, const InstDev<T>* many,
+                                                        const int2* blocks, int& tid) {
+  const int2 b = blocks ? blocks[blockIdx.x] : make_int2(blockIdx.y, blockIdx.x);
+  tid = b.y * PT_TPB + threadIdx.x;
+  return many ? many[b.x] : one;
+}
+
 template <class T>
 __global__ void __launch_bounds__(PT_TPB)
-    point_derive_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many) {
-  const InstDev<T>& I = many ? many[blockIdx.y] : one;
-  const int t = blockIdx.x * PT_TPB + threadIdx.x, row = t / I.n;
+    point_derive_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many, const int2* blocks) {
+  int t;
+  const InstDev<T>& I = point_inst<T>(one, many, blocks, t);
+  const int row = t / I.n;
   if (row >= 6 * I.n) return;
   const long long fs = I.fs, x = (long long)row * I.P + (t - row * I.n);
   derive_store<T>(const_cast<T*>(I.der), fs, x, I.in[x], I.in[fs + x], I.in[2 * fs + x],
@@ -373,12 +385,13 @@ __device__ __forceinline__ bool point_at(int n, int tid, PointAt& o) {
 template <class T, int ORD, int MODE>
 __global__ void __launch_bounds__(PT_TPB, 5)
     point_stage_kernel(const __grid_constant__ InstDev<T> one, const InstDev<T>* many,
-                       const __grid_constant__ Topology tp) {
+                       const __grid_constant__ Topology tp, const int2* blocks) {
   constexpr int NE = Ord<ORD>::NE;
   constexpr bool needB = MODE == MODE_RK1 || MODE == MODE_RK2 || MODE == MODE_RK3;
   constexpr bool needA = MODE == MODE_RK2 || MODE == MODE_RK3 || MODE == MODE_RK4;
-  const InstDev<T>& I = many ? many[blockIdx.y] : one;
-  const int n = I.n, P = I.P, tid = blockIdx.x * PT_TPB + threadIdx.x;
+  int tid;
+  const InstDev<T>& I = point_inst<T>(one, many, blocks, tid);
+  const int n = I.n, P = I.P;
   PointAt at;
   if (!point_at<ORD>(n, tid, at)) return;
   const int p = at.p, i = at.i, j = at.j;
@@ -477,23 +490,24 @@ __global__ void __launch_bounds__(PT_TPB, 5)
 }
 
 // Stencil inputs of I.in, then (launch_point_stage) one stage from them, over
-// ninst instances whose largest edge has max_n nodes.
+// the instances of B.
 template <class T>
-cudaError_t launch_point_derive(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,
-                                cudaStream_t st) {
-  point_derive_kernel<T><<<dim3((6 * max_n * max_n + PT_TPB - 1) / PT_TPB, ninst), PT_TPB, 0, st>>>(one, many);
+cudaError_t launch_point_derive(const InstDev<T>& one, const PointBatch<T>& B, cudaStream_t st) {
+  // with a table: the stage's blocks, which hold at least as many threads
+  const dim3 g = B.blocks ? dim3(B.nblocks) : dim3((6 * B.max_n * B.max_n + PT_TPB - 1) / PT_TPB, B.ninst);
+  point_derive_kernel<T><<<g, PT_TPB, 0, st>>>(one, B.many, B.blocks);
   return cudaGetLastError();
 }
 template <class T, int ORD>
-cudaError_t launch_point_stage_ord(const InstDev<T>& one, const InstDev<T>* many, int ninst, int max_n,
-                                   const Topology& tp, int mode, cudaStream_t st) {
-  const dim3 g(point_ranges<ORD>(max_n).total / PT_TPB, ninst);
+cudaError_t launch_point_stage_ord(const InstDev<T>& one, const PointBatch<T>& B, const Topology& tp, int mode,
+                                   cudaStream_t st) {
+  const dim3 g = B.blocks ? dim3(B.nblocks) : dim3(point_ranges<ORD>(B.max_n).total / PT_TPB, B.ninst);
   switch (mode) {
-    case MODE_APPLY: point_stage_kernel<T, ORD, MODE_APPLY><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
-    case MODE_RK1: point_stage_kernel<T, ORD, MODE_RK1><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
-    case MODE_RK2: point_stage_kernel<T, ORD, MODE_RK2><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
-    case MODE_RK3: point_stage_kernel<T, ORD, MODE_RK3><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
-    case MODE_RK4: point_stage_kernel<T, ORD, MODE_RK4><<<g, PT_TPB, 0, st>>>(one, many, tp); break;
+    case MODE_APPLY: point_stage_kernel<T, ORD, MODE_APPLY><<<g, PT_TPB, 0, st>>>(one, B.many, tp, B.blocks); break;
+    case MODE_RK1: point_stage_kernel<T, ORD, MODE_RK1><<<g, PT_TPB, 0, st>>>(one, B.many, tp, B.blocks); break;
+    case MODE_RK2: point_stage_kernel<T, ORD, MODE_RK2><<<g, PT_TPB, 0, st>>>(one, B.many, tp, B.blocks); break;
+    case MODE_RK3: point_stage_kernel<T, ORD, MODE_RK3><<<g, PT_TPB, 0, st>>>(one, B.many, tp, B.blocks); break;
+    case MODE_RK4: point_stage_kernel<T, ORD, MODE_RK4><<<g, PT_TPB, 0, st>>>(one, B.many, tp, B.blocks); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

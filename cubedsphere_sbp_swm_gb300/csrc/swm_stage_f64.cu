@@ -7,20 +7,24 @@ namespace swm {
 // The FP64 stage has no work units; its contexts report one width.
 constexpr int kReportedWidth = 64;
 
-cudaError_t launch_derive64(const InstDev<double>& one, const InstDev<double>* many, int ninst,
-                            int max_n, cudaStream_t st) {
-  return launch_point_derive<double>(one, many, ninst, max_n, st);
+cudaError_t launch_derive64(const InstDev<double>& one, const PointBatch<double>& b, cudaStream_t st) {
+  return launch_point_derive<double>(one, b, st);
 }
 
-cudaError_t launch_stage64(int order, const InstDev<double>& one, const InstDev<double>* many,
-                           int ninst, int max_n, const Topology& tp, int mode, cudaStream_t st) {
+cudaError_t launch_stage64(int order, const InstDev<double>& one, const PointBatch<double>& b, const Topology& tp,
+                           int mode, cudaStream_t st) {
   switch (order) {
-    case 21: return launch_point_stage_ord<double, 21>(one, many, ninst, max_n, tp, mode, st);
-    case 42: return launch_point_stage_ord<double, 42>(one, many, ninst, max_n, tp, mode, st);
-    case 43: return launch_point_stage_ord<double, 43>(one, many, ninst, max_n, tp, mode, st);
-    case 63: return launch_point_stage_ord<double, 63>(one, many, ninst, max_n, tp, mode, st);
+    case 21: return launch_point_stage_ord<double, 21>(one, b, tp, mode, st);
+    case 42: return launch_point_stage_ord<double, 42>(one, b, tp, mode, st);
+    case 43: return launch_point_stage_ord<double, 43>(one, b, tp, mode, st);
+    case 63: return launch_point_stage_ord<double, 63>(one, b, tp, mode, st);
     default: return cudaErrorInvalidValue;
   }
+}
+
+int stage64_blocks(int order, int n) {
+  return (order == 21 ? point_ranges<21>(n) : order == 42 ? point_ranges<42>(n) : order == 43 ? point_ranges<43>(n)
+                                                                               : point_ranges<63>(n)).total / PT_TPB;
 }
 
 template <>

@@ -424,7 +424,8 @@ void* swm_ensemble_stream(swm_ensemble* ens);
 /* Tile shape: rows per work unit (0: whole panel height) and persistent CTAs
  * of the stage kernel (0: one CTA per work unit).  A new ensemble has
  * SWM_ENSEMBLE_ROWS_AUTO rows: units of equal modelled cost over all members.  What get_shape and tune return can be given back to
- * set_shape. */
+ * set_shape.  An FP64 ensemble keeps what is set, but its stage kernel has no work
+ * units: nunits is its thread blocks then. */
 #define SWM_ENSEMBLE_ROWS_AUTO 2147483647
 int  swm_ensemble_set_shape(swm_ensemble* ens, int seg_rows, int grid);
 /* Consumer width of the members' FP32 stage kernel (64, 96, 128, 160 or 192;

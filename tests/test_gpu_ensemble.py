@@ -203,9 +203,10 @@ def test_default_split_matches_single_instance(prec, sizes):
 
 # the default split of the wider closures (units of three rows can lie inside
 # them), of a crowded ensemble of one size, which has persistent CTAs where its
-# units are more than fit, and of a crowded mix
+# units are more than fit, of a crowded mix, and of one large member among small
+# ones, where the FP64 stage takes its blocks from a table
 @pytest.mark.parametrize("prec,order", [("fp32", 43), ("fp32", 63), ("fp64", 63)])
-@pytest.mark.parametrize("sizes", [(16, 97, 33), (16,) * 130, (20, 40) * 60])
+@pytest.mark.parametrize("sizes", [(16, 97, 33), (16,) * 130, (20, 40) * 60, (97,) + (16,) * 9])
 def test_default_split_of_other_orders_and_crowds(prec, order, sizes):
     start = {N: initial.balanced_zonal(N, 7 + N, 4)[:3] for N in set(sizes)}
     want = {}
