@@ -132,6 +132,7 @@ struct swm_latlon {
   double *wx, *wy, *rot;
   double* out;
   float* out32;
+  double* hout;   // page-locked, for small results (latlon_fetch); null where none are small
   float* hout32;
 };
 
@@ -865,8 +866,9 @@ int op_grad(swm_ctx* ctx, const double* f, double* gx, double* gy) {
 void release_latlon(swm_latlon* r) {
   void* dev[] = {r->base, r->wx, r->wy, r->rot, r->out, r->out32};
   for (void* p : dev) if (p) cudaFree(p);
+  if (r->hout) cudaFreeHost(r->hout);
   if (r->hout32) cudaFreeHost(r->hout32);
-  r->base = nullptr; r->wx = r->wy = r->rot = r->out = nullptr;
+  r->base = nullptr; r->wx = r->wy = r->rot = r->out = r->hout = nullptr;
   r->out32 = r->hout32 = nullptr;
 }
 
@@ -3345,16 +3347,29 @@ int latlon_state(swm_ctx* ctx, swm_latlon* r, const swm_state* s, int c0, int nf
   return SWM_OK;
 }
 
-// The output planes to the caller's arrays (null: not wanted), by the copy
-// engine straight into them: through a page-locked buffer and a host copy the
-// three planes of a 4N x (2N+1) grid took 0.32 ms at N=130 and 1.07 ms at N=250;
-// now 0.12 and 0.27 ms.
+// The output planes to the caller's arrays (null: not wanted).  Planes above
+// kLatlonStaged go by the copy engine straight into them: through a page-locked
+// buffer and a host copy the three planes of a 4N x (2N+1) grid took 0.29 ms at
+// N=130, 0.11 so.  A copy to pageable memory has some 5 us of its own, though, and
+// one copy of all planes and a host copy are quicker up to 128 KB a plane (three
+// planes, cubic): 36 KB 38 us for 57, 101 KB 51 for 58, 145 KB 59 for 59, 197 KB 71 for 62.
+constexpr size_t kLatlonStaged = 128 << 10;
+
 int latlon_fetch(swm_ctx* ctx, const swm_latlon* r, int nf, double* const dst[]) {
-  const size_t np = (size_t)r->nlon * r->nlat;
-  for (int c = 0; c < nf; ++c)
-    if (dst[c])
-      CK(cudaMemcpyAsync(dst[c], r->out + c * np, sizeof(double) * np, cudaMemcpyDeviceToHost, ctx->st), "copy");
-  return sync_check(ctx, ctx->st);
+  const size_t np = (size_t)r->nlon * r->nlat, bytes = sizeof(double) * np;
+  if (bytes <= kLatlonStaged) {
+    CK(cudaMemcpyAsync(r->hout, r->out, nf * bytes, cudaMemcpyDeviceToHost, ctx->st), "copy");
+    if (int rc = sync_check(ctx, ctx->st)) return rc;
+    for (int c = 0; c < nf; ++c)
+      if (dst[c]) std::memcpy(dst[c], r->hout + c * np, bytes);
+    return SWM_OK;
+  }
+  cudaError_t e = cudaSuccess;
+  for (int c = 0; c < nf && e == cudaSuccess; ++c)
+    if (dst[c]) e = cudaMemcpyAsync(dst[c], r->out + c * np, bytes, cudaMemcpyDeviceToHost, ctx->st);
+  const int rc = sync_check(ctx, ctx->st);   // also after a failure: no copy outlives the call
+  CK(e, "copy");
+  return rc;
 }
 
 // Write `count` FP32 values as record rec_num (1-based) of a direct-access
@@ -3398,7 +3413,7 @@ int swm_latlon_create(swm_ctx* ctx, int nlon, int nlat, const char* interp_type,
     return fail(ctx, SWM_E_INVALID, "lat-lon set-up failed");
   USE_DEVICE(ctx);
   swm_latlon* r = new swm_latlon{ctx, nlon, nlat, w, contra, nullptr, nullptr, nullptr, nullptr,
-                                 nullptr, nullptr, nullptr};
+                                 nullptr, nullptr, nullptr, nullptr};
   const size_t np = (size_t)nlon * nlat;
   cudaError_t e = cudaMalloc(&r->base, sizeof(long long) * np);
   if (e == cudaSuccess) e = cudaMalloc(&r->wx, sizeof(double) * 4 * np);
@@ -3406,6 +3421,7 @@ int swm_latlon_create(swm_ctx* ctx, int nlon, int nlat, const char* interp_type,
   if (e == cudaSuccess) e = cudaMalloc(&r->rot, sizeof(double) * 4 * np);
   if (e == cudaSuccess) e = cudaMalloc(&r->out, sizeof(double) * 3 * np);
   if (e == cudaSuccess) e = cudaMalloc(&r->out32, sizeof(float) * 2 * np);
+  if (e == cudaSuccess && sizeof(double) * np <= kLatlonStaged) e = cudaMallocHost(&r->hout, sizeof(double) * 3 * np);
   if (e == cudaSuccess) e = cudaMallocHost(&r->hout32, sizeof(float) * 2 * np);
   if (e == cudaSuccess) e = upload_on(ctx->st, r->base, h.base.data(), sizeof(long long) * np);
   if (e == cudaSuccess) e = upload_on(ctx->st, r->wx, h.wx.data(), sizeof(double) * 4 * np);

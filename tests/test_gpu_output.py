@@ -79,6 +79,31 @@ def test_state_regrid_matches_oracle(interp, width):
     assert np.abs(vg - vo).max() <= 1e-13 * np.abs(uo).max()
 
 
+# Planes of up to 16384 values come back through one page-locked buffer, larger
+# ones straight into the caller's arrays; which components are wanted decides
+# where the planes lie.
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nlon,nlat", [(32, 17), (128, 128), (128, 129)])
+def test_state_regrid_of_some_components(prec, nlon, nlat):
+    op = swm.OperatorSWM(swm.ModelConfig(N=24, precision=prec))
+    s = op.create_stvec()
+    s.upload(*initial.balanced_zonal(24, 2, 6)[:3])
+    rg = swm.LatLonRegrid(op, nlon, nlat)
+    want = rg.regrid_state(s)
+    for wanted in range(8):
+        out = [np.full((nlat, nlon), -1.0) if wanted >> c & 1 else None for c in range(3)]
+        ptr = [None if a is None else a.ctypes.data_as(_abi._D) for a in out]
+        op._check(op._L.swm_latlon_regrid_state(op._h, rg._h, s._h, *ptr))
+        for a, b in zip(out, want):
+            assert a is None or np.array_equal(a, b)
+    if prec == "fp64":   # the single operators, on FP64 fields
+        h, u, v = (op.create_field() for _ in range(3))
+        for f, a in zip((h, u, v), s.download()):
+            f.upload(a)
+        for a, b in zip((rg.do_regrid(h), *rg.do_regrid_vec(u, v)), want):
+            assert np.array_equal(a, b)
+
+
 def test_fp32_state_regrid_uses_the_pair():
     N = 48
     res = {}
