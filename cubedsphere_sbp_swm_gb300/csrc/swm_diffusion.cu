@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(LTPB, 4) lap_tile_kernel(FieldGeom g, int nty,
 // Pass 1: d1x = c D1x(f)*J*Qi12, d1y = c D1y(f)*J*Qi12 of NF fields
 // (laplace_Ah_sbp42_narrow_mod.f90:60-93), c the leading interior coefficient
 // of D1, which pass 2 leaves out of its own derivatives.
-template <int NARROW, int NF>
+template <int NARROW, int NF, int E>
 __global__ void __launch_bounds__(PT_TPB) lap_d1_kernel(FieldGeom g, const double* __restrict__ f,
                                                         const double* __restrict__ mt, double* d1x,
                                                         double* d1y) {
@@ -588,8 +588,11 @@ __global__ void __launch_bounds__(PT_TPB) lap_d1_kernel(FieldGeom g, const doubl
   constexpr T c1 = d_coef<NARROW>(1);
   int p, i, j;
   const int n = g.n, P = g.P;
-  if (!point_node<NE>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
-  const long long x = (long long)p * g.ps + (long long)j * P + i;
+  if (!point_node<E>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
+  const long long x = (long long)p * g.ps + (long long)j * P + i, group = blockIdx.y * NF * g.fs;
+  f += group;
+  d1x += group;
+  d1y += group;
   const T jq = (mt[MJ * g.fs + x] * mt[MQI2 * g.fs + x]) * c1;
   const bool xin = i >= NE && i < n - NE, yin = j >= NE && j < n - NE;
   const T jx = xin ? jq * c1 : jq, jy = yin ? jq * c1 : jq;
@@ -607,18 +610,23 @@ __global__ void __launch_bounds__(PT_TPB) lap_d1_kernel(FieldGeom g, const doubl
 
 // Pass 2: the pre-sync Laplacian of NF fields (laplace_Ah_sbp42_narrow_mod.f90
 // :94-763 with the division by J of lines 52-53).
-template <int NARROW, int NF>
+template <int NARROW, int NF, int E>
 __global__ void __launch_bounds__(PT_TPB) lap_main_kernel(
     FieldGeom g, const double* __restrict__ f, const double* __restrict__ d1x,
     const double* __restrict__ d1y, const double* __restrict__ cx, const double* __restrict__ cy,
     const double* __restrict__ clx, const double* __restrict__ cly, const double* __restrict__ mt,
-    double* out, double* E) {
+    double* out, double* edge) {
   using T = double;
   using S = NarrowShape<NARROW>;
   int p, i, j;
   const int n = g.n, P = g.P;
-  if (!point_node<S::rows>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
+  if (!point_node<E>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
   const long long fs = g.fs, x = (long long)p * g.ps + (long long)j * P + i;
+  const int first = blockIdx.y * NF;   // field of this thread's first
+  f += first * fs;
+  d1x += first * fs;
+  d1y += first * fs;
+  out += first * fs;
   const T rJ = mt[MRJ * fs + x];
   const T inv = rJ * (rJ * mt[MJ * fs + x]);   // 1 / ((hx a)^2 J)
   const bool clxn = i < S::rows || i >= n - S::rows, clyn = j < S::rows || j >= n - S::rows;
@@ -697,7 +705,7 @@ __global__ void __launch_bounds__(PT_TPB) lap_main_kernel(
     v = v * inv;
     out[c * fs + x] = v;
     // panel-boundary values also go to value slot c of the edge buffer
-    auto put = [&](int side, int q) { E[((long long)(p * 4 + side) * 4 + c) * n + q] = v; };
+    auto put = [&](int side, int q) { edge[((long long)(p * 4 + side) * 4 + first + c) * n + q] = v; };
     if (i == 0) put(SIDE_L, j);
     if (i == n - 1) put(SIDE_R, j);
     if (j == 0) put(SIDE_B, i);
@@ -864,6 +872,16 @@ long long narrow_closure_count(int narrow, int n) {
   return 6LL * n * 2 * narrow_rows(narrow) * narrow_cols(narrow);
 }
 
+// The two passes of the FP64 Laplacian, NF fields a thread and a group of NF
+// fields a grid row; ROWS: warps along the row on every column.
+template <int NARROW, int NF, bool ROWS>
+void lap_launch(dim3 grid, const FieldGeom& g, const NarrowTables<double>& t, const double* f, const double* mt,
+                double* d1x, double* d1y, double* out, double* edge, cudaStream_t st) {
+  constexpr int E1 = ROWS ? 0 : Ord<NARROW>::NE, E2 = ROWS ? 0 : NarrowShape<NARROW>::rows;
+  lap_d1_kernel<NARROW, NF, E1><<<grid, PT_TPB, 0, st>>>(g, f, mt, d1x, d1y);
+  lap_main_kernel<NARROW, NF, E2><<<grid, PT_TPB, 0, st>>>(g, f, d1x, d1y, t.cx, t.cy, t.clx, t.cly, mt, out, edge);
+}
+
 template <class T, int NARROW, int NF>
 cudaError_t laplace_nf(const FieldGeom& g, const Topology& tp, const NarrowTables<T>& t, const T* f,
                        const T* mt, double hs, T* d1x, T* d1y, T* out, T* edge, const T* edge_in,
@@ -886,10 +904,23 @@ cudaError_t laplace_nf(const FieldGeom& g, const Topology& tp, const NarrowTable
   } else {
     if (edge_in) return cudaErrorInvalidValue;   // FP64 inputs are synced by their own launch
     if (!d1x || !d1y) return cudaErrorInvalidValue;
+    // A small panel does not fill the GPU, and a node's four fields one after the
+    // other are the launch's latency: up to eight blocks an SM (N=169) the fields are
+    // grid rows.  On the smallest, warps along the row are quicker still: a warp
+    // that meets closure and interior runs both, but its loads are coalesced, and
+    // the closure columns' are not.  Diffusion tendency 6/3 (4/2), us: N=48 135 ->
+    // 85 (116 -> 77) split, 85 (73) with row warps too; N=64 139 -> 97 (115 -> 82), 102
+    // (86); N=128 173 -> 152 (140 -> 120); N=192 250 and 239 (189 and 184; 2/1 128
+    // and 131).  One field 6/3: N=64 28.5 -> 25.6 with row warps, N=72 29.1 -> 25.7, N=80
+    // 29.9 and 30.6.  (The table-driven kernels before these had 132 and 129 at N=48
+    // and 64, and 25.7 for one field.)
     const int blocks = (6 * g.n * g.n + PT_TPB - 1) / PT_TPB;
-    lap_d1_kernel<NARROW, NF><<<blocks, PT_TPB, 0, st>>>(g, f, mt, d1x, d1y);
-    lap_main_kernel<NARROW, NF><<<blocks, PT_TPB, 0, st>>>(g, f, d1x, d1y, t.cx, t.cy, t.clx, t.cly, mt,
-                                                           out, edge);
+    if (blocks <= (NF == 1 ? 256 : 128))
+      lap_launch<NARROW, 1, true>(dim3(blocks, NF), g, t, f, mt, d1x, d1y, out, edge, st);
+    else if (blocks <= 8 * 152)
+      lap_launch<NARROW, 1, false>(dim3(blocks, NF), g, t, f, mt, d1x, d1y, out, edge, st);
+    else
+      lap_launch<NARROW, NF, false>(dim3(blocks), g, t, f, mt, d1x, d1y, out, edge, st);
   }
   return cudaGetLastError();
 }

@@ -78,6 +78,35 @@ def test_diffusion_operator_matches_oracle(uv_narrow, h_narrow):
         assert rel_l2(a, b, J) <= 1e-12
 
 
+# The FP64 kernels take the fields of a small panel apart, with warps along the
+# row on the smallest: panels at either side of the two limits, four fields (three
+# and one where the orders differ) and one.
+@pytest.mark.parametrize("N,uv_narrow,h_narrow", [(51, 42, 42), (52, 63, 63), (52, 63, 42), (51, 21, 42),
+                                                  (160, 42, 42), (161, 42, 63), (161, 21, 21)])
+def test_diffusion_operator_at_the_split_limits(N, uv_narrow, h_narrow):
+    op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=42, precision="fp64"))
+    dop = swm.OperatorSWMDiff(op, UV[uv_narrow], 0.03, H[h_narrow], 0.01)
+    od = oracle.OracleDomain(N, 42)
+    J = od.geometry()["J"]
+    h, u, v = _state(N)
+    x, t = op.create_stvec(), op.create_stvec()
+    x.upload(h, u, v)
+    dop.apply(t, x)
+    for a, b in zip(t.download(), od.diffusion_apply(h, u, v, 0.03, 0.01, uv_narrow, h_narrow)):
+        assert rel_l2(a, b, J) <= 1e-12
+
+
+@pytest.mark.parametrize("N,narrow", [(72, 63), (73, 63), (72, 21), (73, 42)])
+def test_laplace_at_the_row_warp_limit(N, narrow):
+    op = swm.OperatorSWM(swm.ModelConfig(N=N, sbp_order=42, precision="fp64"))
+    od = oracle.OracleDomain(N, 42)
+    f = _state(N)[0]
+    fi, fo = op.create_field(), op.create_field()
+    fi.upload(f)
+    op.laplace(fo, fi, narrow)
+    assert rel_l2(fo.download(), od.laplace(f, narrow), od.geometry()["J"]) <= 1e-12
+
+
 @pytest.mark.parametrize("order,narrow", [(42, 42), (63, 63), (42, 21)])
 def test_model_step_matches_oracle(order, narrow):
     """The 2/1 hyperdiffusion runs after the 4/2 model operator (the Ah
