@@ -1160,7 +1160,7 @@ RhsArgs<T> rhs_args(const CGrid* c) {
   return a;
 }
 
-// Launch grid of rhs_map and its slabs of column warps.
+// Launch grid of rhs_map and its slabs of side columns.
 dim3 rhs_grid(int N, int& strips) {
   dim3 grid((N - 2 * kRhsEdge + kRhsX) / kRhsX, (N + kRhsY) / kRhsY, 6);
   const int blocks = 6 * ((N + kRhsX) / kRhsX), slab = grid.x * grid.y;

@@ -23,9 +23,9 @@
 //     instead of 9.  FP32, where an instruction more is cheap, keeps the
 //     coefficients and the order of the unfused operators' sums, so that its
 //     results are bit for bit what table-driven passes gave.
-//   - The first and last four columns are run by warps along the column
-//     (rhs_map), so that a warp's closure row along x is uniform and no other
-//     warp branches on x.  Along y a warp is one row, and uniform already.
+//   - The first and last four columns are run by warps of their own (rhs_map), in
+//     FP64 along the column, so that a warp's closure row along x is uniform, and
+//     no other warp branches on x.  Along y a warp is one row, and uniform already.
 //   - The six passes of the operators one by one pair up where one does not
 //     read the other's output: 16 launches an RK4 step.
 // Measured at N=384, 4/2 (RK4 step): FP64 1.058 -> 0.705 ms against six
@@ -73,7 +73,7 @@ ScaledOps<T> scaled_ops(const COps& o, int ord) {
 template <class T>
 struct RhsArgs {
   FieldGeom g;
-  int N, L, strips;   // strips: grid.z slabs of the column warps
+  int N, L, strips;   // strips: grid.z slabs of the side columns
   const int* halo;
   std::conditional_t<sizeof(T) == 8, ScaledOps<T>, COpsT<T>> ops;
   // metric: JQi2p, f, Ju, Jv, Qi1u, Qi3v and 1/J (u, v), 1/(J hx a) (corners),
@@ -98,8 +98,8 @@ constexpr int kRhsBlocks = sizeof(T) == 4 ? 8 : 6;
 
 // Point of this thread in slab z: i for the interface outputs along x (0..N) and ip for
 // the centre outputs (0..N-1, or -1 where a thread has none).  The first grid.z
-// slabs hold the column warps: lanes along j, one of the four columns of
-// either side per warp; the others hold the columns between.
+// slabs hold the warps of the four columns at either side, a block 32 rows of
+// them; the others hold the columns between.
 struct RhsPoint {
   int p, i, ip, j;
   bool strip;
@@ -112,8 +112,16 @@ __device__ __forceinline__ bool rhs_map(const RhsArgs<T>& a, int z, RhsPoint& r)
     const int b = (z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
     r.p = b / nb;
     if (r.p >= 6) return false;
-    r.j = (b - r.p * nb) * kRhsX + threadIdx.x;
-    const int c = threadIdx.y;
+    // FP64: a column a warp.  FP32, which waits on memory, 8 rows of the four
+    // columns of a side: 8 cache lines a load and not 32, at the price of closure
+    // rows that differ between lanes.  RK4 step 4/2, us, against columns: N=16 117 ->
+    // 94, N=48 123 -> 109, N=56 125 -> 107, N=80 127 -> 108, N=384 211 -> 207 (2/1: N=56
+    // 102 -> 94, N=192 107 -> 110); FP64 at N=16 195 -> 141 but the FP64 diffusion at
+    // N=128 77 -> 84.
+    const int w = threadIdx.y, l = threadIdx.x;
+    const bool tile = sizeof(T) == 4;
+    r.j = (b - r.p * nb) * kRhsX + (tile ? (w >> 1) * 8 + (l >> 2) : l);
+    const int c = tile ? (w & 1) * kRhsEdge + (l & 3) : w;
     r.i = c < kRhsEdge ? c : N - 2 * kRhsEdge + 1 + c;
     r.ip = c < kRhsEdge ? c : N - 2 * kRhsEdge + c;
     r.strip = true;
