@@ -252,7 +252,8 @@ __device__ __forceinline__ void lap_region(int a0, int len, int n, int& lo, int&
 // closure rows of `rows` nodes at each end.  The last tile ends on the panel
 // edge.  Where the tile before it would reach the far closure rows too (every
 // n = k len + 1 .. k len + rows, so every N that is a multiple of len), it is
-// moved back next to the last one if that leaves it between the closures: a
+// moved back next to the last one if that leaves it between the closures (never
+// along y at 6/3, whose 9 closure rows are more than a tile's 8): a
 // tile with closure nodes costs about 2.5 tiles without (1890 against 770
 // instructions a warp, 4/2), and at N=384 there are 720 of them instead of
 // 1062 in 3822.  Nodes in two tiles get the same value twice.  With the inner
@@ -261,7 +262,7 @@ __device__ __forceinline__ void lap_region(int a0, int len, int n, int& lo, int&
 __device__ __forceinline__ int lap_tile_start(int t, int count, int len, int n, int rows) {
   const int a = min(t * len, n - min(len, n));
   const int b = n - 2 * len;
-  return t == count - 2 && a + len > n - rows && b >= rows ? b : a;
+  return t == count - 2 && a + len > n - rows && b >= rows && b + len <= n - rows ? b : a;
 }
 
 // Coefficient of tap C of the interior D2 row from the variable coefficients

@@ -101,3 +101,38 @@ def test_regions_fit_and_hold_every_stencil(order):
                     if a0 <= k < a0 + ln:
                         a, z = _needs(order, k, n)
                         assert lo <= a and z < hi, (order, N, L, a0, k, a, z, lo, hi)
+
+
+def _start(order, t, count, L, n):
+    """lap_tile_start: the last tile but one moved off the far closure rows where
+    that leaves it between the closures."""
+    rows = _shape(order)[0]
+    a, b = min(t * L, n - min(L, n)), n - 2 * L
+    return b if t == count - 2 and a + L > n - rows and b >= rows and b + L <= n - rows else a
+
+
+@pytest.mark.parametrize("order", [21, 42, 63])
+def test_moved_tiles_cover_the_line_and_hold_every_stencil(order):
+    rows = _shape(order)[0]
+    R, RX, RY = _sizes(order)
+    moved = 0
+    for N in range(16, 2101):
+        n = N + 1
+        if n < 2 * rows:
+            continue
+        for L, cap in ((LTX, RX), (LTY, RY)):
+            ln, count = min(L, n), (n + L - 1) // L
+            starts = [_start(order, t, count, L, n) for t in range(count)]
+            assert starts[0] == 0 and starts[-1] + ln == n
+            assert all(0 < b - a <= ln for a, b in zip(starts, starts[1:]))   # no gap, in order
+            for t, a0 in enumerate(starts):
+                if a0 == min(t * L, n - ln):
+                    continue   # as in the check above
+                moved += 1
+                assert rows <= a0 and a0 + ln <= n - rows   # an inner tile along this line
+                lo, hi = _region(order, a0, ln, n)
+                assert (lo, hi) == (a0 - R, a0 + ln + R) and hi - lo <= cap
+                for k in (a0, a0 + ln - 1):
+                    a, z = _needs(order, k, n)
+                    assert lo <= a and z < hi
+    assert (moved > 0) == (rows > 1)   # the last tile but one ends on node n - 2 at the latest
