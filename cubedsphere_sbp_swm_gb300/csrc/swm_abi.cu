@@ -254,6 +254,9 @@ long long round_up(long long a, long long b) { return (a + b - 1) / b * b; }
 // make one warp diverge, and the per-row barrier makes the CTA wait for
 // it); a closure row at a panel end costs 1 + row_closure_cost; every unit adds
 // kUnitHalo * rmax rows for its halo.
+// The shape an FP64 context reports: its stage kernel has no tiles.
+constexpr StageShape kFp64Shape{1, 64, 0, 0, 0, 0, 0};
+
 constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
 constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
 constexpr double kCrowdHalo = 3.3;     // the same where an ensemble's whole-panel units fill the GPU
@@ -687,7 +690,7 @@ int stage_layout(swm_ctx* ctx, int cols, int seg_rows = 0, int grid = 0, int box
   StageShape sh = ctx->shape;
   const SbpC& tab = kTables[sbp_index(ctx->order)];
   if (sh.tma) {
-    const int bmax = ctx->prec == SWM_FP32_FUSED ? stage_boxw_max<float>(cols) : stage_boxw_max<double>(cols);
+    const int bmax = stage_boxw_max(cols);
     if (bmax <= 0) return fail(ctx, SWM_E_INVALID, "no stage kernel of that width");
     std::vector<WorkUnit> strips;
     if (!make_units(tab, ctx->n, cols, 1, strips, why)) return fail(ctx, SWM_E_INVALID, why);
@@ -698,12 +701,8 @@ int stage_layout(swm_ctx* ctx, int cols, int seg_rows = 0, int grid = 0, int box
       bw = std::max(bw, (w.cl1 - cal + al - 1) / al * al);
     }
     if (bw > bmax) return fail(ctx, SWM_E_INVALID, "work split exceeds the TMA box");
-    const bool f32 = ctx->prec == SWM_FP32_FUSED;
-    auto occ = [&](int w, bool fixed) {
-      return f32 ? stage_occupancy<float>(ctx->order, w, cols, fixed)
-                 : stage_occupancy<double>(ctx->order, w, cols, fixed);
-    };
-    const bool fits = f32 && bmax <= ctx->P;
+    auto occ = [&](int w, bool fixed) { return stage_occupancy(ctx->order, w, cols, fixed); };
+    const bool fits = bmax <= ctx->P;
     if (box == SWM_BOX_WIDEST && !fits) return fail(ctx, SWM_E_INVALID, "the widest box exceeds the pitch");
     const int occ_strip = occ(bw, false);
     const bool fixed = box == SWM_BOX_WIDEST || (box == SWM_BOX_AUTO && fits && occ(bmax, true) >= occ_strip);
@@ -717,12 +716,14 @@ int stage_layout(swm_ctx* ctx, int cols, int seg_rows = 0, int grid = 0, int box
   if (!make_units(tab, ctx->n, sh.cols, std::max(1, sh.ctas_per_sm) * ctx->num_sms, units, why, nseg))
     return fail(ctx, SWM_E_INVALID, why);
   CK(cudaStreamSynchronize(ctx->st), "sync");
-  WorkUnit* d = nullptr;
-  CK(cudaMalloc(&d, sizeof(WorkUnit) * units.size()), "alloc");
-  cudaError_t e = upload_on(ctx->st, d, units.data(), sizeof(WorkUnit) * units.size());
-  if (e != cudaSuccess) { cudaFree(d); return cuda_fail(ctx, e, "copy units"); }
-  if (ctx->units) cudaFree(ctx->units);
-  ctx->units = d;
+  if (sh.tma) {   // the FP64 stage reads no units; its contexts only report them
+    WorkUnit* d = nullptr;
+    CK(cudaMalloc(&d, sizeof(WorkUnit) * units.size()), "alloc");
+    cudaError_t e = upload_on(ctx->st, d, units.data(), sizeof(WorkUnit) * units.size());
+    if (e != cudaSuccess) { cudaFree(d); return cuda_fail(ctx, e, "copy units"); }
+    if (ctx->units) cudaFree(ctx->units);
+    ctx->units = d;
+  }
   ctx->nunits = (int)units.size();
   ctx->shape = sh;
   ctx->seg_rows = seg_rows;
@@ -1042,7 +1043,7 @@ int swm_ctx_create_named(const swm_config* cfg, const char* div_op_name, const c
   CKC(cudaMalloc(&ctx->qw, sizeof(double) * 4 * ctx->n), "alloc");
   CKC(cudaMalloc(&ctx->Aw, sizeof(double) * ctx->n), "alloc");
   CKC(cudaMalloc(&ctx->edge64, sizeof(double) * 16 * 6 * ctx->n), "alloc");
-  CKC(cudaMalloc(&ctx->edge, (size_t)ctx->elt * 16 * 6 * ctx->n), "alloc");
+  if (ctx->prec == SWM_FP32_FUSED) CKC(cudaMalloc(&ctx->edge, sizeof(float) * 16 * 6 * ctx->n), "alloc");
   CKC(cudaMalloc(&ctx->ya, (size_t)ctx->elt * 3 * ctx->fs), "alloc");
   CKC(cudaMalloc(&ctx->yb, (size_t)ctx->elt * 3 * ctx->fs), "alloc");
   CKC(cudaMalloc(&ctx->acc, (size_t)ctx->elt * 3 * ctx->fs), "alloc");
@@ -1072,9 +1073,8 @@ int swm_ctx_create_named(const swm_config* cfg, const char* div_op_name, const c
     *out = ctx;
     return SWM_OK;
   }
-  CKC(ctx->prec == SWM_FP32_FUSED ? prepare_stage<float>(od, &ctx->shape)
-                                  : prepare_stage<double>(od, &ctx->shape),
-      "stage kernel attributes");
+  if (ctx->prec == SWM_FP32_FUSED) CKC(prepare_stage(od, &ctx->shape), "stage kernel attributes");
+  else ctx->shape = kFp64Shape;
   if (ctx->shape.tma && !encode_tiled()) {
     free_ctx(ctx);
     return fail(nullptr, SWM_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
@@ -2582,8 +2582,7 @@ void ens_box(swm_ensemble* ens) {
   }
   ens->boxw = boxw;
   ens->fixbw = fixed;
-  ens->occ = ens->prec == SWM_FP32_FUSED ? stage_occupancy<float>(ens->order, ens->boxw, ens->cols, fixed)
-                                         : stage_occupancy<double>(ens->order, ens->boxw, ens->cols, fixed);
+  ens->occ = ens->prec == SWM_FP32_FUSED ? stage_occupancy(ens->order, ens->boxw, ens->cols, fixed) : 1;
 }
 
 // Consumer width of the members' FP32 stage kernel: every member's box and
@@ -2911,10 +2910,11 @@ int adjoint_ws(swm_ctx* ctx, bool tl) {
   const size_t b = (size_t)ctx->elt * (size_t)(kAdWork + 3 * kAdStates) * ctx->fs;
   CK(cudaMalloc(&ctx->adw, b), "alloc adjoint work");
   CK(cudaMemsetAsync(ctx->adw, 0, b, ctx->st), "memset");
-  // two edge buffers: transposed-sync pulls, base-curl edge values
-  const size_t eb = (size_t)ctx->elt * 2 * 16 * 6 * ctx->n;
-  CK(cudaMalloc(&ctx->adC, eb), "alloc adjoint edge buffers");
-  CK(cudaMemsetAsync(ctx->adC, 0, eb, ctx->st), "memset");
+  if (ctx->prec == SWM_FP32_FUSED) {   // two edge buffers: transposed-sync pulls, base-curl edge values
+    const size_t eb = sizeof(float) * 2 * 16 * 6 * ctx->n;
+    CK(cudaMalloc(&ctx->adC, eb), "alloc adjoint edge buffers");
+    CK(cudaMemsetAsync(ctx->adC, 0, eb, ctx->st), "memset");
+  }
   return SWM_OK;
 }
 

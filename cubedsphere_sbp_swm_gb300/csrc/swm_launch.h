@@ -22,13 +22,10 @@ cudaError_t launch_stage(int order, int cols, bool fixbw, const StageMaps* maps,
 // Sets the launch attributes of the stage kernels of one SBP order, every
 // consumer width (called at context creation, outside any stream capture),
 // and returns the default shape.
-template <class T>
 cudaError_t prepare_stage(int order, StageShape* shape);
 // Resident stage-kernel CTAs per SM when the TMA box is boxw columns wide.
-template <class T>
 int stage_occupancy(int order, int boxw, int cols, bool fixbw);
 // Widest TMA box of the kernel of consumer width cols (0: width not built).
-template <class T>
 int stage_boxw_max(int cols);
 
 // Consumer widths of the FP32 TMA stage kernel; each is instantiated in its

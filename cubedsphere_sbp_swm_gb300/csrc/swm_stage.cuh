@@ -611,7 +611,7 @@ __device__ void sync_vector_node(const EdgeView<T>& ev, const Topology& tp, cons
 
 
 // ---------------------------------------------------------------------------
-// Edge kernel: finishes every panel-boundary node of every instance.
+// FP32 edge kernel: finishes every panel-boundary node of every instance.
 // blockIdx.y = instance, x covers 6*(4n-4) nodes.
 // ---------------------------------------------------------------------------
 template <class T>
@@ -650,11 +650,10 @@ __global__ void edge_kernel(InstDev<T> one, const InstDev<T>* many, Topology tp,
           q3 = I.metric[MQI3 * fs + idx];
   const T J = I.metric[MJ * fs + idx], f = I.metric[MF * fs + idx];
   // RK inputs of the node, loaded with everything else
-  const bool fp32 = sizeof(T) == 4;
-  const bool needB = mode == MODE_RK1 || mode == MODE_RK2 || mode == MODE_RK3 ||
-                     (fp32 && mode == MODE_RK4);
+  static_assert(sizeof(T) == 4, "the FP64 stage kernel finishes its boundary nodes itself");
+  const bool needB = mode != MODE_APPLY;
   const bool needA = mode == MODE_RK2 || mode == MODE_RK3 || mode == MODE_RK4;
-  const bool needL = fp32 && mode == MODE_RK4;
+  const bool needL = mode == MODE_RK4;
   const T* bsrc = mode == MODE_RK4 ? I.base_out : I.base;
   T rb[3], ra[3], rlo[3];
 #pragma unroll

@@ -23,8 +23,7 @@ cudaError_t launch_stage<float>(int order, int cols, bool fixbw, const StageMaps
   }
 }
 
-template <>
-int stage_occupancy<float>(int order, int boxw, int cols, bool fixbw) {
+int stage_occupancy(int order, int boxw, int cols, bool fixbw) {
   switch (cols) {
     case 64: return stage_f32_occupancy<64>(order, fixbw, boxw);
     case 96: return stage_f32_occupancy<96>(order, fixbw, boxw);
@@ -35,8 +34,7 @@ int stage_occupancy<float>(int order, int boxw, int cols, bool fixbw) {
   }
 }
 
-template <>
-int stage_boxw_max<float>(int cols) {
+int stage_boxw_max(int cols) {
   switch (cols) {
     case 64: return TmaLayout<float, 42, 64>::BOXW_MAX;
     case 96: return TmaLayout<float, 42, 96>::BOXW_MAX;
@@ -47,8 +45,7 @@ int stage_boxw_max<float>(int cols) {
   }
 }
 
-template <>
-cudaError_t prepare_stage<float>(int order, StageShape* shape) {
+cudaError_t prepare_stage(int order, StageShape* shape) {
   cudaError_t e = stage_f32_prepare<64>(order);
   if (e == cudaSuccess) e = stage_f32_prepare<96>(order);
   if (e == cudaSuccess) e = stage_f32_prepare<128>(order);
@@ -57,11 +54,11 @@ cudaError_t prepare_stage<float>(int order, StageShape* shape) {
   if (e != cudaSuccess) return e;
   shape->cols = TMA_CONS_DEFAULT;
   shape->tma = 1;
-  shape->boxw = stage_boxw_max<float>(shape->cols);
+  shape->boxw = stage_boxw_max(shape->cols);
   shape->rps = TmaLayout<float, 42, TMA_CONS_DEFAULT>::RPS;
   shape->nf = TmaLayout<float, 42, TMA_CONS_DEFAULT>::NF;
   shape->fixbw = 0;
-  shape->ctas_per_sm = stage_occupancy<float>(order, shape->boxw, shape->cols, false);
+  shape->ctas_per_sm = stage_occupancy(order, shape->boxw, shape->cols, false);
   return cudaGetLastError();
 }
 

@@ -4,9 +4,6 @@
 
 namespace swm {
 
-// The FP64 stage has no work units; its contexts report one width.
-constexpr int kReportedWidth = 64;
-
 cudaError_t launch_derive64(const InstDev<double>& one, const PointBatch<double>& b, cudaStream_t st) {
   return launch_point_derive<double>(one, b, st);
 }
@@ -25,32 +22,6 @@ cudaError_t launch_stage64(int order, const InstDev<double>& one, const PointBat
 int stage64_blocks(int order, int n) {
   return (order == 21 ? point_ranges<21>(n) : order == 42 ? point_ranges<42>(n) : order == 43 ? point_ranges<43>(n)
                                                                                : point_ranges<63>(n)).total / PT_TPB;
-}
-
-template <>
-cudaError_t prepare_stage<double>(int order, StageShape* shape) {
-  (void)order;
-  shape->ctas_per_sm = 1;
-  shape->cols = kReportedWidth;
-  shape->tma = 0;
-  shape->boxw = shape->rps = shape->nf = 0;
-  shape->fixbw = 0;
-  return cudaSuccess;
-}
-
-template <>
-int stage_boxw_max<double>(int cols) {
-  (void)cols;
-  return 0;
-}
-
-template <>
-int stage_occupancy<double>(int order, int boxw, int cols, bool fixbw) {
-  (void)order;
-  (void)boxw;
-  (void)cols;
-  (void)fixbw;
-  return 1;
 }
 
 }  // namespace swm
