@@ -1458,11 +1458,11 @@ int swm_apply(swm_ctx* ctx, swm_state* vout, const swm_state* vin) {
   USE_DEVICE(ctx);
   if (ctx->cg) {
     if (ctx->prec == SWM_FP64_PLAIN) {
-      CK(cgrid_apply(ctx->cg, ctx->topo, ctx->edge64, ctx->hs64, (const double*)vin->hi, (double*)vout->hi, ctx->st),
+      CK(cgrid_apply(ctx->cg, ctx->hs64, (const double*)vin->hi, (double*)vout->hi, ctx->st),
          "C-grid apply");
     } else {  // tendencies of the high part, in FP32
       CK(cudaMemsetAsync(vout->lo, 0, sizeof(float) * 3 * ctx->fs, ctx->st), "memset");
-      CK(cgrid_apply32(ctx->cg, ctx->topo, (float*)ctx->edge, (const float*)ctx->hsT, (const float*)vin->hi,
+      CK(cgrid_apply32(ctx->cg, (const float*)ctx->hsT, (const float*)vin->hi,
                        (float*)vout->hi, ctx->st),
          "C-grid apply");
     }
@@ -1565,9 +1565,9 @@ int graph_steps(swm_ctx* ctx, swm_state* v0, double dt, int kind, int nsteps, F 
 int enqueue_rk4_any(swm_ctx* ctx, swm_state* v0, double dt) {
   if (ctx->cg) {
     if (ctx->prec == SWM_FP64_PLAIN)
-      CK(cgrid_rk4(ctx->cg, ctx->topo, ctx->edge64, ctx->hs64, (double*)v0->hi, dt, ctx->st), "C-grid RK4 step");
+      CK(cgrid_rk4(ctx->cg, ctx->hs64, (double*)v0->hi, dt, ctx->st), "C-grid RK4 step");
     else
-      CK(cgrid_rk4_32(ctx->cg, ctx->topo, (float*)ctx->edge, (const float*)ctx->hsT, (float*)v0->hi, v0->lo, dt,
+      CK(cgrid_rk4_32(ctx->cg, (const float*)ctx->hsT, (float*)v0->hi, v0->lo, dt,
                       ctx->st),
          "C-grid RK4 step");
     return SWM_OK;
@@ -1820,10 +1820,10 @@ int enqueue_diffusion_step(swm_ctx* ctx, swm_state* v0, double dt) {
   if (ctx->cg) {
     const double cu = diff_coeff4(ctx, ctx->diff_uv_coeff), ch = diff_coeff4(ctx, ctx->diff_h_coeff);
     if (ctx->prec == SWM_FP64_PLAIN)
-      CK(cgrid_diffusion_step(ctx->cg, ctx->topo, ctx->edge64, ctx->diff_uv, cu, ch, (double*)v0->hi, dt, ctx->st),
+      CK(cgrid_diffusion_step(ctx->cg, ctx->diff_uv, cu, ch, (double*)v0->hi, dt, ctx->st),
          "C-grid diffusion step");
     else
-      CK(cgrid_diffusion_step32(ctx->cg, ctx->topo, (float*)ctx->edge, ctx->diff_uv, cu, ch, (float*)v0->hi, v0->lo,
+      CK(cgrid_diffusion_step32(ctx->cg, ctx->diff_uv, cu, ch, (float*)v0->hi, v0->lo,
                                 dt, ctx->st),
          "C-grid diffusion step");
     return SWM_OK;
@@ -1931,12 +1931,12 @@ int swm_apply_diffusion(swm_ctx* ctx, swm_state* vout, const swm_state* vin) {
   if (ctx->cg) {
     const double cu = diff_coeff4(ctx, ctx->diff_uv_coeff), ch = diff_coeff4(ctx, ctx->diff_h_coeff);
     if (ctx->prec == SWM_FP64_PLAIN) {
-      CK(cgrid_diffusion(ctx->cg, ctx->topo, ctx->edge64, ctx->diff_uv, cu, ch, (const double*)vin->hi,
+      CK(cgrid_diffusion(ctx->cg, ctx->diff_uv, cu, ch, (const double*)vin->hi,
                          (double*)vout->hi, ctx->st),
          "C-grid diffusion");
     } else {
       CK(cudaMemsetAsync(vout->lo, 0, sizeof(float) * 3 * fs, ctx->st), "memset");
-      CK(cgrid_diffusion32(ctx->cg, ctx->topo, (float*)ctx->edge, ctx->diff_uv, cu, ch, (const float*)vin->hi,
+      CK(cgrid_diffusion32(ctx->cg, ctx->diff_uv, cu, ch, (const float*)vin->hi,
                            (float*)vout->hi, ctx->st),
          "C-grid diffusion");
     }

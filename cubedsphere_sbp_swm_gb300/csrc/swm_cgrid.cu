@@ -146,9 +146,10 @@ void fill_ops(int order, COps& o) {
 // GB300's FP64 pipe is narrow, so the divisions of the operators are taken
 // once on the host: reciprocal fields 1/J and 1/(J hx a), and J Qi12.  The
 // covariant metric (J Q12, Q11, Q22) and 1/(J hx a) on the faces serve the
-// contra2co transform and grad_perp of the hyperdiffusion.  The M_S* fields are
-// 1/J (faces), 1/(J hx a) (corners), 1/(2J) and 1/(J hx a) (centres) times the
-// stencil scales of the context's order (swm_cgrid_rhs.cuh).
+// contra2co transform and grad_perp of the hyperdiffusion.  The M_S* fields, last
+// and in FP64 contexts only, are 1/J (faces), 1/(J hx a) (corners), 1/(2J) and
+// 1/(J hx a) (centres) times the stencil scales of the context's order
+// (swm_cgrid_rhs.cuh).
 enum { M_JP = 0, M_QI2P, M_FP, M_RJP, M_RJPHA, M_JQI2P,  // centres
        M_JU, M_QI1U, M_RJU,                              // x-faces
        M_JV, M_QI3V, M_RJV,                              // y-faces
@@ -1044,7 +1045,7 @@ struct CGrid {
   COps ops21{};             // the 2/1 operators of the hyperdiffusion (any order)
   COpsT<float> ops21_32{};
   ScaledOps<double> sops{}, sops21{};  // the fused FP64 passes' operators
-  double* met = nullptr;   // M_COUNT fields
+  double* met = nullptr;   // M_COUNT fields (contexts of the FP32 form: M_SJU)
   float* met32 = nullptr;  // their FP32 copies (contexts of the FP32 form)
   double* wk = nullptr;    // W_COUNT fields
   double* rk = nullptr;    // Y, Kb, acc: 3 fields each
@@ -1525,8 +1526,9 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
   cudaError_t e = cudaSuccess;
   auto ok = [&](cudaError_t x) { if (e == cudaSuccess) e = x; return e == cudaSuccess; };
   const size_t fb = sizeof(double) * g.fs;
+  const int nmet = fp32 ? M_SJU : M_COUNT;
   if (!tables_only) {
-    ok(cudaMalloc(&c->met, M_COUNT * fb));
+    ok(cudaMalloc(&c->met, nmet * fb));
     ok(cudaMalloc(&c->wk, W_COUNT * fb));
     ok(cudaMalloc(&c->rk, 9 * fb));
   }
@@ -1557,7 +1559,7 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
       const std::vector<double>&ta = ci ? tc : tn, &tb = cj ? tc : tn;
       for (int j = 0; j < ny; ++j)
         for (int i = 0; i < nx; ++i) mm[(size_t)j * nx + i] = metric_of_tan(ta[i], tb[j]);
-      for (int k = 0; k < M_COUNT && e == cudaSuccess; ++k) {
+      for (int k = 0; k < nmet && e == cudaSuccess; ++k) {
         if (kMetricMesh[k] != mesh) continue;
         std::fill(hm.begin(), hm.end(), 0.0);
         double* dst = c->met + (size_t)k * g.fs;
@@ -1603,8 +1605,8 @@ int create_impl(const FieldGeom& g, int N, int order, double radius, double grav
     ok(cudaMemcpyAsync(c->ecs_jr, ejr.data(), sizeof(double) * ejr.size(), cudaMemcpyHostToDevice, st));
     ok(cudaMemcpyAsync(c->xy_w, xyw.data(), sizeof(double) * xyw.size(), cudaMemcpyHostToDevice, st));
     ok(cudaMemcpyAsync(c->xy_ind, xyind.data(), sizeof(int) * xyind.size(), cudaMemcpyHostToDevice, st));
-    if (fp32 && !tables_only && ok(cudaMalloc(&c->met32, sizeof(float) * M_COUNT * g.fs)))
-      ok(launch_to_f32(c->met, c->met32, (long long)M_COUNT * g.fs, st));  // rounded once
+    if (fp32 && !tables_only && ok(cudaMalloc(&c->met32, sizeof(float) * nmet * g.fs)))
+      ok(launch_to_f32(c->met, c->met32, (long long)nmet * g.fs, st));  // rounded once
     ok(cudaMemcpyAsync(c->wts, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice, st));
     ok(cudaStreamSynchronize(st));  // the host buffers go out of scope
   }
@@ -1712,7 +1714,7 @@ cudaError_t cgrid_coriolis(CGrid* c, const double* hu, const double* hv, const d
   return run_faces_b(c, a, st);
 }
 
-cudaError_t cgrid_apply(CGrid* c, const Topology& tp, double* edge, const double* hs, const double* in, double* out,
+cudaError_t cgrid_apply(CGrid* c, const double* hs, const double* in, double* out,
                         cudaStream_t st) {
   RhsArgs<double> a = rhs_args<double>(c);
   a.hs = hs;
@@ -1720,7 +1722,7 @@ cudaError_t cgrid_apply(CGrid* c, const Topology& tp, double* edge, const double
   return rhs(c, a, 0, in, st);
 }
 
-cudaError_t cgrid_apply32(CGrid* c, const Topology& tp, float* edge, const float* hs, const float* in, float* out,
+cudaError_t cgrid_apply32(CGrid* c, const float* hs, const float* in, float* out,
                           cudaStream_t st) {
   if (!c->met32) return cudaErrorInvalidValue;
   RhsArgs<float> a = rhs_args<float>(c);
@@ -1732,7 +1734,7 @@ cudaError_t cgrid_apply32(CGrid* c, const Topology& tp, float* edge, const float
 // The FP32 form: stage inputs are the state's high part (stage 1) or Y in
 // FP32; the increments add up in acc and the last stage adds them to the
 // (hi, lo) pair with an exact two-sum.  In-place safety as for FP64.
-cudaError_t cgrid_rk4_32(CGrid* c, const Topology& tp, float* edge, const float* hs, float* hi, float* lo, double dt,
+cudaError_t cgrid_rk4_32(CGrid* c, const float* hs, float* hi, float* lo, double dt,
                          cudaStream_t st) {
   if (!c->met32) return cudaErrorInvalidValue;
   RhsArgs<float> a = rhs_args<float>(c);
@@ -1751,7 +1753,7 @@ cudaError_t cgrid_rk4_32(CGrid* c, const Topology& tp, float* edge, const float*
 // stage input at neighbouring points (rhs1, rhs2) run before the two that
 // write it (rhs3 h, rhs4 u and v), and of it those read only h at their own
 // point (rhs3), before writing it.
-cudaError_t cgrid_rk4(CGrid* c, const Topology& tp, double* edge, const double* hs, double* y0, double dt,
+cudaError_t cgrid_rk4(CGrid* c, const double* hs, double* y0, double dt,
                       cudaStream_t st) {
   RhsArgs<double> a = rhs_args<double>(c);
   a.hs = hs;
@@ -1805,25 +1807,25 @@ cudaError_t cgrid_diffusion_prepare(CGrid* c) {
   return e;
 }
 
-cudaError_t cgrid_diffusion(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion(CGrid* c, int parts, double c4uv, double c4h,
                             const double* in, double* out, cudaStream_t st) {
   if (in == out || parts < 1 || parts > 3) return cudaErrorInvalidValue;
   return diffusion<double>(c, parts, c4uv, c4h, in, out, nullptr, 0.0, 0, st);
 }
 
-cudaError_t cgrid_diffusion_step(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion_step(CGrid* c, int parts, double c4uv, double c4h,
                                  double* y0, double dt, cudaStream_t st) {
   if (parts < 1 || parts > 3) return cudaErrorInvalidValue;
   return diffusion<double>(c, parts, c4uv, c4h, y0, y0, nullptr, dt, 1, st);
 }
 
-cudaError_t cgrid_diffusion32(CGrid* c, const Topology& tp, float* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion32(CGrid* c, int parts, double c4uv, double c4h,
                               const float* in, float* out, cudaStream_t st) {
   if (!c->met32 || in == out || parts < 1 || parts > 3) return cudaErrorInvalidValue;
   return diffusion<float>(c, parts, c4uv, c4h, in, out, nullptr, 0.0, 0, st);
 }
 
-cudaError_t cgrid_diffusion_step32(CGrid* c, const Topology& tp, float* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion_step32(CGrid* c, int parts, double c4uv, double c4h,
                                    float* hi, float* lo, double dt, cudaStream_t st) {
   if (!c->met32 || parts < 1 || parts > 3) return cudaErrorInvalidValue;
   return diffusion<float>(c, parts, c4uv, c4h, hi, hi, lo, dt, 2, st);

@@ -56,17 +56,17 @@ cudaError_t cgrid_coriolis(CGrid* c, const double* hu, const double* hv, const d
 
 // operator_swm_t%apply (vector-invariant form): tendencies (th, tu, tv) of
 // the state (h, u, v); each state is 3 fields spaced g.fs apart.  hs nullable.
-cudaError_t cgrid_apply(CGrid* c, const Topology& tp, double* edge, const double* hs, const double* in,
+cudaError_t cgrid_apply(CGrid* c, const double* hs, const double* in,
                         double* out, cudaStream_t st);
 // One rk4_t%step of the state y0 in place (rk4_mod.f90:20-42).
-cudaError_t cgrid_rk4(CGrid* c, const Topology& tp, double* edge, const double* hs, double* y0,
+cudaError_t cgrid_rk4(CGrid* c, const double* hs, double* y0,
                       double dt, cudaStream_t st);
 // The FP32 form (contexts created with fp32): the same passes in FP32 on
 // FP32 states; the RK4 step keeps the state as an FP32 (hi, lo) pair and
 // adds the stage increments with an exact two-sum.
-cudaError_t cgrid_apply32(CGrid* c, const Topology& tp, float* edge, const float* hs, const float* in,
+cudaError_t cgrid_apply32(CGrid* c, const float* hs, const float* in,
                           float* out, cudaStream_t st);
-cudaError_t cgrid_rk4_32(CGrid* c, const Topology& tp, float* edge, const float* hs, float* hi, float* lo,
+cudaError_t cgrid_rk4_32(CGrid* c, const float* hs, float* hi, float* lo,
                          double dt, cudaStream_t st);
 // A mesh field in the dense host layout (6 panels of ny rows of nx points)
 // to / from its pitched device field: FP64 (lo == nullptr), or the FP32
@@ -90,13 +90,13 @@ cudaError_t cgrid_contra2co(CGrid* c, const double* ut, const double* vt, double
 // fields; call it once, outside any stream capture, before the others (they
 // return cudaErrorInvalidValue until then).
 cudaError_t cgrid_diffusion_prepare(CGrid* c);
-cudaError_t cgrid_diffusion(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion(CGrid* c, int parts, double c4uv, double c4h,
                             const double* in, double* out, cudaStream_t st);
-cudaError_t cgrid_diffusion_step(CGrid* c, const Topology& tp, double* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion_step(CGrid* c, int parts, double c4uv, double c4h,
                                  double* y0, double dt, cudaStream_t st);
-cudaError_t cgrid_diffusion32(CGrid* c, const Topology& tp, float* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion32(CGrid* c, int parts, double c4uv, double c4h,
                               const float* in, float* out, cudaStream_t st);
-cudaError_t cgrid_diffusion_step32(CGrid* c, const Topology& tp, float* edge, int parts, double c4uv, double c4h,
+cudaError_t cgrid_diffusion_step32(CGrid* c, int parts, double c4uv, double c4h,
                                    float* hi, float* lo, double dt, cudaStream_t st);
 // The ECS_O scalar halo of a cell-centre field (equiang_cs/ecs_halo_mod.f90:
 // 95-475, create_halo_procedure "ECS_O") and gradient_a2_ecs (gradient/
