@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(PT_TPB) lap_d1_kernel(FieldGeom g, const doubl
   int p, i, j;
   const int n = g.n, P = g.P;
   if (!point_node<E>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
-  const long long x = (long long)p * g.ps + (long long)j * P + i, group = blockIdx.y * NF * g.fs;
+  const long long x = (long long)p * g.ps + (long long)j * P + i, group = NF == 1 ? blockIdx.y * g.fs : 0;
   f += group;
   d1x += group;
   d1y += group;
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(PT_TPB) lap_main_kernel(
   const int n = g.n, P = g.P;
   if (!point_node<E>(n, blockIdx.x * PT_TPB + threadIdx.x, p, i, j)) return;
   const long long fs = g.fs, x = (long long)p * g.ps + (long long)j * P + i;
-  const int first = blockIdx.y * NF;   // field of this thread's first
+  const int first = NF == 1 ? blockIdx.y : 0;   // field of this thread's first
   f += first * fs;
   d1x += first * fs;
   d1y += first * fs;
@@ -873,8 +873,8 @@ long long narrow_closure_count(int narrow, int n) {
   return 6LL * n * 2 * narrow_rows(narrow) * narrow_cols(narrow);
 }
 
-// The two passes of the FP64 Laplacian, NF fields a thread and a group of NF
-// fields a grid row; ROWS: warps along the row on every column.
+// The two passes of the FP64 Laplacian, all NF fields of a node by one thread, or
+// (NF 1) a field a grid row; ROWS: warps along the row on every column.
 template <int NARROW, int NF, bool ROWS>
 void lap_launch(dim3 grid, const FieldGeom& g, const NarrowTables<double>& t, const double* f, const double* mt,
                 double* d1x, double* d1y, double* out, double* edge, cudaStream_t st) {
