@@ -397,11 +397,17 @@ __global__ void __launch_bounds__(PT_TPB, 5)
   const int p = at.p, i = at.i, j = at.j;
   const long long fs = I.fs, x = (long long)p * I.ps + (long long)j * P + i;
   T rb[3] = {}, ra[3] = {}, rl[3] = {};
+  auto rk_load = [&]() {
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (needB) rb[c] = I.base[c * fs + x];
-    if (needA) ra[c] = I.acc ? I.acc[c * fs + x] : T(0);
-  }
+    for (int c = 0; c < 3; ++c) {
+      if (needB) rb[c] = I.base[c * fs + x];
+      if (needA) ra[c] = I.acc ? I.acc[c * fs + x] : T(0);
+    }
+  };
+  // At 6/3 the nine taps and these inputs together spill 68 bytes in stages 2 and
+  // 3 (N=256 0.218 ms a step, 0.216 so), so a boundary node reads them last.
+  constexpr bool late = Taps<ORD>::NT > 6 && needA && needB;
+  if (!(late && at.boundary)) rk_load();
   const T f = I.metric[MF * fs + x];
   const T jut = I.der[DR_JUT * fs + x], jvt = I.der[DR_JVT * fs + x];
   T kh, ku, kv;
@@ -445,6 +451,7 @@ __global__ void __launch_bounds__(PT_TPB, 5)
     sz += __shfl_xor_sync(0xffffffffu, sz, 1);
     sd += __shfl_xor_sync(0xffffffffu, sd, 1);
     if (!own || !at.live) return;
+    if (late) rk_load();
     const T w = lr && bt ? T(1.0 / 3.0) : T(0.5);
     const T fz = f + w * sz;
     kh = -(w * sd);
