@@ -260,7 +260,7 @@ constexpr StageShape kFp64Shape{1, 64, 0, 0, 0, 0, 0};
 constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
 constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
 constexpr double kCrowdHalo = 3.3;     // the same where an ensemble's whole-panel units fill the GPU
-constexpr int kSpread = 152;           // units that give every SM of a GB300 one
+constexpr int kSpread = 152;           // units that give each of a GB300's 152 SMs one
 double row_closure_cost(const SbpC& s) { return s.ne >= 6 ? 2.0 : 1.0; }
 
 // The column strips of a panel of n nodes a side and the cost model of its rows.
@@ -2377,8 +2377,8 @@ std::string mem_err(swm_ensemble* ens) {
 // ones that give 1 to 4 waves of units (few members need short units to fill
 // the GPU, many need several waves to even out their sizes).  Whole-panel
 // units, the earlier default, left a small ensemble on a few CTAs: 9 members
-// (3 each of N=48, 96, 192, d42, FP32) 485 us a step, with 456 such units
-// 125 us; 96 members 1044 us whole-panel, 1010 with 1728 units.
+// (3 each of N=48, 96, 192, d42, FP32) 487 us a step, with 900 such units
+// 128 us; 96 members 1031 us whole-panel, 942 with 1344 units.
 // A crowded ensemble, whose whole-panel units take half of the CTA slots or
 // more, has CTAs beside each other on every SM, and a shorter unit costs it more:
 // its halo rows are issue slots that another unit would have used.  From the

@@ -90,8 +90,12 @@ struct RhsArgs {
 
 constexpr int kRhsX = 32, kRhsY = 8, kRhsEdge = 4;
 // Resident blocks per SM the passes are compiled for.  FP32 waits on memory
-// and wants every warp slot: 8 blocks (32 registers) 0.365 ms a model step at
-// N=384, unconstrained 0.380, 6 blocks 0.394, 4 blocks 0.455.  FP64 waits on
+// and wants every warp slot on large panels: 8 blocks (32 registers) 0.365 ms a
+// model step at N=384, unconstrained 0.380, 6 blocks 0.394, 4 blocks 0.455; up to
+// N=160, where few blocks are resident at all, 3, 4 and 6 blocks measured 0 to 5%
+// faster (RK4 step 4/2, side columns still in warps along the column: N=48 119 us
+// for 123, N=96 111 for 115), which two compiled variants of every pass are not
+// worth.  FP64 waits on
 // its pipe and measures the same at 6 and 8 (3% slower unconstrained).
 template <class T>
 constexpr int kRhsBlocks = sizeof(T) == 4 ? 8 : 6;

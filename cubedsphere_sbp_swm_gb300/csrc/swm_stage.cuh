@@ -138,10 +138,9 @@ __device__ __forceinline__ void node_tendency(T gx, T gy, T zeta, T dv, T f, T J
 // once in 64 cycles, so the FP64 instructions per node are the cost and
 // memory traffic is nearly free beside them.  Hence:
 //   - the pointwise stencil inputs are formed once per node, by the kernel
-//     that makes the state, and kept in fields (a row-streaming kernel that
-//     formed them for its halo rows and columns as well took 0.451 ms a step
-//     at N=384 d42 and 0.251 ms at N=192, where units had 8 rows and 6 halo
-//     rows);
+//     that makes the state, and kept in fields (the earlier row-streaming
+//     kernel formed them for its halo rows and columns as well: units of 8 rows
+//     had 6 halo rows at N=192);
 //   - one thread per node and no work units, so that every SM quarter gets
 //     the same number of warps at any size;
 //   - the nodes of the NE closure columns at either panel side are separate
@@ -153,14 +152,14 @@ __device__ __forceinline__ void node_tendency(T gx, T gy, T zeta, T dv, T f, T J
 //     first, instead of a second launch that exchanges them (one lane for
 //     both: 0.126 against 0.073 ms a step at N=48, before the Taps);
 //   - differences are taken before they are scaled, and the constants come
-//     from the host: 32 FP64 instructions a node and 11 for the stencil inputs
-//     (4/2), against 58; with constants formed per thread 50 instead of 45
-//     (0.343 against 0.306 ms a step).
-// Measured, RK4 steps d42 of one instance: N=48 0.239 -> 0.052 ms, N=192 0.251
-// -> 0.112 ms, N=384 0.560 -> 0.351 ms.  The FP64 pipe is 82% busy in a launch
-// at N=384.  Blocks of 64 and 256 threads measured within 1% of 128; compiled
-// for 4 blocks an SM 4% slower at N=384 and 8% faster at N=48 than for 5, for 7
-// the reverse.
+//     from the host: 32 FP64 instructions an inner node and 11 for its stencil
+//     inputs (4/2), against 58 (constants formed per thread would be 5 more).
+// Measured, RK4 steps d42 of one instance back to back, against the row-streaming
+// kernel: N=48 0.237 -> 0.049 ms, N=384 0.546 -> 0.345 ms, N=1024 2.93 -> 2.17
+// ms.  The FP64 pipe is 82% busy in a launch at N=384.  Blocks of 64 and 256 threads
+// measured within 1% of 128; compiled for 4 blocks an SM 4% slower at N=384 and 8%
+// faster at N=48 than for 5, for 7 the reverse: 5 gives up 1% at N=384 (0.342 ms
+// before the taps and the bound) for the small panels.
 // ---------------------------------------------------------------------------
 constexpr int PT_TPB = 128;
 

@@ -1,6 +1,6 @@
 // swm_stage_tma.cuh -- fused RHS + RK stage kernel, TMA-pipelined.
 //
-// Same arithmetic as stage_kernel (swm_stage.cuh), different data movement.
+// The FP32 stage (the FP64 one, bound by GB300's FP64 rate, is in swm_stage.cuh).
 // Every buffer is described to the TMA unit as a 3-D tensor (column, row of
 // all panels, field).  One producer warp streams a work unit (a panel strip
 // plus its halo columns) through an NST-deep shared-memory pipeline: each

@@ -394,9 +394,10 @@ int swm_quadrature_weights(swm_ctx* ctx, double* w_host);
 /* job): independent members, each with its own N, initial state and time   */
 /* step, sharing SBP order, constants and precision.  Each member is a full */
 /* context; an ensemble RK4 step is one CUDA graph with, per RK stage, one  */
-/* stage-kernel launch over the work units of all members (persistent CTAs  */
-/* in the FP32 form) and one edge-kernel launch.  Each member's arithmetic  */
-/* is exactly that of swm_rk4_step on the member alone.                     */
+/* stage-kernel launch over all members and, in the FP32 form, one edge-    */
+/* kernel launch (FP64: one more for the stencil inputs of the first stage).*/
+/* Each member's arithmetic is exactly that of swm_rk4_step on the member   */
+/* alone.                                                                   */
 /* ---------------------------------------------------------------------- */
 typedef struct swm_ensemble swm_ensemble;
 
