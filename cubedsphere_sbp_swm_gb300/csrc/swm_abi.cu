@@ -2827,7 +2827,6 @@ int swm_ensemble_tune(swm_ensemble* ens, int steps, int* seg_rows_out, int* grid
       if (f32 && seg != kAutoRows && seg >= ens->max_n) continue;
       for (int gi = 0; gi < ngrid && rc == SWM_OK; ++gi) {
         const int cta = f32 ? grids[gi] : set_grid;
-        if (f32 && seg == kAutoRows && cta != 0) continue;
         if ((rc = ens_rebuild(ens, seg, cta))) break;
         cudaGraphLaunch(ens->graph, ens->st);                          // warm-up
         cudaEventRecord(a, ens->st);

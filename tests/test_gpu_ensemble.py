@@ -224,3 +224,29 @@ def test_default_split_of_other_orders_and_crowds(prec, order, sizes):
     for m, N in enumerate(sizes):
         for a, b in zip(ens.download(m), want[N]):
             assert np.array_equal(a, b), f"member {m} (N={N}) differs"
+
+
+def test_tuner_knows_the_crowded_default():
+    """A crowded ensemble of one size has persistent CTAs on the default units;
+    the tuner times that shape too, and a tuned ensemble steps on as before."""
+    sizes = (16,) * 130
+    ens = swm.Ensemble(swm.ModelConfig(N=16, precision="fp32"), sizes, [_dt(16)] * len(sizes))
+    default = ens.get_shape()
+    assert default["seg_rows"] == ens.ROWS_AUTO and default["grid"] > 0
+    x = initial.balanced_zonal(16, 3, 4)[:3]
+    for m in range(len(sizes)):
+        ens.upload(m, *x)
+    res = ens.tune(steps=3)
+    ens.set_shape(default["seg_rows"], default["grid"])
+    ens.set_width(default["width"])
+    assert ens.get_shape() == default
+    ens.set_width(res["width"])
+    ens.set_shape(res["seg_rows"], res["grid"])
+    ens.step(2)
+    op = swm.OperatorSWM(swm.ModelConfig(N=16, precision="fp32"))
+    s = op.create_stvec()
+    s.upload(*x)
+    swm.RK4().step(s, op, _dt(16), 2)
+    for m in (0, len(sizes) - 1):
+        for a, b in zip(ens.download(m), s.download()):
+            assert np.array_equal(a, b)
