@@ -259,7 +259,7 @@ constexpr StageShape kFp64Shape{1, 64, 0, 0, 0, 0, 0};
 
 constexpr double kStripEdge = 0.3;     // extra cost of a row of a panel-edge strip
 constexpr double kUnitHalo = 0.8;      // cost of a unit's halo, in rows per RMAX
-constexpr double kCrowdHalo = 3.3;     // the same where an ensemble's whole-panel units fill the GPU
+constexpr double kCrowdHalo = 3.3;     // the same in a crowded ensemble (ens_units)
 constexpr int kSpread = 152;           // units that give each of a GB300's 152 SMs one
 double row_closure_cost(const SbpC& s) { return s.ne >= 6 ? 2.0 : 1.0; }
 
@@ -2382,7 +2382,7 @@ std::string mem_err(swm_ensemble* ens) {
 // A crowded ensemble, whose whole-panel units take half of the CTA slots or
 // more, has CTAs beside each other on every SM, and a shorter unit costs it more:
 // its halo rows are issue slots that another unit would have used.  From the
-// times of 17 such ensembles the halo of a unit is 3.3 rows per RMAX there.  With
+// times of a dozen such ensembles at 4/2 and 6/3 the halo of a unit is 3.3 rows per RMAX there.  With
 // 0.8: 60 members of N=32 157 us a step, 133 with 3.3 (whole-panel units 133); 100
 // of N=16 155 and 138 (152); 100 of N=20 d63 223 and 190 (215).  Ensembles below
 // half, where 3.3 gave 6% less for 10 members of N=128 d63 and 11% less for one of
